@@ -103,6 +103,35 @@ def test_gpu_gradients_match_oracle(torch, n_in, n_out, batch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n_in,hidden,layers,n_out,batch,rows", [
+    (1, 1, 1, 1, 16, 1),          # one fragment of one tile everywhere
+    (17, 100, 2, 65, 80, 63),     # ragged tiles in every dimension
+    (163, 64, 5, 161, 1040, 65),  # the deepest network, a last slice of 16 rows
+    (300, 256, 1, 12, 4096, 129)])
+def test_gpu_tiles_and_slices(torch, n_in, hidden, layers, n_out, batch, rows):
+    """Tile remainders, batch slices of the weight gradient and depths: the
+    bounds of test_gpu_gradients_match_oracle (BF16 products, 2^-9 relative
+    each, of which single roundings flip)."""
+    from zerork_b200.predictor import Mlp
+    rng = np.random.default_rng(5)
+    net = Mlp(n_in, n_out, hidden, layers, seed=3)
+    d, w, b = _net(rng, n_in, hidden, layers, n_out)
+    net.set_params(w, b)
+    x = rng.standard_normal((batch, n_in)).astype(np.float32)
+    t = rng.standard_normal((batch, n_out)).astype(np.float32)
+    loss = torch.zeros(1, dtype=torch.float32, device="cuda")
+    net.gradients(torch.from_numpy(x).cuda(), torch.from_numpy(t).cuda(), loss)
+    gw, gb = net.grads()
+    lo, ow, ob, yo = mo.forward_backward(w, b, d, x, t.astype(np.float64))
+    y = net.forward(torch.from_numpy(x[:rows]).cuda()).cpu().numpy()
+    assert np.max(np.abs(y - yo[:rows])) <= 1e-2 * np.abs(yo).max()
+    assert abs(float(loss.item()) - lo) <= 1e-2 * lo
+    for g, go in zip(mo.unpack(gw, gb, d), mo.unpack(ow, ob, d)):
+        for a, o in zip(g, go):
+            assert np.linalg.norm(a - o) <= 1e-2 * max(np.linalg.norm(o), 1e-30)
+
+
+@pytest.mark.gpu
 def test_gpu_training_reduces_loss(torch):
     from zerork_b200.predictor import train
     rng = np.random.default_rng(4)

@@ -37,11 +37,13 @@ class Mlp {
   MlpDev device_view() const;
 
  private:
-  cudaError_t ensure_ws(int rows);
-  void carve(int rows, std::vector<__nv_bfloat16 *> &X, std::vector<float *> &Z, float *&dZf,
-             __nv_bfloat16 *&dZ, float *&dA, float *&row_sq);
-  cudaError_t forward_ws(int rows, const float *x, std::vector<__nv_bfloat16 *> &X, std::vector<float *> &Z,
-                         cudaStream_t s);
+  struct Work {  // device workspace of one call
+    __nv_bfloat16 *X[kMlpMaxLayers], *dZ[2];
+    float *Z[kMlpMaxLayers], *dW[kMlpMaxLayers], *db[kMlpMaxLayers], *loss;
+    int slices[kMlpMaxLayers], chunk[kMlpMaxLayers];
+  };
+  cudaError_t carve(int rows, bool train, Work &w);
+  cudaError_t hidden_layers(int n, int rows, const float *x, const Work &w, bool keep, cudaStream_t s);
   int n_in_, n_out_;
   std::vector<int> dims_;
   std::vector<long> woff_, boff_;
@@ -50,7 +52,6 @@ class Mlp {
   void *wbf_ = nullptr;
   void *ws_ = nullptr;
   size_t ws_bytes_ = 0;
-  int ws_rows_ = 0;
   long step_ = 0;
 };
 
