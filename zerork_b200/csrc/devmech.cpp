@@ -152,6 +152,10 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     jr_ptr.push_back((int)jr_kk.size());
   }
 
+  std::vector<int> nz_rc(p.nnz);
+  for (int j = 0; j < p.n; ++j)
+    for (int k = p.col_ptr[j]; k < p.col_ptr[j + 1]; ++k) nz_rc[k] = p.row_idx[k] | (j << 16);
+
   // cost-sorted work lists (stable: ties keep index order)
   auto sorted_by = [](std::vector<double> cost) {
     std::vector<int> idx(cost.size());
@@ -207,6 +211,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   size_t o_lr = b.add(p.last_row);
   size_t o_ndp = b.add(nzd_ptr), o_nds = b.add(nzd_step), o_ncp = b.add(nzc_ptr), o_ncs = b.add(nzc_step);
   size_t o_jrp = b.add(jr_ptr), o_jrk = b.add(jr_kk), o_jrc = b.add(jr_col);
+  size_t o_rc = b.add(nz_rc);
   size_t o_ro = b.add(rxn_order), o_co = b.add(col_order);
   bytes_ = b.bytes.size();
   check(cudaMalloc(&blob_, bytes_), "cudaMalloc(mechanism tables)");
@@ -260,6 +265,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.jr_ptr = (const int *)P(o_jrp);
   view_.jr_kk = (const int *)P(o_jrk);
   view_.jr_col = (const int *)P(o_jrc);
+  view_.nz_rc = (const int *)P(o_rc);
   view_.rxn_order = (const int *)P(o_ro);
   view_.spc_order = (const int *)P(o_so);
   view_.col_order = (const int *)P(o_co);

@@ -72,6 +72,7 @@ struct DevMech {
   // into the compressed-column values) in columns jr_col[p], p in
   // [jr_ptr[i], jr_ptr[i+1])
   const int *jr_ptr, *jr_kk, *jr_col;
+  const int *nz_rc;  // per Jacobian nonzero: row | column << 16
   // work lists sorted by decreasing estimated cost, for snake-order
   // assignment to thread groups: reactions, species (production gathers),
   // species Jacobian columns

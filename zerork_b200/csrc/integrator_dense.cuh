@@ -27,15 +27,18 @@ constexpr double kMinFactor = 0.2;
 constexpr double kMaxFactor = 10.0;
 constexpr double kEtaKeep = 1.5;
 constexpr int kMaxl = 10;  // Krylov dimension (no restarts)
+constexpr int kPanelMax = 8;  // widest panel of the inversion
 constexpr int kPredBuf = 256;  // widest predictor layer (padded)
 
 struct Smem {
-  double *red;  // 128 slots: block sums [0, 33), pivot candidates [64, 112)
+  double *red;  // 128 slots: block sums [0, 33); the inversion keeps the pivot columns here
   double *C, *G, *U, *ROP;
   double *D, *y, *f, *f0, *ypred, *psi, *d, *scale, *tmp, *yp;
   void *A;      // n x lda inverse (LT)
-  int *perm;    // n: row i of the factored matrix is scaled row perm[i]
-  double *colk; // n (LT-sized use)
+  double *rows; // kPanelMax x n pivot rows of the inversion: overlays vectors that are dead then
+  int *perm;    // n + 1: low half of entry j the pivot row of column j, high half of entry i
+                // the column that row i was the pivot of; entry n the singular flag
+  double *colk; // n: operator product of the Krylov path
   double *wlu;  // n: error-weight scale the stored inverse was formed with
   double *bs;   // n: scaled right-hand side
   double *V;    // FP32 path: (kMaxl + 1) Krylov vectors, then 2 work vectors
@@ -238,273 +241,253 @@ __device__ __noinline__ int jac_cta(const DevMech &m, const IntegOpts &o, const 
 // species spanning 20 decades of mass fraction and keeps the inverse
 // accurate in the weighted norm the Newton test uses.
 //
-// Gauss-Jordan with partial pivoting, in place, two pivots per sweep of the
-// matrix.  Row interchanges are accumulated in perm (row i of the factored
-// matrix is row perm[i] of Pw), so A ends as (Pi Pw)^-1 = Pw^-1 Pi^T and the
-// right-hand side is permuted on application instead of unswapping columns.
-// Per pair of pivots (k, k+1), four barriers:
-//   S1  pick pivot k from the per-warp candidates (every thread makes the
-//       same choice), swap rows, scaled pivot row r1 (kept in colk);
-//   C   column k+1 as it will be after eliminating column k,
-//       g_i = a_i[k+1] - a_i[k] r1[k+1], gives the candidates for pivot k+1
-//       (each carries its a_i[k]);
-//   S2  pick pivot k+1, swap the raw rows, r2 = scaled (a_{k+1} - a_{k+1}[k]
-//       r1), row k becomes r1 - r1[k+1] r2;
-//   U   every other row in one pass, a_i - a_i[k] r1 - g_i r2 (columns k and
-//       k+1 get their Gauss-Jordan values from the lanes that own them), warp
-//       w owning rows i = w (mod warps), two rows per pass with every load
-//       issued before the stores, lane l the columns l (mod 32) with r1 and
-//       r2 in registers; it leaves the candidates for column k+2.
-// A lone last pivot is swept on its own.  Returns nonzero (all threads) for a
-// singular or non-finite matrix.
-__device__ __forceinline__ void track(double &ca, int &ci, double &cv, double &cf, double a, int i, double f) {
-  const double d = fabs(a);
-  if (d > ca) {
-    ca = d;
-    ci = i;
-    cv = a;
-    cf = f;
-  }
+// Blocked Gauss-Jordan in place with partial pivoting, PB columns at a time
+// (Quintana-Orti et al., SIAM J. Sci. Comput. 22 (2001) 1762, with look-ahead
+// and without moving rows):
+//   * warp 0 holds the panel of PB columns in registers (lane l the rows l,
+//     l + 32, ...) and exchanges its PB pivots with warp reductions and
+//     shuffles alone, no block barrier; the columns end as W, the panel's
+//     part of the inverse;
+//   * every other column then changes by one rank-PB product,
+//     A_ij = (i a pivot row ? 0 : A_ij) + sum_s W_is R_sj, with R the pivot
+//     rows before the update (copied to s.rows);
+//   * the next panel's columns are updated first, so warp 0 factors them
+//     while the other warps finish the rest.
+// Rows are never swapped: column j's pivot row is noted in perm, unknown j of
+// the inverse sits in that row and the right-hand side is gathered in that
+// order.  Pivots are the largest by the upper word of |a| (20 mantissa bits,
+// ties to the lowest row): one redux instead of a 64-bit shuffle tree.
+//
+// The sweep by pairs of pivots that this replaces went over the whole matrix
+// once per pair (162 passes of shared memory at n = 161) with four block
+// barriers each.  Panel width: what the registers of the panel warp hold,
+// NC x PB values (128 registers a thread at 512 threads).
+//   n = 161 FP64 (160 species)  1,410 K cycles before, 577 K now
+//   n = 80 FP64                   407 K cycles before, 172 K now
+template <class LT>
+__device__ __forceinline__ unsigned pivot_key(LT a) {
+  if constexpr (sizeof(LT) == 8) return (unsigned)__double2hiint(a) & 0x7fffffffu;
+  else return __float_as_uint(a) & 0x7fffffffu;
 }
 
-// Largest |value| over the warp, ties to the lowest row; every lane ends
-// with the same (a, i, v, f).
-__device__ __forceinline__ void warp_argmax(double &a, int &i, double &v, double &f) {
+// Exchange of the panel columns [k, k + pw) by one warp; `used` has bit r set
+// when this lane's row lane + 32 r has been a pivot.  Returns nonzero (all
+// lanes) for a singular or non-finite panel.
+template <class LT, int NC, int PB>
+__device__ __forceinline__ int panel_warp(LT *A, int lda, int n, int k, int pw, int *perm, unsigned &used) {
+  constexpr unsigned kInf = sizeof(LT) == 8 ? 0x7ff00000u : 0x7f800000u;
+  const int lane = threadIdx.x & 31;
+  LT a[NC][PB];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double oa = __shfl_xor_sync(kFull, a, o), ov = __shfl_xor_sync(kFull, v, o);
-    const double of = __shfl_xor_sync(kFull, f, o);
-    const int oi = __shfl_xor_sync(kFull, i, o);
-    if (oa > a || (oa == a && oi < i)) {
-      a = oa;
-      i = oi;
-      v = ov;
-      f = of;
+  for (int r = 0; r < NC; ++r)
+#pragma unroll
+    for (int c = 0; c < PB; ++c)
+      a[r][c] = (lane + 32 * r < n && c < pw) ? A[(lane + 32 * r) * lda + k + c] : (LT)0;
+  // a rolled loop: every exchange rotates the panel left by one column in
+  // registers, so the pivot column is always the first
+#pragma unroll 1
+  for (int t = 0; t < pw; ++t) {
+    unsigned key = 0, row = 0xffffffffu;
+    bool nan = false;
+#pragma unroll
+    for (int r = 0; r < NC; ++r) {
+      const unsigned q = pivot_key(a[r][0]);
+      nan |= q >= kInf;
+      if (!(used >> r & 1) && q > key) {  // (rows past n hold zeros)
+        key = q;
+        row = lane + 32 * r;
+      }
+    }
+    const unsigned best = __reduce_max_sync(kFull, key);
+    if (best == 0 || __any_sync(kFull, nan)) return 1;
+    const int p = (int)__reduce_min_sync(kFull, key == best ? row : 0xffffffffu);
+    const int slot = p >> 5, owner = p & 31;
+    LT v[PB];
+#pragma unroll
+    for (int r = 0; r < NC; ++r)
+      if (r == slot)
+#pragma unroll
+        for (int c = 0; c < PB; ++c) v[c] = a[r][c];
+#pragma unroll
+    for (int c = 0; c < PB; ++c) v[c] = __shfl_sync(kFull, v[c], owner);
+    v[0] = (LT)1 / v[0];
+#pragma unroll
+    for (int c = 1; c < PB; ++c) v[c] *= v[0];
+#pragma unroll
+    for (int r = 0; r < NC; ++r) {
+      const LT f = a[r][0];
+      const bool pr = r == slot && lane == owner;
+#pragma unroll
+      for (int c = 1; c < PB; ++c) {
+        const LT e = a[r][c] - f * v[c];
+        a[r][c - 1] = pr ? v[c] : e;
+      }
+      a[r][PB - 1] = pr ? v[0] : -f * v[0];
+    }
+    if (lane == owner) used |= 1u << slot;
+    if (lane == 0) {
+      reinterpret_cast<short *>(perm + k + t)[0] = (short)p;
+      reinterpret_cast<short *>(perm + p)[1] = (short)(k + t);
     }
   }
+#pragma unroll
+  for (int c = 0; c < PB; ++c) {
+    const int oc = c + pw - (c + pw >= PB ? PB : 0);  // the column at place c after pw rotations
+#pragma unroll
+    for (int r = 0; r < NC; ++r)
+      if (lane + 32 * r < n && oc < pw) A[(lane + 32 * r) * lda + k + oc] = a[r][c];
+  }
+  return 0;
 }
 
-template <class LT, int NC>
+__device__ __forceinline__ int pivot_row(const int *perm, int j) { return perm[j] & 0xffff; }
+__device__ __forceinline__ int pivot_col(const int *perm, int i) { return perm[i] >> 16; }
+
+template <class LT, int NC, int PB>
 __device__ __noinline__ int invert_cta(const DevMech &m, const Smem &s, const double *J, double c, int n,
                                        int lda) {
   LT *A = (LT *)s.A;
-  LT *r1b = (LT *)s.colk;
+  LT *R = (LT *)s.rows;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
-  double *cand = s.red + 64;  // [0,16) |pivot|, [16,32) row, [32,48) value, [48,64) a_row[k]
   for (int i = tid; i < n * lda; i += nt) A[i] = (LT)0;
   for (int i = tid; i < n; i += nt) {
-    s.wlu[i] = s.scale[i];
-    s.perm[i] = i;
+    const double sc = s.scale[i];
+    s.wlu[i] = sc;
+    s.rows[i] = -c / sc;
+    s.perm[i] = -1;  // no pivot yet: pivot_col < 0
   }
+  if (tid == 0) s.perm[n] = 0;
   __syncthreads();
-  for (int i = tid; i < n; i += nt) {  // Jacobian row i from the row-wise view
-    const double ci = -c / s.wlu[i];
-    for (int q = m.jr_ptr[i]; q < m.jr_ptr[i + 1]; ++q) {
-      const int j = m.jr_col[q];
-      A[i * lda + j] = (LT)(ci * J[m.jr_kk[q]] * s.wlu[j]);
-    }
+#pragma unroll 4
+  for (int q = tid; q < m.nnz; q += nt) {
+    const int rc = m.nz_rc[q], i = rc & 0xffff, j = rc >> 16;
+    const double v = s.rows[i] * J[q] * s.wlu[j];
+    A[i * lda + j] = (LT)v;
   }
   __syncthreads();
   for (int i = tid; i < n; i += nt) A[i * lda + i] += (LT)1;
   __syncthreads();
-  auto publish = [&](double ca, int ci, double cv, double cf) {
-    warp_argmax(ca, ci, cv, cf);
-    if (lane == 0) {
-      cand[w] = ca;
-      cand[16 + w] = (double)ci;
-      cand[32 + w] = cv;
-      cand[48 + w] = cf;
-    }
-  };
-  // the pivot every thread picks from the candidates; -1 if singular
-  auto pick = [&](double &pv, double &pf) -> int {
-    double best = lane < nw ? cand[lane] : -1.0, v = lane < nw ? cand[32 + lane] : 0.0;
-    double f = lane < nw ? cand[48 + lane] : 0.0;
-    int p = lane < nw ? (int)cand[16 + lane] : n;
-    warp_argmax(best, p, v, f);
-    pv = v;
-    pf = f;
-    return (!(best > 0.0) || !isfinite(best) || p >= n) ? -1 : p;
-  };
-  {  // candidates for column 0
-    double ca = -1.0, cv = 0.0, cf = 0.0;
-    int ci = n;
-    for (int i = tid; i < n; i += nt) track(ca, ci, cv, cf, (double)A[i * lda], i, 0.0);
-    publish(ca, ci, cv, cf);
-  }
+  unsigned used = 0;
+  if (w == 0 && panel_warp<LT, NC, PB>(A, lda, n, 0, min(PB, n), s.perm, used)) s.perm[n] = 1;
   __syncthreads();
-  int bad = 0;
-  for (int k = 0; k < n;) {
-    // ---- S1: first pivot of the pair
-    double pv1, unused;
-    const int p1 = pick(pv1, unused);
-    if (p1 < 0) {
-      bad = 1;
-      break;  // uniform: every thread made the same choice
-    }
-    const LT pinv1 = (LT)1 / (LT)pv1;
-    if (tid == 0) {
-      const int t = s.perm[k];
-      s.perm[k] = s.perm[p1];
-      s.perm[p1] = t;
-    }
-    for (int j = tid; j < n; j += nt) {
-      const LT a = A[k * lda + j], b = A[p1 * lda + j];
-      A[p1 * lda + j] = a;
-      const LT r = (j == k ? (LT)1 : b) * pinv1;
-      A[k * lda + j] = r;
-      r1b[j] = r;
+  for (int k = 0; k < n && !s.perm[n]; k += PB) {
+    const int pw = min(PB, n - k), k2 = k + pw, pw2 = min(PB, n - k2);
+    auto in_panel = [&](int i) { return (unsigned)(pivot_col(s.perm, i) - k) < (unsigned)pw; };
+    for (int q = tid; q < pw * n; q += nt) {  // the pivot rows before the update
+      const int t = q / n, j = q - t * n;
+      R[q] = A[pivot_row(s.perm, k + t) * lda + j];
     }
     __syncthreads();
-    if (k + 1 == n) {  // lone last pivot
-      for (int i = w; i < n; i += nw) {
-        if (i == k) continue;
-        const LT f = A[i * lda + k];
-        __syncwarp();
-        if (f != (LT)0)
-          for (int j = lane; j < n; j += 32) A[i * lda + j] = (j == k ? (LT)0 : A[i * lda + j]) - f * r1b[j];
+    if (pw2 > 0) {
+      for (int q = tid; q < pw2 * n; q += nt) {  // the next panel's columns
+        const int t = q / n, i = q - t * n;
+        const LT *W = A + i * lda + k;
+        LT a = in_panel(i) ? (LT)0 : A[i * lda + k2 + t];
+#pragma unroll
+        for (int u = 0; u < PB; ++u)
+          if (u < pw) a += W[u] * R[u * n + k2 + t];
+        A[i * lda + k2 + t] = a;
       }
       __syncthreads();
-      break;
     }
-    // ---- C: candidates for the second pivot
-    const LT r1k1 = r1b[k + 1];
-    {
-      double ca = -1.0, cv = 0.0, cf = 0.0;
-      int ci = n;
-      for (int i = k + 1 + tid; i < n; i += nt) {
-        const LT f = A[i * lda + k];
-        track(ca, ci, cv, cf, (double)(A[i * lda + k + 1] - f * r1k1), i, (double)f);
+    const bool ahead = pw2 > 0;
+    if (ahead && w == 0 && panel_warp<LT, NC, PB>(A, lda, n, k2, pw2, s.perm, used)) s.perm[n] = 1;
+    if (!ahead || w > 0 || nw == 1) {  // the remaining columns, three 32-wide chunks at a time
+      const int i0 = (ahead && nw > 1) ? w - 1 : w, di = (ahead && nw > 1) ? nw - 1 : nw;
+      constexpr int CH = NC < 3 ? NC : 3;
+      for (int c0 = 0; c0 < NC; c0 += CH) {
+        LT r[PB][CH];
+        bool on[CH];
+#pragma unroll
+        for (int t = 0; t < CH; ++t) {
+          const int j = lane + 32 * (c0 + t);
+          on[t] = j < n && (j < k || j >= k2 + pw2);
+#pragma unroll
+          for (int u = 0; u < PB; ++u) r[u][t] = (on[t] && u < pw) ? R[u * n + j] : (LT)0;
+        }
+#pragma unroll 2
+        for (int i = i0; i < n; i += di) {
+          LT *row = A + i * lda;
+          // (the pivots of the next panel may be noted meanwhile, in entries
+          // that this test reads as outside [k, k2))
+          const bool piv = in_panel(i);
+          LT a[CH], wv[PB];
+#pragma unroll
+          for (int u = 0; u < PB; ++u) wv[u] = u < pw ? row[k + u] : (LT)0;
+#pragma unroll
+          for (int t = 0; t < CH; ++t) a[t] = (on[t] && !piv) ? row[lane + 32 * (c0 + t)] : (LT)0;
+#pragma unroll
+          for (int u = 0; u < PB; ++u)
+#pragma unroll
+            for (int t = 0; t < CH; ++t) a[t] += wv[u] * r[u][t];
+#pragma unroll
+          for (int t = 0; t < CH; ++t)
+            if (on[t]) row[lane + 32 * (c0 + t)] = a[t];
+        }
       }
-      publish(ca, ci, cv, cf);
     }
     __syncthreads();
-    // ---- S2: second pivot, from the raw row
-    double pv2, f2d;
-    const int p2 = pick(pv2, f2d);
-    if (p2 < 0) {
-      bad = 1;
-      break;
-    }
-    const LT pinv2 = (LT)1 / (LT)pv2, f2 = (LT)f2d;
-    if (tid == 0) {
-      const int t = s.perm[k + 1];
-      s.perm[k + 1] = s.perm[p2];
-      s.perm[p2] = t;
-    }
-    for (int j = tid; j < n; j += nt) {
-      const LT a = A[(k + 1) * lda + j], b = A[p2 * lda + j];
-      A[p2 * lda + j] = a;
-      const LT ap = (j == k ? (LT)0 : b) - f2 * r1b[j];
-      const LT r2 = (j == k + 1 ? (LT)1 : ap) * pinv2;
-      A[(k + 1) * lda + j] = r2;
-      A[k * lda + j] = (j == k + 1 ? (LT)0 : r1b[j]) - r1k1 * r2;
-    }
-    __syncthreads();
-    // ---- U: every other row in one pass
-    LT r1v[NC], r2v[NC];
-#pragma unroll
-    for (int t = 0; t < NC; ++t) {
-      const int j = lane + 32 * t;
-      const bool jv = t < NC - 1 || j < n;
-      r1v[t] = (jv && j != k + 1) ? r1b[j] : (LT)0;
-      r2v[t] = jv ? A[(k + 1) * lda + j] : (LT)0;
-    }
-    const LT r1kk = r1b[k], r2k = A[(k + 1) * lda + k], r2k1 = A[(k + 1) * lda + k + 1];
-    const int ck = k & 31, ck1 = (k + 1) & 31, t2 = (k + 2) >> 5, c2 = (k + 2) & 31;
-    double ca = -1.0, cv = 0.0, cf = 0.0;
-    int ci = n;
-    for (int i0 = w; i0 < n; i0 += 2 * nw) {
-      const int i1 = i0 + nw;
-      const bool in1 = i1 < n;
-      const bool u0 = i0 != k && i0 != k + 1, u1 = in1 && i1 != k && i1 != k + 1;
-      const LT f0 = u0 ? A[i0 * lda + k] : (LT)0, f1 = u1 ? A[i1 * lda + k] : (LT)0;
-      const LT g0 = u0 ? A[i0 * lda + k + 1] - f0 * r1k1 : (LT)0;
-      const LT g1 = u1 ? A[i1 * lda + k + 1] - f1 * r1k1 : (LT)0;
-      LT a0[NC], a1[NC];
-#pragma unroll
-      for (int t = 0; t < NC; ++t) {
-        const int j = lane + 32 * t;
-        const bool jv = t < NC - 1 || j < n;
-        a0[t] = jv ? A[i0 * lda + j] : (LT)0;
-        a1[t] = (jv && in1) ? A[i1 * lda + j] : (LT)0;
-      }
-      __syncwarp();
-      const bool s0 = f0 != (LT)0 || g0 != (LT)0, s1 = f1 != (LT)0 || g1 != (LT)0;
-#pragma unroll
-      for (int t = 0; t < NC; ++t) {
-        const int j = lane + 32 * t;
-        const bool jv = t < NC - 1 || j < n;
-        a0[t] = a0[t] - f0 * r1v[t] - g0 * r2v[t];
-        a1[t] = a1[t] - f1 * r1v[t] - g1 * r2v[t];
-        if (jv && s0) A[i0 * lda + j] = a0[t];
-        if (jv && s1) A[i1 * lda + j] = a1[t];
-      }
-      if (lane == ck) {  // Gauss-Jordan values of the eliminated columns
-        if (s0) A[i0 * lda + k] = -f0 * r1kk - g0 * r2k;
-        if (s1) A[i1 * lda + k] = -f1 * r1kk - g1 * r2k;
-      }
-      if (lane == ck1) {
-        if (s0) A[i0 * lda + k + 1] = -g0 * r2k1;
-        if (s1) A[i1 * lda + k + 1] = -g1 * r2k1;
-      }
-      if (lane == c2 && k + 2 < n) {  // candidates for column k + 2
-        LT v0 = a0[0], v1 = a1[0];
-#pragma unroll
-        for (int t = 1; t < NC; ++t)
-          if (t == t2) {
-            v0 = a0[t];
-            v1 = a1[t];
-          }
-        if (i0 >= k + 2) track(ca, ci, cv, cf, (double)v0, i0, 0.0);
-        if (in1 && i1 >= k + 2) track(ca, ci, cv, cf, (double)v1, i1, 0.0);
-      }
-    }
-    publish(ca, ci, cv, cf);
-    __syncthreads();
-    k += 2;
   }
-  return __syncthreads_or(bad);
+  return __syncthreads_or(s.perm[n]);
 }
 
 // invert_cta for the register-chunk count nc = ceil(n / 32) (1..8).
 template <class LT>
 __device__ __forceinline__ int invert_any(int nc, const DevMech &m, const Smem &s, const double *J,
                                           double c, int n, int lda) {
+  constexpr bool F64 = sizeof(LT) == 8;
   switch (nc) {
-    case 1: return invert_cta<LT, 1>(m, s, J, c, n, lda);
-    case 2: return invert_cta<LT, 2>(m, s, J, c, n, lda);
-    case 3: return invert_cta<LT, 3>(m, s, J, c, n, lda);
-    case 4: return invert_cta<LT, 4>(m, s, J, c, n, lda);
-    case 5: return invert_cta<LT, 5>(m, s, J, c, n, lda);
-    case 6: return invert_cta<LT, 6>(m, s, J, c, n, lda);
-    case 7: return invert_cta<LT, 7>(m, s, J, c, n, lda);
-    default: return invert_cta<LT, 8>(m, s, J, c, n, lda);
+    case 1: return invert_cta<LT, 1, 8>(m, s, J, c, n, lda);
+    case 2: return invert_cta<LT, 2, 8>(m, s, J, c, n, lda);
+    case 3: return invert_cta<LT, 3, 8>(m, s, J, c, n, lda);
+    case 4: return invert_cta<LT, 4, 8>(m, s, J, c, n, lda);
+    case 5:
+    case 6: return invert_cta<LT, 6, F64 ? 6 : 8>(m, s, J, c, n, lda);
+    default: return invert_cta<LT, 8, F64 ? 4 : 8>(m, s, J, c, n, lda);
   }
 }
 
-// x = (I - c_lu J)^{-1} b with the stored inverse: x = W A (perm of W^-1 b).
-// Thread per row, four independent partial sums to hide the FMA latency.
+// x = (I - c_lu J)^{-1} b with the stored inverse: x = W A (pivot order of
+// W^-1 b), the rows of A in pivot order.  Eight lanes a row, each a contiguous
+// share of its columns, and up to three rows a thread that share every
+// right-hand-side load; a share of 2 (mod 4) columns and the odd row stride
+// put the lanes of two neighbouring rows in different banks.
 template <class LT>
 __device__ void apply_inverse(const Smem &s, int n, int lda, const double *b, double *x) {
   const LT *A = (const LT *)s.A;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int pi = s.perm[i];
+    const int pi = pivot_row(s.perm, i);
     s.bs[i] = b[pi] / s.wlu[pi];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const LT *row = A + (size_t)i * lda;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    int j = 0;
-    for (; j + 3 < n; j += 4) {
-      a0 += (double)row[j] * s.bs[j];
-      a1 += (double)row[j + 1] * s.bs[j + 1];
-      a2 += (double)row[j + 2] * s.bs[j + 2];
-      a3 += (double)row[j + 3] * s.bs[j + 3];
+  int share = (n + 7) >> 3;
+  share += (6 - (share & 3)) & 3;  // the next 2 (mod 4)
+  const int g = threadIdx.x & 7, nr = blockDim.x >> 3;
+  const int j0 = min(n, g * share), j1 = min(n, j0 + share);
+  // every lane of a warp runs the same trips, for the shuffles
+  for (int p0 = threadIdx.x >> 3; p0 - ((threadIdx.x & 31) >> 3) < n; p0 += 3 * nr) {
+    const int p[3] = {p0, p0 + nr, p0 + 2 * nr};
+    double acc[3] = {0.0, 0.0, 0.0};
+    const LT *row[3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) row[e] = A + min(p[e], n - 1) * lda;
+#pragma unroll 2
+    for (int j = j0; j < j1; ++j) {
+      const double v = s.bs[j];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) acc[e] += (double)row[e][j] * v;
     }
-    for (; j < n; ++j) a0 += (double)row[j] * s.bs[j];
-    x[i] = ((a0 + a1) + (a2 + a3)) * s.wlu[i];
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+      for (int e = 0; e < 3; ++e) acc[e] += __shfl_xor_sync(kFull, acc[e], o);
+    if (g == 0)
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+        if (p[e] < n) {
+          const int k = pivot_col(s.perm, p[e]);
+          x[k] = acc[e] * s.wlu[k];
+        }
   }
   __syncthreads();
 }
@@ -519,31 +502,45 @@ __device__ void rank1_fix(const Smem &s, int n, double r1k, double *x) {
   __syncthreads();
 }
 
-__device__ void change_D_cta(double *D, int n, int order, double fac) {
-  double R[kMaxOrder + 1][kMaxOrder + 1], U[kMaxOrder + 1][kMaxOrder + 1];
-  for (int pass = 0; pass < 2; ++pass) {
-    const double f = pass == 0 ? fac : 1.0;
-    double (*A)[kMaxOrder + 1] = pass == 0 ? R : U;
-    for (int j = 0; j <= order; ++j) {
-      A[0][j] = 1.0;
-      for (int i = 1; i <= order; ++i) A[i][j] = A[i - 1][j] * (j == 0 ? 0.0 : (i - 1 - f * j) / i);
+// (-1)^k binomial(j, k), [k][j]: the difference transform of a unit step
+// ratio (Shampine and Reichelt's U).
+__device__ const double kSignedBinom[kMaxOrder + 1][kMaxOrder + 1] = {
+    {1, 1, 1, 1, 1, 1},   {0, -1, -2, -3, -4, -5}, {0, 0, 1, 3, 6, 10},
+    {0, 0, 0, -1, -4, -10}, {0, 0, 0, 0, 1, 5},      {0, 0, 0, 0, 0, -1}};
+
+// Differences of the history for the step size h fac: D <- (R(fac) U)^T D.  A
+// thread forms one entry of R U in registers (every thread forming the whole
+// product in local arrays took 47 K cycles a call, 2 K now) into mat, 36
+// doubles of shared memory.
+__device__ void change_D_cta(double *D, int n, int order, double fac, double *mat) {
+  constexpr int M = kMaxOrder + 1;
+  const double inv[M] = {0.0, 1.0, 0.5, 1.0 / 3.0, 0.25, 0.2};
+  __syncthreads();  // mat may still be read, D written
+  for (int q = threadIdx.x; q < M * M; q += blockDim.x) {
+    const int i = q / M, j = q - i * M;
+    double ru = 0.0;
+#pragma unroll
+    for (int k = 0; k < M; ++k) {
+      double r = (k > 0 || i == 0) ? 1.0 : 0.0;
+#pragma unroll
+      for (int t = 1; t < M; ++t)
+        if (k > 0 && t <= i) r *= (t - 1 - fac * k) * inv[t];
+      ru += r * kSignedBinom[k][j];
     }
+    mat[q] = ru;
   }
-  double RU[kMaxOrder + 1][kMaxOrder + 1];
-  for (int i = 0; i <= order; ++i)
-    for (int j = 0; j <= order; ++j) {
-      double t = 0.0;
-      for (int k = 0; k <= order; ++k) t += R[i][k] * U[k][j];
-      RU[i][j] = t;
-    }
   __syncthreads();
   for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    double old[kMaxOrder + 1];
-    for (int k = 0; k <= order; ++k) old[k] = D[k * n + c];
-    for (int i = 0; i <= order; ++i) {
+    double old[M];
+#pragma unroll
+    for (int k = 0; k < M; ++k) old[k] = k <= order ? D[k * n + c] : 0.0;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
       double t = 0.0;
-      for (int k = 0; k <= order; ++k) t += RU[k][i] * old[k];
-      D[i * n + c] = t;
+#pragma unroll
+      for (int k = 0; k < M; ++k)
+        if (k <= order) t += mat[k * M + i] * old[k];
+      if (i <= order) D[i * n + c] = t;
     }
   }
   __syncthreads();
@@ -832,11 +829,11 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
     int nef = 0, ncf = 0;  // this step's error-test and convergence failures
     while (!accepted) {
       if (h > o.max_dt) {
-        change_D_cta(s.D, n, q, o.max_dt / h);
+        change_D_cta(s.D, n, q, o.max_dt / h, s.red + 64);
         h = o.max_dt;
       }
       if (t + h > t_end) {
-        change_D_cta(s.D, n, q, (t_end - t) / h);
+        change_D_cta(s.D, n, q, (t_end - t) / h, s.red + 64);
         h = t_end - t;
       }
       if (!(t + h > t)) { rc = -5; goto failed; }
@@ -937,7 +934,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
           continue;
         }
         if (++ncf >= kMaxConvFails) { rc = -8; goto failed; }
-        change_D_cta(s.D, n, q, 0.5);
+        change_D_cta(s.D, n, q, 0.5, s.red + 64);
         h *= 0.5;
         st.nrej++;
         continue;
@@ -957,7 +954,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
         if (nef > kErrFailsBeforeCut) {  // order and step cut (integrator.h)
           if (q > 1) {
             --q;
-            change_D_cta(s.D, n, q, kEtaMinErrFail);
+            change_D_cta(s.D, n, q, kEtaMinErrFail, s.red + 64);
           } else {
             st.nrhs++;
             if (rhs_cta(m, o, s, v, t_off + t, s.D, s.tmp, false, nullptr)) { rc = -6; goto failed; }
@@ -969,7 +966,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
           continue;
         }
         const double fac = fmax(kMinFactor, safety * pow(err_norm, -1.0 / (q + 1)));
-        change_D_cta(s.D, n, q, fac);
+        change_D_cta(s.D, n, q, fac, s.red + 64);
         h *= fac;
         continue;
       }
@@ -1041,7 +1038,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
     q += dq;
     double fac = fmin(kMaxFactor, safety * best);
     if (fac < kEtaKeep) fac = 1.0;
-    change_D_cta(s.D, n, q, fac);
+    change_D_cta(s.D, n, q, fac, s.red + 64);
     h *= fac;
     neq = 0;
   }
@@ -1067,9 +1064,18 @@ __global__ void __launch_bounds__(512, 1) integrate_dense_kernel(DevMech m, Inte
   double *p = smem_dyn;
   double *g = a.rop_scratch + (size_t)blockIdx.x * ((size_t)N + (kMaxOrder + 6) * (size_t)n);
   s.red = p; p += 128;
+  // pivot rows of the inversion over what is dead during one: the rates
+  // workspace and six vectors, 3 S + 6 n >= kPanelMax n doubles
+  s.rows = p;
   s.C = p; p += S;
   s.G = p; p += S;
   s.U = p; p += S;
+  s.f = p; p += n;
+  s.f0 = p; p += n;
+  s.tmp = p; p += n;
+  s.yp = p; p += n;
+  s.colk = p; p += n;
+  s.bs = p; p += n;
   if (spill & 1) { s.ROP = g; } else { s.ROP = p; p += N; }
   if (spill & 2) { s.D = g + N; } else { s.D = p; p += (kMaxOrder + 3) * n; }
   s.Jsm = nullptr;
@@ -1079,17 +1085,11 @@ __global__ void __launch_bounds__(512, 1) integrate_dense_kernel(DevMech m, Inte
   s.r1d = s.r1g + n;
   s.r1w = s.r1d + n;
   s.y = p; p += n;
-  s.f = p; p += n;
-  s.f0 = p; p += n;
   s.ypred = p; p += n;
   s.psi = p; p += n;
   s.d = p; p += n;
   s.scale = p; p += n;
-  s.tmp = p; p += n;
-  s.yp = p; p += n;
-  s.colk = p; p += n;
   s.wlu = p; p += n;
-  s.bs = p; p += n;
   s.V = nullptr;
   if (sizeof(LT) == sizeof(float)) {
     s.V = p;

@@ -54,6 +54,7 @@ struct GroupKArgs {
   double *slots;     // one slot of slot_stride doubles per group position
   long slot_stride;
   int lda;
+  int ws_doubles;    // shared memory of the reduction slots and the rates workspace
   double *part;      // [n_group][kPart]
   const double *T, *P, *Y, *ysrc, *dpdt, *tdel_in;
 };
@@ -74,6 +75,7 @@ __device__ Bound bind(const GroupKArgs &k, double *smem) {
   double *p = smem;
   Smem &s = b.s;
   s.red = p; p += 128;
+  s.rows = p;  // the inversion's pivot rows over the rates workspace
   s.C = p; p += S;
   s.G = p; p += S;
   s.U = p; p += S;
@@ -121,12 +123,12 @@ __device__ __forceinline__ double atol_of(const DevMech &m, const IntegOpts &o, 
 __device__ void apply_inverse_g(const Smem &s, int n, int lda, const double *A, const double *b, double *x) {
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
   for (int i = tid; i < n; i += nt) {
-    const int pi = s.perm[i];
+    const int pi = pivot_row(s.perm, i);
     s.bs[i] = b[pi] / s.wlu[pi];
   }
   __syncthreads();
   for (int i = w; i < n; i += nw) {
-    const double *row = A + (size_t)i * lda;
+    const double *row = A + (size_t)pivot_row(s.perm, i) * lda;
     double acc = 0.0;
     for (int j = lane; j < n; j += 32) acc += row[j] * s.bs[j];
 #pragma unroll
@@ -247,14 +249,14 @@ __global__ void __launch_bounds__(512) grp_start(GroupKArgs k, double t_off, dou
   }
   __syncthreads();
   int bad = jac_cta(k.m, k.o, s, b.hdr[0], t_off, s.y, s.f0, b.J);
-  if (!bad) bad = factor_g(k, b, c, fac_smem ? smem + 128 + 3 * k.m.nsp + k.m.nstep : nullptr);
+  if (!bad) bad = factor_g(k, b, c, fac_smem ? smem + k.ws_doubles : nullptr);
   put_part(k, 4, bad ? 1.0 : 0.0);
 }
 
 __global__ void __launch_bounds__(512) grp_change(GroupKArgs k, int q, double fac) {
   extern __shared__ double smem[];
   Bound b = bind(k, smem);
-  change_D_cta(b.s.D, k.m.nsp + 1, q, fac);
+  change_D_cta(b.s.D, k.m.nsp + 1, q, fac, b.s.red + 64);
 }
 
 // Predictor of a step of order q: ypred = sum D_k, psi, error weights.
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(512) grp_factor(GroupKArgs k, double t_abs, do
     bad = rhs_cta(k.m, k.o, s, b.hdr[0], t_abs, s.ypred, s.f0, false, nullptr);
     if (!bad) bad = jac_cta(k.m, k.o, s, b.hdr[0], t_abs, s.ypred, s.f0, b.J);
   }
-  if (!bad) bad = factor_g(k, b, c, fac_smem ? smem + 128 + 3 * k.m.nsp + k.m.nstep : nullptr);
+  if (!bad) bad = factor_g(k, b, c, fac_smem ? smem + k.ws_doubles : nullptr);
   put_part(k, 4, bad ? 1.0 : 0.0);
 }
 
@@ -664,7 +666,10 @@ cudaError_t integrate_group(const DevMech &m, const IntegOpts &o, const IntegArg
   drv.st = stream;
   drv.part_h = part_host;
   make_consts(drv.bc);
-  drv.smem = (128 + 3 * (size_t)S + m.nstep) * sizeof(double);
+  // reduction slots, then the rates workspace or the inversion's pivot rows
+  const size_t ws = std::max(3 * (size_t)S + m.nstep, (size_t)kPanelMax * n);
+  drv.k.ws_doubles = (int)(128 + ws);
+  drv.smem = (128 + ws) * sizeof(double);
   const size_t kSmemMax = 227 * 1024;
   drv.smem_fac = drv.smem + (size_t)n * lda * sizeof(double);
   drv.fac_smem = drv.smem_fac <= kSmemMax ? 1 : 0;
