@@ -110,6 +110,12 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     sc_step.insert(sc_step.end(), sc[j].begin(), sc[j].end());
     sc_ptr.push_back((int)sc_step.size());
   }
+  std::vector<int> sn_ptr(1, 0), sn_step;
+  for (int j = 0; j < ns; ++j) {
+    for (int st : sd[j]) sn_step.push_back((int)(st | 0x80000000u));
+    sn_step.insert(sn_step.end(), sc[j].begin(), sc[j].end());
+    sn_ptr.push_back((int)sn_step.size());
+  }
   // Jacobian per-nonzero gather lists, in term-list order
   // (reactor_nvector_serial.cpp:659-673: all destruction terms, then creation)
   std::vector<std::vector<int>> nzd(p.nnz), nzc(p.nnz);
@@ -126,12 +132,13 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   // flat species-column list for the rates kernel's Jacobian phase
   std::vector<int2> jw;
   std::vector<unsigned short> jt;
-  std::vector<int> jt_ptr(1, 0), jcost(1, 0), jf_ptr(1, 0);
+  std::vector<int> jt_ptr(1, 0), jcost(1, 0), jf_ptr(1, 0), jf_col;
   for (int j = 0; j < ns; ++j) {
     for (int k = p.col_ptr[j]; k < p.col_ptr[j + 1] - 1; ++k) {  // the last entry is the T row
       const int nd = nzd_ptr[k + 1] - nzd_ptr[k], nc = nzc_ptr[k + 1] - nzc_ptr[k];
       if (nd > 0xffff || nc > 0xffff || t.nstep > 0xffff)
         throw std::runtime_error("mechanism too large for 16-bit Jacobian term lists");
+      jf_col.push_back(j);
       jw.push_back(make_int2(p.row_idx[k], nd | (nc << 16)));
       for (int q = nzd_ptr[k]; q < nzd_ptr[k + 1]; ++q) jt.push_back((unsigned short)nzd_step[q]);
       for (int q = nzc_ptr[k]; q < nzc_ptr[k + 1]; ++q) jt.push_back((unsigned short)nzc_step[q]);
@@ -189,6 +196,19 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   // the kernel may stage [blob, blob + hot_bytes) in shared memory.
   std::vector<RxnRec> rec_by_cost;
   for (int p : rxn_order) rec_by_cost.push_back(rec[p]);
+  std::vector<RxnRec> slots;
+  for (int kind = 0; kind < 4; ++kind) {
+    for (int p : rxn_order) {
+      const int fl = rec[p].flags;
+      if (((fl & kPlog) ? 0 : (fl & kFalloff) ? 1 : (fl & kThirdBody) ? 2 : 3) == kind) slots.push_back(rec[p]);
+    }
+    while (slots.size() % 32) {
+      RxnRec none;
+      std::memset(&none, 0, sizeof(none));
+      none.flags = kNoRxn;
+      slots.push_back(none);
+    }
+  }
   Blob b;
   const size_t h = 16;
   size_t o_rbc = b.add(rec_by_cost, h);
@@ -207,7 +227,9 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   size_t o_jw = b.add(jw, h), o_jt = b.add(jt, h), o_jtp = b.add(jt_ptr, h), o_jc = b.add(jcost, h),
          o_jf = b.add(jf_ptr, h);
   const size_t hot = (b.bytes.size() + 15) & ~size_t(15);
-  size_t o_rec = b.add(rec);
+  size_t o_rec = b.add(rec), o_slot = b.add(slots);
+  size_t o_jfc = b.add(jf_col);
+  size_t o_snp = b.add(sn_ptr), o_sns = b.add(sn_step);
   size_t o_lr = b.add(p.last_row);
   size_t o_ndp = b.add(nzd_ptr), o_nds = b.add(nzd_step), o_ncp = b.add(nzc_ptr), o_ncs = b.add(nzc_step);
   size_t o_jrp = b.add(jr_ptr), o_jrk = b.add(jr_kk), o_jrc = b.add(jr_col);
@@ -249,6 +271,8 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.sd_step = (const int *)P(o_sds);
   view_.sc_ptr = (const int *)P(o_scp);
   view_.sc_step = (const int *)P(o_scs);
+  view_.sn_ptr = (const int *)P(o_snp);
+  view_.sn_step = (const int *)P(o_sns);
   view_.col_ptr = (const int *)P(o_cp);
   view_.row_idx = (const int *)P(o_ri);
   view_.last_row = (const int *)P(o_lr);
@@ -262,6 +286,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.jt_ptr = (const int *)P(o_jtp);
   view_.jcost = (const int *)P(o_jc);
   view_.jf_ptr = (const int *)P(o_jf);
+  view_.jf_col = (const int *)P(o_jfc);
   view_.jr_ptr = (const int *)P(o_jrp);
   view_.jr_kk = (const int *)P(o_jrk);
   view_.jr_col = (const int *)P(o_jrc);
@@ -270,6 +295,8 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.spc_order = (const int *)P(o_so);
   view_.col_order = (const int *)P(o_co);
   view_.rxn_by_cost = (const RxnRec *)P(o_rbc);
+  view_.rxn_slots = (const RxnRec *)P(o_slot);
+  view_.nblocks = (int)(slots.size() / 32);
 }
 
 DeviceMechanism::~DeviceMechanism() {

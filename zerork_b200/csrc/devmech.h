@@ -26,6 +26,7 @@ enum RxnFlags : int {
   kThirdBody = 4,
   kFalloff = 8,
   kPlog = 16,        // forward rate from the PLOG table (aux: PLOG index)
+  kNoRxn = 32,       // padding of rxn_slots: no reaction
 };
 
 struct alignas(16) RxnRec {
@@ -54,6 +55,8 @@ struct DevMech {
   const double *plog_p, *plog_lnp, *plog_lnA, *plog_sgn, *plog_n, *plog_Ta;
   // species production gather lists (step indices in ascending step order)
   const int *sd_ptr, *sd_step, *sc_ptr, *sc_step;
+  // both lists of a species in one: step | 1 << 31 for a destruction term
+  const int *sn_ptr, *sn_step;
   // Jacobian pattern and per-nonzero gather lists
   const int *col_ptr, *row_idx, *last_row;
   const int *nzd_ptr, *nzd_step, *nzc_ptr, *nzc_step;
@@ -68,6 +71,7 @@ struct DevMech {
   const int2 *jw;
   const unsigned short *jt;
   const int *jt_ptr, *jcost, *jf_ptr;
+  const int *jf_col;  // column of each item
   // row-wise view of the Jacobian pattern: row i has entries jr_kk[p] (index
   // into the compressed-column values) in columns jr_col[p], p in
   // [jr_ptr[i], jr_ptr[i+1])
@@ -80,6 +84,12 @@ struct DevMech {
   // the reaction records in rxn_order order (position p holds reaction
   // rxn_order[p]): one load instead of two dependent ones per work item
   const RxnRec *rxn_by_cost;
+  // The same records for one reactor per CTA, a reaction a lane: grouped by
+  // kind (PLOG, falloff, third body, the rest) in blocks of 32 of one kind,
+  // padded with kNoRxn records, so that a warp runs one kind's code and the
+  // long falloff chains run beside the others instead of after them.
+  const RxnRec *rxn_slots;
+  int nblocks;
   // The tables the rates kernel reads form the first hot_bytes bytes of the
   // allocation at base (16-byte aligned), so a CTA can stage them in shared
   // memory and address them at a fixed offset from their global copies.

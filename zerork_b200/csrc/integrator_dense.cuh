@@ -31,7 +31,7 @@ constexpr int kPanelMax = 8;  // widest panel of the inversion
 constexpr int kPredBuf = 256;  // widest predictor layer (padded)
 
 struct Smem {
-  double *red;  // 128 slots: block sums [0, 33); the inversion keeps the pivot columns here
+  double *red;  // 128 slots: block sums [0, 16), the right-hand side's [16, 64), change_D [64, 100)
   double *C, *G, *U, *ROP;
   double *D, *y, *f, *f0, *ypred, *psi, *d, *scale, *tmp, *yp;
   void *A;      // n x lda inverse (LT)
@@ -57,35 +57,28 @@ struct RhsOut {
   double cx, T, v;
 };
 
-// Sum over the CTA; every thread gets thread 0's total (deterministic).
-__device__ __forceinline__ double block_sum(double v, double *red) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Sum over the CTA; every thread gets the same total (deterministic: warp
+// trees, then the warps' sums in four chains).  The slots belong to one call
+// site: between two uses of them every thread passes another barrier after
+// its reads, so one barrier suffices.
+__device__ __forceinline__ double block_sum_at(double v, double *slots) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  if (lane == 0) slots[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < nw; ++i) s += red[i];
-    red[32] = s;
-  }
-  __syncthreads();
-  return red[32];
+  if (nw == 1) return v;
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    if (i < nw) a[i & 3] += slots[i];
+  return (a[0] + a[1]) + (a[2] + a[3]);
 }
 
-__device__ __forceinline__ double gather4(const double *v, const int *idx, int q0, int q1) {
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-  int q = q0;
-  for (; q + 3 < q1; q += 4) {
-    const int i0 = idx[q], i1 = idx[q + 1], i2 = idx[q + 2], i3 = idx[q + 3];
-    a0 += v[i0];
-    a1 += v[i1];
-    a2 += v[i2];
-    a3 += v[i3];
-  }
-  for (; q < q1; ++q) a0 += v[idx[q]];
-  return (a0 + a1) + (a2 + a3);
+// The same with slots that any call may have used last.
+__device__ __forceinline__ double block_sum(double v, double *red) {
+  __syncthreads();
+  return block_sum_at(v, red);
 }
 
 // Source / constant-pressure adjustment of T and v (reactor_src.cuh).
@@ -112,7 +105,13 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
   double v = v0;
   if (o.cp || s.src.dpdt != 0.0 || s.src.esrc != 0.0)
     source_cta(m, o, s, t, y, clamp, v0, T_force, T, v);
-  const double logT = log(T), invT = 1.0 / T, lprt = log(kPatmD / (kRuD * T));
+  // this warp's first block of reactions: its records arrive during the
+  // species pass
+  const int lane = tid & 31, w = tid >> 5, nw = nt >> 5;
+  RxnRec R;
+  R.flags = kNoRxn;
+  if (w < m.nblocks) R = load_rxn(m.rxn_slots + w * 32 + lane);
+  const double logT = log(T), invT = 1.0 / T, lprt = kLnPatmRu - logT;
   const double dens = 1.0 / v;
   const double ush = o.cp ? 0.0 : 1.0;  // h/RT - 1 = u/RT; c_p/R - 1 = c_v/R
   double pc = 0.0, pcv = 0.0;
@@ -128,33 +127,52 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
     pc += c;
     pcv += ((cp - ush) * m.ru_inv_mw[k]) * ys;
   }
-  const double Csum = block_sum(pc, s.red);
-  const double cv = block_sum(pcv, s.red);
-  // reactions by decreasing cost in snake order over the threads
-  for (int rr = 0; rr * nt < m.nrxn; ++rr) {
-    const int pos = rr * nt + ((rr & 1) ? nt - 1 - tid : tid);
-    if (pos < m.nrxn)
-      reaction_item<1, 1>(m, load_rxn(m.rxn_by_cost + pos), 0, s.C, s.G, s.ROP, &T, &logT, &invT, &lprt, &Csum,
-                          o.lim);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) pcv += __shfl_xor_sync(kFull, pcv, off);
+  if (lane == 0) s.red[32 + w] = pcv;  // read after the barrier of the next sum
+  const double Csum = block_sum_at(pc, s.red + 16);
+  // blocks of reactions in snake order over the warps
+  for (int rr = 0; rr * nw < m.nblocks; ++rr) {
+    const RxnRec cur = R;
+    const int nb = (rr + 1) * nw + ((rr & 1) ? w : nw - 1 - w);
+    R.flags = kNoRxn;
+    if (nb < m.nblocks) R = load_rxn(m.rxn_slots + nb * 32 + lane);
+    if (!(cur.flags & kNoRxn))
+      reaction_item<1, 1>(m, cur, 0, s.C, s.G, s.ROP, &T, &logT, &invT, &lprt, &Csum, o.lim);
   }
+  double cv = 0.0;
+  for (int i = 0; i < nw; ++i) cv += s.red[32 + i];
   __syncthreads();
+  // net production rates: eight lanes a species, the longest lists first (a
+  // thread a species walked lists of hundreds of steps with the index loads
+  // in its chain)
   double pe = 0.0;
-  for (int k = tid; k < S; k += nt) {
-    // four independent partial sums per list keep several rate loads in
-    // flight (the rates of progress may sit in L2)
-    const double des = gather4(s.ROP, m.sd_step, m.sd_ptr[k], m.sd_ptr[k + 1]);
-    const double cre = gather4(s.ROP, m.sc_step, m.sc_ptr[k], m.sc_ptr[k + 1]);
-    const double net = cre - des;
-    if (s.ysrc) {  // reactor_constant_volume_cpu.cpp:108-113
-      const double ys = s.ysrc[k];
-      ydot[k] = net * m.mw[k] * v + ys;
-      pe += s.U[k] * (net * v + ys * m.inv_mw[k]);
-    } else {
-      ydot[k] = net * m.mw[k] * v;
-      pe += s.U[k] * net * v;
+  for (int p0 = tid >> 3; p0 - (lane >> 3) < S; p0 += nt >> 3) {
+    const int k = p0 < S ? m.spc_order[p0] : -1;
+    double net = 0.0;
+    if (k >= 0) {
+      const int e1 = m.sn_ptr[k + 1];
+#pragma unroll 4
+      for (int e = m.sn_ptr[k] + (lane & 7); e < e1; e += 8) {
+        const int st = m.sn_step[e];
+        const double r = s.ROP[st & 0x7fffffff];
+        net += st < 0 ? -r : r;
+      }
+    }
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) net += __shfl_xor_sync(kFull, net, off);
+    if (k >= 0 && (lane & 7) == 0) {
+      if (s.ysrc) {  // reactor_constant_volume_cpu.cpp:108-113
+        const double ys = s.ysrc[k];
+        ydot[k] = net * m.mw[k] * v + ys;
+        pe += s.U[k] * (net * v + ys * m.inv_mw[k]);
+      } else {
+        ydot[k] = net * m.mw[k] * v;
+        pe += s.U[k] * net * v;
+      }
     }
   }
-  const double es = block_sum(pe, s.red);
+  const double es = block_sum_at(pe, s.red + 48);
   if (tid == 0)
     ydot[S] = s.src.fixT ? 0.0 : -es * kRuD * yS / cv + (s.src.esrc + s.src.dpdt * v) / (cv * o.Tref);
   if (out) *out = RhsOut{cv, T, v};
@@ -185,25 +203,43 @@ __device__ __noinline__ int jac_cta(const DevMech &m, const IntegOpts &o, const 
   const double multFact = -1.0 / ro.cx;
   const double T = ro.T, v = o.cp ? ro.v : v0;
   const double ush = o.cp ? 0.0 : 1.0;
-  for (int jj = tid; jj < S; jj += nt) {  // one column per thread, costliest first
-    const int j = m.col_order[jj];
-    const double t2 = m.mw[j] / clamp_mass_fraction(y[j], o.mmf) * v;
-    const int k0 = m.col_ptr[j], k1 = m.col_ptr[j + 1] - 1;
-    const double wcol = m.inv_mw[j];
-    double trow = 0.0;
-    for (int kk = k0; kk < k1; ++kk) {
-      const int row = m.row_idx[kk];
-      const double des = gather4(s.ROP, m.nzd_step, m.nzd_ptr[kk], m.nzd_ptr[kk + 1]);
-      const double cre = gather4(s.ROP, m.nzc_step, m.nzc_ptr[kk], m.nzc_ptr[kk + 1]);
-      const double val = (0.0 - des * t2) + cre * t2;
-      trow += val * s.U[row];
-      J[kk] = val * (m.mw[row] * wcol);
+  // species columns: a thread a nonzero (the flat item list of devmech.h), as
+  // P_ij = dF_i / dC_j; then the temperature row, eight lanes a column
+  for (int k = tid; k < S; k += nt) s.yp[k] = m.mw[k] / clamp_mass_fraction(y[k], o.mmf) * v;
+  __syncthreads();
+#pragma unroll 2
+  for (int f = tid; f < m.nj; f += nt) {
+    const int2 it = m.jw[f];
+    const unsigned short *st = m.jt + m.jt_ptr[f];
+    const int j = m.jf_col[f], nd = it.y & 0xffff, nt_ = nd + (it.y >> 16);
+    double des = 0.0, cre = 0.0;
+    for (int e = 0; e < nt_; ++e) {
+      const double r = s.ROP[st[e]];
+      if (e < nd) des += r;
+      else cre += r;
     }
-    const double cvj = (nasa_cp(m.thermo + 16 * j, T) - ush) * m.ru_inv_mw[j];
-    double tr = trow * RuTemp;
-    tr += TdC * cvj * m.mw[j];
-    tr *= wcol * multFact;
-    J[k1] = s.src.fixT ? 0.0 : tr;  // no temperature row when T is not solved
+    const double t2 = s.yp[j];
+    J[f + j] = ((0.0 - des * t2) + cre * t2) * (m.mw[it.x] * m.inv_mw[j]);
+  }
+  __syncthreads();
+  for (int j0 = tid >> 3; j0 - ((tid & 31) >> 3) < S; j0 += nt >> 3) {
+    const int j = min(j0, S - 1), k1 = m.col_ptr[j + 1] - 1;
+    double trow = 0.0;
+#pragma unroll 4
+    for (int kk = m.col_ptr[j] + (tid & 7); kk < k1; kk += 8) {
+      const int row = m.row_idx[kk];
+      trow += J[kk] * (m.inv_mw[row] * s.U[row]);
+    }
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) trow += __shfl_xor_sync(kFull, trow, off);
+    if (j0 < S && (tid & 7) == 0) {
+      const double wcol = m.inv_mw[j];
+      const double cvj = (nasa_cp(m.thermo + 16 * j, T) - ush) * m.ru_inv_mw[j];
+      double tr = trow * m.mw[j] * RuTemp;
+      tr += TdC * cvj * m.mw[j];
+      tr *= wcol * multFact;
+      J[k1] = s.src.fixT ? 0.0 : tr;  // no temperature row when T is not solved
+    }
   }
   __syncthreads();
   const double ySp = yS + yS * o.sqrt_ur;

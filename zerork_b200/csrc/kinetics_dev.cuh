@@ -12,6 +12,67 @@ namespace zrk {
 constexpr double kRuD = 8.314462618e3;  // src/zerork/constants.h:10
 constexpr double kPatmD = 1.01325e5;    // src/zerork/constants.h:12
 
+constexpr double kLnPatmRu = 2.50033668997960945;  // ln(kPatmD / kRuD)
+
+// exp(x) without branches, so that the calls of independent states and steps
+// interleave (the library's function ends in a branch, behind which the next
+// call's chain of some twenty dependent operations has to wait): Cody and
+// Waite's reduction by ln 2 in two parts (Software Manual for the Elementary
+// Functions, 1980), the Taylor polynomial of degree 13 on |r| <= ln 2 / 2
+// (remainder 4e-18) summed as a tree, and 2^n in two factors, which covers
+// overflow to infinity and gradual underflow.  NaN passes through.  Within one
+// ulp of the correctly rounded value (tests/test_exp_gpu.py).
+__device__ __forceinline__ double exp_tree(double x) {
+  x = x > 720.0 ? 720.0 : x;    // infinity from 710 on
+  x = x < -760.0 ? -760.0 : x;  // zero below -746
+  const double big = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
+  const double t = fma(x, 1.4426950408889634074, big), k = t - big;
+  const int n = __double2loint(t), n1 = n >> 1;
+  double r = fma(k, -0.69314718055994530942, x);
+  r = fma(k, -2.3190468138462995584e-17, r);  // ln 2 minus its nearest double
+  const double r2 = r * r, r4 = r2 * r2, r8 = r4 * r4;
+  const double a = fma(1.0 / 6.0, r, 0.5), b = fma(1.0 / 120.0, r, 1.0 / 24.0);
+  const double c = fma(1.0 / 5040.0, r, 1.0 / 720.0), d = fma(1.0 / 362880.0, r, 1.0 / 40320.0);
+  const double e = fma(1.0 / 39916800.0, r, 1.0 / 3628800.0), f = fma(1.0 / 6227020800.0, r, 1.0 / 479001600.0);
+  const double lo = fma(b, r2, a), mid = fma(d, r2, c), hi = fma(f, r2, e);
+  const double q = fma(hi, r8, fma(mid, r4, lo));
+  const double p = 1.0 + fma(r2, q, r);
+  return p * __hiloint2double((n1 + 1023) << 20, 0) * __hiloint2double((n - n1 + 1023) << 20, 0);
+}
+
+// q[i] = a[i] / d[i].  When every operand is well inside the range of
+// doubles: a reciprocal from the hardware's approximation by one cubic
+// iteration, and the quotient corrected by its residual (Markstein, IA-64 and
+// Elementary Functions, 2000), all K interleaved; otherwise the language's
+// division.
+__device__ __forceinline__ bool mid_range(double x) {
+  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 300u < 1440u;  // 2^-723 <= |x| < 2^717
+}
+template <int K>
+__device__ __forceinline__ void quotients(const double (&a)[K], const double (&d)[K], double (&q)[K]) {
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < K; ++i) ok = ok && mid_range(a[i]) && mid_range(d[i]);
+  if (ok) {
+    double y[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y[i]) : "d"(d[i]));
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const double e = fma(-d[i], y[i], 1.0);
+      y[i] = fma(y[i], fma(e, e, e), y[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const double g = a[i] * y[i];
+      q[i] = fma(fma(-d[i], g, a[i]), y[i], g);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < K; ++i) q[i] = a[i] / d[i];
+  }
+}
+
 // A mechanism table as the kernel reads it: its copy in the CTA's shared
 // memory when the kernel staged the hot tables (tab = the copy of the block
 // that starts at the global base), the global table itself for tab = null.
@@ -101,11 +162,57 @@ __device__ __forceinline__ RxnRec load_rxn(const RxnRec *p) {
   return R;
 }
 
+// Species sums and products of a reaction's side: sides of up to three
+// species without a loop, so their rows are read together.
+template <int V, int GS, class F>
+__device__ __forceinline__ void each_species(int count, const short *spc, F f) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (i < count) f(spc[i]);
+  if (count > 3) {
+#pragma unroll
+    for (int i = 3; i < kMaxSide; ++i)
+      if (i < count) f(spc[i]);
+  }
+}
+
+// Third-body concentration: Csum plus the efficiency list, four entries at a
+// time (the table loads are independent of the sums, which keep the list
+// order).
+template <int TS, int V>
+__device__ __forceinline__ void third_body(const int *__restrict__ spc, const double *__restrict__ alpha, int e0, int e1,
+                                           int q, const double *__restrict__ sC, const double *Csum, double *Cm) {
+  constexpr int GS = TS / V;
+#pragma unroll
+  for (int k = 0; k < V; ++k) Cm[k] = Csum[k];
+  int e = e0;
+  for (; e + 3 < e1; e += 4) {
+    const double a0 = alpha[e], a1 = alpha[e + 1], a2 = alpha[e + 2], a3 = alpha[e + 3];
+    const double *c0 = sC + spc[e] * TS + q, *c1 = sC + spc[e + 1] * TS + q, *c2 = sC + spc[e + 2] * TS + q,
+                 *c3 = sC + spc[e + 3] * TS + q;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      Cm[k] += c0[k * GS] * a0;
+      Cm[k] += c1[k * GS] * a1;
+      Cm[k] += c2[k * GS] * a2;
+      Cm[k] += c3[k * GS] * a3;
+    }
+  }
+  for (; e < e1; ++e) {
+    const double a = alpha[e];
+    const double *cp = sC + spc[e] * TS + q;
+#pragma unroll
+    for (int k = 0; k < V; ++k) Cm[k] += cp[k * GS] * a;
+  }
+}
+
 // One reaction (both steps) for the V states a thread owns (states
 // q + k*GS of the tile): rate constants, third body, falloff, step limiter
 // (one scalar for all steps, or one per step when lim_step is given) and
-// concentration products.  The V independent chains give the scheduler
-// instruction-level parallelism across states.
+// concentration products.  The V independent chains, and the forward and
+// reverse exponentials of each, give the scheduler instruction-level
+// parallelism: the exponentials and the limiter's quotients are branch-free
+// and run side by side.
 template <int TS, int V>
 __device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R, int q,
                                               const double *__restrict__ sC,
@@ -116,63 +223,45 @@ __device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R,
                                               const double *lim_step = nullptr, const char *tab = nullptr) {
   constexpr int GS = TS / V;
   double kf[V], kr[V];
+  // exponents first, then the exponentials together
+  double ar[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) ar[k] = 0.0;
+  if (R.flags & kRevArr) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) ar[k] = R.lnA_r + R.n_r * logT[k] - R.Ta_r * invT[k];
+  } else if (R.flags & kRevKeq) {
+    each_species<V, GS>(R.np, R.p, [&](int sp) {
+      const double *gp = sG + sp * TS + q;
+#pragma unroll
+      for (int k = 0; k < V; ++k) ar[k] += gp[k * GS];
+    });
+    each_species<V, GS>(R.nr, R.r, [&](int sp) {
+      const double *gr = sG + sp * TS + q;
+#pragma unroll
+      for (int k = 0; k < V; ++k) ar[k] -= gr[k * GS];
+    });
+#pragma unroll
+    for (int k = 0; k < V; ++k) ar[k] -= R.lnA_r * lprt[k];
+  }
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    kf[k] = exp_tree(R.lnA + R.n * logT[k] - R.Ta * invT[k]);
+    kr[k] = exp_tree(ar[k]);
+  }
   if (R.flags & kPlog) {  // at the pressure of the concentrations, Csum Ru T (rate_const.cpp:548-567)
 #pragma unroll
     for (int k = 0; k < V; ++k) kf[k] = plog_rate(m, R.aux, T[k], invT[k], logT[k], Csum[k] * kRuD * T[k], tab);
-  } else {
-#pragma unroll
-    for (int k = 0; k < V; ++k) kf[k] = exp(R.lnA + R.n * logT[k] - R.Ta * invT[k]);
   }
-  if (R.flags & kRevArr) {
+  if (!(R.flags & kRevArr)) {
+    const bool keq = (R.flags & kRevKeq) != 0;
 #pragma unroll
-    for (int k = 0; k < V; ++k) kr[k] = exp(R.lnA_r + R.n_r * logT[k] - R.Ta_r * invT[k]);
-  } else if (R.flags & kRevKeq) {
-    double s[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k) s[k] = 0.0;
-    for (int i = 0; i < R.np; ++i) {
-      const double *gp = sG + R.p[i] * TS + q;
-#pragma unroll
-      for (int k = 0; k < V; ++k) s[k] += gp[k * GS];
-    }
-    for (int i = 0; i < R.nr; ++i) {
-      const double *gr = sG + R.r[i] * TS + q;
-#pragma unroll
-      for (int k = 0; k < V; ++k) s[k] -= gr[k * GS];
-    }
-#pragma unroll
-    for (int k = 0; k < V; ++k) kr[k] = exp(s[k] - R.lnA_r * lprt[k]) * kf[k];
-  } else {
-#pragma unroll
-    for (int k = 0; k < V; ++k) kr[k] = 0.0;
+    for (int k = 0; k < V; ++k) kr[k] = keq ? kr[k] * kf[k] : 0.0;
   }
   if (R.flags & kThirdBody) {
     double Cm[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k) Cm[k] = Csum[k];
-    // efficiencies four at a time: the table loads are independent of the
-    // sums, which keep the list order
-    const int e0 = rb(m.tb_ptr, tab, m.base)[R.aux], e1 = rb(m.tb_ptr, tab, m.base)[R.aux + 1];
-    int e = e0;
-    for (; e + 3 < e1; e += 4) {
-      const double a0 = rb(m.tb_alpha, tab, m.base)[e], a1 = rb(m.tb_alpha, tab, m.base)[e + 1], a2 = rb(m.tb_alpha, tab, m.base)[e + 2],
-                   a3 = rb(m.tb_alpha, tab, m.base)[e + 3];
-      const double *c0 = sC + rb(m.tb_spc, tab, m.base)[e] * TS + q, *c1 = sC + rb(m.tb_spc, tab, m.base)[e + 1] * TS + q,
-                   *c2 = sC + rb(m.tb_spc, tab, m.base)[e + 2] * TS + q, *c3 = sC + rb(m.tb_spc, tab, m.base)[e + 3] * TS + q;
-#pragma unroll
-      for (int k = 0; k < V; ++k) {
-        Cm[k] += c0[k * GS] * a0;
-        Cm[k] += c1[k * GS] * a1;
-        Cm[k] += c2[k * GS] * a2;
-        Cm[k] += c3[k * GS] * a3;
-      }
-    }
-    for (; e < e1; ++e) {
-      const double a = rb(m.tb_alpha, tab, m.base)[e];
-      const double *cp = sC + rb(m.tb_spc, tab, m.base)[e] * TS + q;
-#pragma unroll
-      for (int k = 0; k < V; ++k) Cm[k] += cp[k * GS] * a;
-    }
+    const int *tp = rb(m.tb_ptr, tab, m.base);
+    third_body<TS, V>(rb(m.tb_spc, tab, m.base), rb(m.tb_alpha, tab, m.base), tp[R.aux], tp[R.aux + 1], q, sC, Csum, Cm);
 #pragma unroll
     for (int k = 0; k < V; ++k) {
       kf[k] *= Cm[k];
@@ -184,64 +273,64 @@ __device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R,
     const double *p = rb(m.fo_par, tab, m.base) + 8 * f;
     const int fs = rb(m.fo_spc, tab, m.base)[f];
     const int ty = rb(m.fo_type, tab, m.base)[f];
-    double Cm[V];
+    const double p3 = p[3], p4 = p[4], p5 = p[5], p6 = p[6];
+    double Klow[V], Cm[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) Klow[k] = exp_tree(p[0] + p[1] * logT[k] - p[2] * invT[k]);
     if (fs >= 0) {
 #pragma unroll
       for (int k = 0; k < V; ++k) Cm[k] = sC[fs * TS + q + k * GS];
     } else {
+      const int *fp = rb(m.fo_ptr, tab, m.base);
+      third_body<TS, V>(rb(m.fo_spc_eff, tab, m.base), rb(m.fo_alpha, tab, m.base), fp[f], fp[f + 1], q, sC, Csum, Cm);
+    }
+    double Pr[V], fT[V];
 #pragma unroll
-      for (int k = 0; k < V; ++k) Cm[k] = Csum[k];
-      const int e0 = rb(m.fo_ptr, tab, m.base)[f], e1 = rb(m.fo_ptr, tab, m.base)[f + 1];
-      int e = e0;
-      for (; e + 3 < e1; e += 4) {
-        const double a0 = rb(m.fo_alpha, tab, m.base)[e], a1 = rb(m.fo_alpha, tab, m.base)[e + 1], a2 = rb(m.fo_alpha, tab, m.base)[e + 2],
-                     a3 = rb(m.fo_alpha, tab, m.base)[e + 3];
-        const double *c0 = sC + rb(m.fo_spc_eff, tab, m.base)[e] * TS + q, *c1 = sC + rb(m.fo_spc_eff, tab, m.base)[e + 1] * TS + q,
-                     *c2 = sC + rb(m.fo_spc_eff, tab, m.base)[e + 2] * TS + q, *c3 = sC + rb(m.fo_spc_eff, tab, m.base)[e + 3] * TS + q;
+    for (int k = 0; k < V; ++k) {
+      Klow[k] *= Cm[k];
+      fT[k] = 1.0;
+    }
+    quotients<V>(Klow, kf, Pr);
 #pragma unroll
-        for (int k = 0; k < V; ++k) {
-          Cm[k] += c0[k * GS] * a0;
-          Cm[k] += c1[k * GS] * a1;
-          Cm[k] += c2[k * GS] * a2;
-          Cm[k] += c3[k * GS] * a3;
-        }
+    for (int k = 0; k < V; ++k)
+      if (Pr[k] < 1.0e-300) Pr[k] = 1.0e-300;
+    if (ty == kTroe3 || ty == kTroe4) {
+      double e1[V], e2[V], e3[V];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        e1[k] = exp_tree(p4 != 0.0 ? -T[k] / p4 : 0.0);
+        e2[k] = exp_tree(p5 != 0.0 ? -T[k] / p5 : 0.0);
+        e3[k] = exp_tree(-p6 * invT[k]);
       }
-      for (; e < e1; ++e) {
-        const double a = rb(m.fo_alpha, tab, m.base)[e];
-        const double *cp = sC + rb(m.fo_spc_eff, tab, m.base)[e] * TS + q;
 #pragma unroll
-        for (int k = 0; k < V; ++k) Cm[k] += cp[k * GS] * a;
+      for (int k = 0; k < V; ++k) {
+        double Fc = 0.0;
+        if (p4 != 0.0) Fc += (1.0 - p3) * e1[k];
+        if (p5 != 0.0) Fc += p3 * e2[k];
+        if (ty == kTroe4) Fc += e3[k];
+        if (Fc < 1.0e-300) Fc = 1.0e-300;
+        const double lF = log10(Fc);
+        const double nT = 0.75 - 1.27 * lF;
+        double x = log10(Pr[k]) - (0.4 + 0.67 * lF);
+        x = x / (nT - 0.14 * x);
+        x *= x;
+        fT[k] = exp_tree(lF / (1.0 + x) * 2.30258509299404568402);  // 10^
+      }
+    } else if (ty == kSRI) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const double lPr = log10(Pr[k]);
+        const double xp = 1.0 / (1.0 + lPr * lPr);
+        double t = p3 * exp_tree(-p4 * invT[k]);
+        if (p5 > 0) t += exp_tree(-T[k] * p5);
+        t = pow(t, xp);
+        t *= p6;
+        fT[k] = t * pow(T[k], p[7]);
       }
     }
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      const double Klow = exp(p[0] + p[1] * logT[k] - p[2] * invT[k]);
-      double Pr = Klow * Cm[k] / kf[k];
-      if (Pr < 1.0e-300) Pr = 1.0e-300;
-      double lPr = log10(Pr);
-      double fT = 1.0;
-      if (ty == kTroe3 || ty == kTroe4) {
-        double Fc = 0.0;
-        if (p[4] != 0) Fc += (1.0 - p[3]) * exp(-T[k] / p[4]);
-        if (p[5] != 0) Fc += p[3] * exp(-T[k] / p[5]);
-        if (ty == kTroe4) Fc += exp(-p[6] * invT[k]);
-        if (Fc < 1.0e-300) Fc = 1.0e-300;
-        fT = log10(Fc);
-        const double nT = 0.75 - 1.27 * fT;
-        lPr -= (0.4 + 0.67 * fT);
-        lPr = lPr / (nT - 0.14 * lPr);
-        lPr *= lPr;
-        fT /= (1.0 + lPr);
-        fT = exp10(fT);
-      } else if (ty == kSRI) {
-        const double xp = 1.0 / (1.0 + lPr * lPr);
-        fT = p[3] * exp(-p[4] * invT[k]);
-        if (p[5] > 0) fT += exp(-T[k] * p[5]);
-        fT = pow(fT, xp);
-        fT *= p[6];
-        fT *= pow(T[k], p[7]);
-      }
-      const double Pc = fT * Pr / (1.0 + Pr);
+      const double Pc = fT[k] * Pr[k] / (1.0 + Pr[k]);
       kf[k] *= Pc;
       kr[k] *= Pc;
     }
@@ -260,25 +349,33 @@ __device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R,
       }
     }
   } else if (0.0 < lim && lim < 1.0e300) {  // the plugin's step_limiter option
+    double num[2 * V], den[2 * V], w[2 * V];
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      kf[k] *= lim / (lim + kf[k]);
-      if (R.rev >= 0) kr[k] *= lim / (lim + kr[k]);
+      num[k] = num[V + k] = lim;
+      den[k] = lim + kf[k];
+      den[V + k] = lim + kr[k];
+    }
+    quotients<2 * V>(num, den, w);
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      kf[k] *= w[k];
+      kr[k] *= w[V + k];
     }
   }
-  for (int i = 0; i < R.nr; ++i) {
-    const double *cp = sC + R.r[i] * TS + q;
+  each_species<V, GS>(R.nr, R.r, [&](int sp) {
+    const double *cp = sC + sp * TS + q;
 #pragma unroll
     for (int k = 0; k < V; ++k) kf[k] *= cp[k * GS];
-  }
+  });
 #pragma unroll
   for (int k = 0; k < V; ++k) sROP[R.fwd * TS + q + k * GS] = kf[k];
   if (R.rev >= 0) {
-    for (int i = 0; i < R.np; ++i) {
-      const double *cp = sC + R.p[i] * TS + q;
+    each_species<V, GS>(R.np, R.p, [&](int sp) {
+      const double *cp = sC + sp * TS + q;
 #pragma unroll
       for (int k = 0; k < V; ++k) kr[k] *= cp[k * GS];
-    }
+    });
 #pragma unroll
     for (int k = 0; k < V; ++k) sROP[R.rev * TS + q + k * GS] = kr[k];
   }
