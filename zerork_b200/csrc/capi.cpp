@@ -49,6 +49,64 @@ LaunchCfg default_launch(const DevMech &m) {
   return c;
 }
 
+// The mapping of a call of n states on a handle whose mapping was not set.
+// 16 warps, one CTA per SM; what remains is the tile size.  A wave of 148
+// tiles costs, relative to 8-state tiles, 1.5 with 16 states and 2.25 with 32
+// (53 species: 50, 76 and 114 us a wave; in global workspace, 650 species: 1,
+// 1.56 and 2.7), so the fewest weighted waves win: 8-state tiles up to some
+// 1,200 states, 32-state tiles for large batches (131,072 states 3.19 ms,
+// against 4.23 with 16 and 4.7 with 8).  A thread takes two states where there
+// are reactions enough for the groups (8-state tiles: 325 reactions 56 us a
+// wave with one state, 69 with two; 900 reactions 128 and 113).  A mechanism of
+// a few dozen reactions costs the same per tile at any size (27 reactions:
+// 28-30 us), so it takes the largest, one state a thread (262,144 states 1.38
+// ms, 2.12 with two).  Without the Jacobian two 8-warp CTAs of 16-state tiles
+// hide more latency (131,072 states 1.12 ms against 1.19).
+static LaunchCfg pick_launch(const DevMech &m, int n, bool jac) {
+  const size_t kMaxSmem = 227 * 1024;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  LaunchCfg c;
+  c.warps = 16;
+  if (m.nrxn < 128) {
+    c.v = 1;
+    for (int ts : {32, 16, 8}) {
+      c.ts = ts;
+      if (rates_jac_ws_bytes(m, c) <= kMaxSmem) return c;
+    }
+  }
+  if (!jac && n >= 32 * sms) {
+    LaunchCfg two;
+    two.ts = 16;
+    two.v = 2;
+    two.warps = 8;
+    two.minb = 2;
+    if (2 * (rates_jac_ws_bytes(m, two) + 1024) <= 228 * 1024) return two;
+  }
+  LaunchCfg best;
+  double best_cost = 0.0;
+  for (int global = 0; global < 2 && best_cost == 0.0; ++global)
+    for (int ts : {8, 16, 32}) {
+      c.ts = ts;
+      c.v = ts == 8 && m.nrxn <= 600 ? 1 : 2;
+      c.global_ws = global != 0;
+      c.grid = global ? sms : 0;
+      if (!global && rates_jac_ws_bytes(m, c) > kMaxSmem) continue;
+      const long tiles = ((long)n + ts - 1) / ts, waves = (tiles + sms - 1) / sms;
+      const double cost = waves * (ts == 8 ? 1.0 : ts == 16 ? 1.5 : global ? 2.7 : 2.25);
+      if (best_cost == 0.0 || cost < best_cost) {
+        best_cost = cost;
+        best = c;
+      }
+    }
+  return best;
+}
+
+LaunchCfg MechHandle::launch_for(int n, bool jac) const {
+  return mapping_set ? cfg : pick_launch(dev->view(), n, jac);
+}
+
 MechHandle::~MechHandle() {
   if (scratch) cudaFree(scratch);
   if (pipe) cudaFree(pipe);
@@ -216,6 +274,7 @@ int zrk_mech_set_launch(zrk_mech_t m, int ts, int v, int warps, int flags, int g
   if (!h->dev) return set_error(ZRK_ERR_NO_DEVICE, "handle has no device tables (zrk_mech_parse)");
   if (ts == 0) {
     h->cfg = default_launch(h->dev->view());
+    h->mapping_set = false;
     return ZRK_OK;
   }
   LaunchCfg c;
@@ -231,6 +290,7 @@ int zrk_mech_set_launch(zrk_mech_t m, int ts, int v, int warps, int flags, int g
   if (rates_jac_smem_bytes(h->dev->view(), c) > 227 * 1024)
     return set_error(ZRK_ERR_INVALID_ARGUMENT, "workspace and staged tables do not fit in shared memory");
   h->cfg = c;
+  h->mapping_set = true;
   return ZRK_OK;
 }
 
@@ -258,6 +318,9 @@ int zrk_mech_autotune(zrk_mech_t m, int n, int ld, const double *T, const double
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   LaunchCfg best = h->cfg;
+  const bool was_set = h->mapping_set;
+  bool found = false;
+  h->mapping_set = true;
   float best_t = 1e30f;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -294,12 +357,14 @@ int zrk_mech_autotune(zrk_mech_t m, int n, int ld, const double *T, const double
           if (ok && cudaGetLastError() == cudaSuccess && t < best_t) {
             best_t = t;
             best = c;
+            found = true;
           }
         }
       }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   h->cfg = best;
+  h->mapping_set = found || was_set;
   if (best_ms) *best_ms = best_t / 2;
   return ZRK_OK;
 }
@@ -322,17 +387,18 @@ int zrk_rates_jac_dev(zrk_mech_t m, int n, int ld, const double *T, const double
   a.jac = jac;
   a.ydot = ydot;
   KinParams kp{h->Tref, h->mmf, h->lim, std::sqrt(2.2204460492503131e-16)};
-  if (h->cfg.global_ws) {
-    const int ntiles = (n + h->cfg.ts - 1) / h->cfg.ts;
-    int grid = h->cfg.grid > 0 ? h->cfg.grid : ntiles;
+  const LaunchCfg cfg = h->launch_for(n, jac != nullptr);
+  if (cfg.global_ws) {
+    const int ntiles = (n + cfg.ts - 1) / cfg.ts;
+    int grid = cfg.grid > 0 ? cfg.grid : ntiles;
     if (grid > ntiles) grid = ntiles;
-    size_t need = (size_t)grid * rates_jac_ws_bytes(h->dev->view(), h->cfg);
+    size_t need = (size_t)grid * rates_jac_ws_bytes(h->dev->view(), cfg);
     cudaError_t e = h->ensure_scratch(need);
     if (e != cudaSuccess) return cuda_error(e, "scratch allocation");
     a.scratch = (double *)h->scratch;
     a.scratch_bytes = h->scratch_bytes;
   }
-  cudaError_t e = launch_rates_jac(h->dev->view(), a, kp, h->cfg, (cudaStream_t)stream);
+  cudaError_t e = launch_rates_jac(h->dev->view(), a, kp, cfg, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_error(e, "rates_jac launch");
   return ZRK_OK;
 }
@@ -427,7 +493,7 @@ int zrk_rates_jac_host(zrk_mech_t m, int n, const double *T, const double *P, co
   for (long c0 = 0, i = 0; c0 < n; c0 += chunk, ++i) {
     const int cn = (int)std::min<long>(chunk, n - c0);
     // the global-workspace mapping shares one scratch area: keep one stream
-    cudaStream_t st = h->pipe_stream[h->cfg.global_ws ? 0 : i % 2];
+    cudaStream_t st = h->pipe_stream[h->launch_for(cn, jac != nullptr).global_ws ? 0 : i % 2];
     double *base = (double *)h->pipe + (i % 2) * chunk * (per_state / dp);
     double *dT = base, *dP = dT + chunk, *dY = dP + chunk, *dW = dY + (size_t)S * chunk;
     double *dJ = jac ? dW + (size_t)S * chunk : nullptr;

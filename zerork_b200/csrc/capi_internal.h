@@ -17,6 +17,7 @@ struct MechHandle {
   JacPattern pattern;
   std::unique_ptr<DeviceMechanism> dev;
   LaunchCfg cfg;
+  bool mapping_set = false;  // cfg was set or tuned; else each call takes the mapping for its size
   double Tref = 1.0, mmf = 1.0e-30, lim = 1.0e22;
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
@@ -25,6 +26,7 @@ struct MechHandle {
   size_t pipe_bytes = 0;
   cudaStream_t pipe_stream[2] = {nullptr, nullptr};
   ~MechHandle();
+  LaunchCfg launch_for(int n, bool jac) const;
   cudaError_t ensure_scratch(size_t bytes);
   cudaError_t ensure_pipe(size_t bytes);
 };

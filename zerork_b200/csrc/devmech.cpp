@@ -132,21 +132,38 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   // flat species-column list for the rates kernel's Jacobian phase
   std::vector<int2> jw;
   std::vector<unsigned short> jt;
+  std::vector<int4> jit;
+  std::vector<int2> jext;
   std::vector<int> jt_ptr(1, 0), jcost(1, 0), jf_ptr(1, 0), jf_col;
   for (int j = 0; j < ns; ++j) {
     for (int k = p.col_ptr[j]; k < p.col_ptr[j + 1] - 1; ++k) {  // the last entry is the T row
       const int nd = nzd_ptr[k + 1] - nzd_ptr[k], nc = nzc_ptr[k + 1] - nzc_ptr[k];
-      if (nd > 0xffff || nc > 0xffff || t.nstep > 0xffff)
+      if (nd > 0xffff || nc > 0xffff || t.nstep > 0xffff || ns > 0xffff)
         throw std::runtime_error("mechanism too large for 16-bit Jacobian term lists");
       jf_col.push_back(j);
       jw.push_back(make_int2(p.row_idx[k], nd | (nc << 16)));
       for (int q = nzd_ptr[k]; q < nzd_ptr[k + 1]; ++q) jt.push_back((unsigned short)nzd_step[q]);
       for (int q = nzc_ptr[k]; q < nzc_ptr[k + 1]; ++q) jt.push_back((unsigned short)nzc_step[q]);
       jt_ptr.push_back((int)jt.size());
-      jcost.push_back(jcost.back() + 3 + nd + nc);
+      {
+        unsigned q4[4];
+        const int t0 = jt_ptr[jt_ptr.size() - 2], nt = nd + nc, chunks = (nt + 3) / 4;
+        auto four = [&](int c) {
+          for (int e = 0; e < 4; ++e) q4[e] = 4 * c + e < nt ? jt[t0 + 4 * c + e] : (unsigned)t.nstep;
+        };
+        four(0);
+        jit.push_back(make_int4((int)((unsigned)p.row_idx[k] | (unsigned)nd << 16), (int)(q4[0] | q4[1] << 16),
+                                (int)(q4[2] | q4[3] << 16), (int)jext.size()));
+        for (int c = 1; c < chunks; ++c) {
+          four(c);
+          jext.push_back(make_int2((int)(q4[0] | q4[1] << 16), (int)(q4[2] | q4[3] << 16)));
+        }
+        jcost.push_back(jcost.back() + 12 + 4 * std::max(1, chunks));
+      }
     }
     jf_ptr.push_back((int)jw.size());
   }
+  jit.push_back(make_int4(0, 0, 0, (int)jext.size()));
   std::vector<std::vector<std::pair<int, int>>> rows(p.n);
   for (int j = 0; j < p.n; ++j)
     for (int k = p.col_ptr[j]; k < p.col_ptr[j + 1]; ++k) rows[p.row_idx[k]].push_back({k, j});
@@ -190,7 +207,15 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
       w += 1.0 + (nzd_ptr[kk + 1] - nzd_ptr[kk]) + (nzc_ptr[kk + 1] - nzc_ptr[kk]);
     cc[k] = w;
   }
-  const std::vector<int> rxn_order = sorted_by(rc), spc_order = sorted_by(sc2), col_order = sorted_by(cc);
+  // reactions of one kind together (a warp's groups then run one kind's code),
+  // costliest kind first, by cost within
+  auto kind_of = [&](int j) {
+    const int fl = rec[j].flags;
+    return (fl & kPlog) ? 0 : (fl & kFalloff) ? 1 : (fl & kThirdBody) ? 2 : 3;
+  };
+  std::vector<int> rxn_order = sorted_by(rc);
+  std::stable_sort(rxn_order.begin(), rxn_order.end(), [&](int a, int b) { return kind_of(a) < kind_of(b); });
+  const std::vector<int> spc_order = sorted_by(sc2), col_order = sorted_by(cc);
 
   // The tables of the rates kernel first, 16-byte aligned and contiguous:
   // the kernel may stage [blob, blob + hot_bytes) in shared memory.
@@ -198,10 +223,8 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   for (int p : rxn_order) rec_by_cost.push_back(rec[p]);
   std::vector<RxnRec> slots;
   for (int kind = 0; kind < 4; ++kind) {
-    for (int p : rxn_order) {
-      const int fl = rec[p].flags;
-      if (((fl & kPlog) ? 0 : (fl & kFalloff) ? 1 : (fl & kThirdBody) ? 2 : 3) == kind) slots.push_back(rec[p]);
-    }
+    for (int p : rxn_order)
+      if (kind_of(p) == kind) slots.push_back(rec[p]);
     while (slots.size() % 32) {
       RxnRec none;
       std::memset(&none, 0, sizeof(none));
@@ -224,10 +247,10 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
          o_scs = b.add(sc_step, h);
   size_t o_so = b.add(spc_order, h);
   size_t o_cp = b.add(p.col_ptr, h), o_ri = b.add(p.row_idx, h);
-  size_t o_jw = b.add(jw, h), o_jt = b.add(jt, h), o_jtp = b.add(jt_ptr, h), o_jc = b.add(jcost, h),
-         o_jf = b.add(jf_ptr, h);
+  size_t o_jit = b.add(jit, h), o_jext = b.add(jext, h), o_jc = b.add(jcost, h), o_jf = b.add(jf_ptr, h);
   const size_t hot = (b.bytes.size() + 15) & ~size_t(15);
   size_t o_rec = b.add(rec), o_slot = b.add(slots);
+  size_t o_jw = b.add(jw), o_jt = b.add(jt), o_jtp = b.add(jt_ptr);
   size_t o_jfc = b.add(jf_col);
   size_t o_snp = b.add(sn_ptr), o_sns = b.add(sn_step);
   size_t o_lr = b.add(p.last_row);
@@ -282,6 +305,8 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.nzc_step = (const int *)P(o_ncs);
   view_.nj = (int)jw.size();
   view_.jw = (const int2 *)P(o_jw);
+  view_.jit = (const int4 *)P(o_jit);
+  view_.jext = (const int2 *)P(o_jext);
   view_.jt = (const unsigned short *)P(o_jt);
   view_.jt_ptr = (const int *)P(o_jtp);
   view_.jcost = (const int *)P(o_jc);

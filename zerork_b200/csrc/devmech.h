@@ -63,12 +63,17 @@ struct DevMech {
   // Species-column Jacobian entries as one flat list in column-major order
   // without each column's temperature row (nj items; column j holds items
   // [jf_ptr[j], jf_ptr[j+1]), and item f is nonzero f + j of the compressed
-  // columns): per item {row, n_des | n_cre << 16}, its destruction then
-  // creation step indices from jt[jt_ptr[f]], and the cumulative work
-  // estimate jcost[f] (3 + n_des + n_cre per item) that splits the list into
-  // equal shares for the thread groups of the rates kernel.
+  // columns).  jw / jt: per item {row, n_des | n_cre << 16} and its
+  // destruction then creation step indices from jt[jt_ptr[f]].  jit: the same
+  // as 16-byte records {row | n_des << 16, the first four steps as 16-bit
+  // indices, the item's first record of further steps}, four further steps a
+  // record of jext; unused places hold nstep, the workspace's row of zeros;
+  // one sentinel item ends the list.  jcost: the cumulative work estimate (12
+  // and 4 per record of four steps) that splits the list into equal shares for
+  // the thread groups of the rates kernel.
   int nj;
-  const int2 *jw;
+  const int2 *jw, *jext;
+  const int4 *jit;
   const unsigned short *jt;
   const int *jt_ptr, *jcost, *jf_ptr;
   const int *jf_col;  // column of each item

@@ -111,7 +111,7 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
   RxnRec R;
   R.flags = kNoRxn;
   if (w < m.nblocks) R = load_rxn(m.rxn_slots + w * 32 + lane);
-  const double logT = log(T), invT = 1.0 / T, lprt = kLnPatmRu - logT;
+  const double logT = log(T), invT = 1.0 / T;
   const double dens = 1.0 / v;
   const double ush = o.cp ? 0.0 : 1.0;  // h/RT - 1 = u/RT; c_p/R - 1 = c_v/R
   double pc = 0.0, pcv = 0.0;
@@ -138,7 +138,7 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
     R.flags = kNoRxn;
     if (nb < m.nblocks) R = load_rxn(m.rxn_slots + nb * 32 + lane);
     if (!(cur.flags & kNoRxn))
-      reaction_item<1, 1>(m, cur, 0, s.C, s.G, s.ROP, &T, &logT, &invT, &lprt, &Csum, o.lim);
+      reaction_item<1, 1>(m, cur, 0, s.C, s.G, s.ROP, &T, &logT, &invT, &Csum, o.lim);
   }
   double cv = 0.0;
   for (int i = 0; i < nw; ++i) cv += s.red[32 + i];

@@ -52,6 +52,11 @@ struct RatesTCArgs {
 size_t rates_tc_smem_bytes(const DevMech &m, int ts, int threads);
 cudaError_t launch_rates_tc(const DevMech &m, const RatesTCArgs &a, cudaStream_t stream);
 
+// Partial-sum rows of the workspace: as many as thread groups, so that each can
+// take a share of the Jacobian, when they fit in shared memory, else two per
+// warp (the groups beyond then have no share).
+int rates_jac_part_rows(const DevMech &m, const LaunchCfg &cfg);
+// The whole workspace of a tile.
 size_t rates_jac_ws_bytes(const DevMech &m, const LaunchCfg &cfg);
 // Dynamic shared memory of a launch: the workspace (unless global) plus the
 // staged tables (cfg.stage).

@@ -162,9 +162,65 @@ __device__ __forceinline__ RxnRec load_rxn(const RxnRec *p) {
   return R;
 }
 
+// V consecutive doubles of a workspace row (16-byte aligned for V > 1).
+template <int V>
+__device__ __forceinline__ void ldv(const double *p, double (&x)[V]) {
+  if constexpr (V == 1) {
+    x[0] = p[0];
+  } else {
+#pragma unroll
+    for (int k = 0; k < V; k += 2) {
+      const double2 t = *reinterpret_cast<const double2 *>(p + k);
+      x[k] = t.x;
+      x[k + 1] = t.y;
+    }
+  }
+}
+template <int V>
+__device__ __forceinline__ void stv(double *p, const double (&x)[V]) {
+  if constexpr (V == 1) {
+    p[0] = x[0];
+  } else {
+#pragma unroll
+    for (int k = 0; k < V; k += 2) *reinterpret_cast<double2 *>(p + k) = make_double2(x[k], x[k + 1]);
+  }
+}
+
+// Sum over the groups of a warp (lanes q, q+GS, ...) with shuffles; lanes
+// q < GS of each warp then hold the warp's partial for their states.
+template <int GS>
+__device__ __forceinline__ double warp_group_sum(double v) {
+#pragma unroll
+  for (int o = GS; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Gather-sum of rates of progress over an index list, V states; four rows in
+// flight, added in list order.
+template <int TS, int V>
+__device__ __forceinline__ void gather_rop(const double *__restrict__ sROP, const int *__restrict__ list,
+                                           int b, int e, int q, double (&acc)[V]) {
+  int i = b;
+  for (; i + 3 < e; i += 4) {
+    double r[4][V];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) ldv<V>(sROP + list[i + u] * TS + q, r[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int k = 0; k < V; ++k) acc[k] += r[u][k];
+  }
+  for (; i < e; ++i) {
+    double r[V];
+    ldv<V>(sROP + list[i] * TS + q, r);
+#pragma unroll
+    for (int k = 0; k < V; ++k) acc[k] += r[k];
+  }
+}
+
 // Species sums and products of a reaction's side: sides of up to three
 // species without a loop, so their rows are read together.
-template <int V, int GS, class F>
+template <class F>
 __device__ __forceinline__ void each_species(int count, const short *spc, F f) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
@@ -182,46 +238,45 @@ __device__ __forceinline__ void each_species(int count, const short *spc, F f) {
 template <int TS, int V>
 __device__ __forceinline__ void third_body(const int *__restrict__ spc, const double *__restrict__ alpha, int e0, int e1,
                                            int q, const double *__restrict__ sC, const double *Csum, double *Cm) {
-  constexpr int GS = TS / V;
 #pragma unroll
   for (int k = 0; k < V; ++k) Cm[k] = Csum[k];
   int e = e0;
   for (; e + 3 < e1; e += 4) {
-    const double a0 = alpha[e], a1 = alpha[e + 1], a2 = alpha[e + 2], a3 = alpha[e + 3];
-    const double *c0 = sC + spc[e] * TS + q, *c1 = sC + spc[e + 1] * TS + q, *c2 = sC + spc[e + 2] * TS + q,
-                 *c3 = sC + spc[e + 3] * TS + q;
+    double a[4], c[4][V];
 #pragma unroll
-    for (int k = 0; k < V; ++k) {
-      Cm[k] += c0[k * GS] * a0;
-      Cm[k] += c1[k * GS] * a1;
-      Cm[k] += c2[k * GS] * a2;
-      Cm[k] += c3[k * GS] * a3;
+    for (int i = 0; i < 4; ++i) {
+      a[i] = alpha[e + i];
+      ldv<V>(sC + spc[e + i] * TS + q, c[i]);
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int k = 0; k < V; ++k) Cm[k] += c[i][k] * a[i];
   }
   for (; e < e1; ++e) {
     const double a = alpha[e];
-    const double *cp = sC + spc[e] * TS + q;
+    double c[V];
+    ldv<V>(sC + spc[e] * TS + q, c);
 #pragma unroll
-    for (int k = 0; k < V; ++k) Cm[k] += cp[k * GS] * a;
+    for (int k = 0; k < V; ++k) Cm[k] += c[k] * a;
   }
 }
 
-// One reaction (both steps) for the V states a thread owns (states
-// q + k*GS of the tile): rate constants, third body, falloff, step limiter
+// One reaction (both steps) for the V states a thread owns (states q .. q +
+// V - 1 of the tile): rate constants, third body, falloff, step limiter
 // (one scalar for all steps, or one per step when lim_step is given) and
 // concentration products.  The V independent chains, and the forward and
 // reverse exponentials of each, give the scheduler instruction-level
 // parallelism: the exponentials and the limiter's quotients are branch-free
-// and run side by side.
+// and run side by side.  gs: the sum of g/RT over products minus reactants.
 template <int TS, int V>
-__device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R, int q,
+__device__ __forceinline__ void reaction_eval(const DevMech &m, const RxnRec &R, int q,
                                               const double *__restrict__ sC,
-                                              const double *__restrict__ sG, double *sROP,
+                                              const double *gs, double *sROP,
                                               const double *T, const double *logT,
-                                              const double *invT, const double *lprt,
+                                              const double *invT,
                                               const double *Csum, double lim,
                                               const double *lim_step = nullptr, const char *tab = nullptr) {
-  constexpr int GS = TS / V;
   double kf[V], kr[V];
   // exponents first, then the exponentials together
   double ar[V];
@@ -231,18 +286,8 @@ __device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R,
 #pragma unroll
     for (int k = 0; k < V; ++k) ar[k] = R.lnA_r + R.n_r * logT[k] - R.Ta_r * invT[k];
   } else if (R.flags & kRevKeq) {
-    each_species<V, GS>(R.np, R.p, [&](int sp) {
-      const double *gp = sG + sp * TS + q;
 #pragma unroll
-      for (int k = 0; k < V; ++k) ar[k] += gp[k * GS];
-    });
-    each_species<V, GS>(R.nr, R.r, [&](int sp) {
-      const double *gr = sG + sp * TS + q;
-#pragma unroll
-      for (int k = 0; k < V; ++k) ar[k] -= gr[k * GS];
-    });
-#pragma unroll
-    for (int k = 0; k < V; ++k) ar[k] -= R.lnA_r * lprt[k];
+    for (int k = 0; k < V; ++k) ar[k] = gs[k] - R.lnA_r * (kLnPatmRu - logT[k]);
   }
 #pragma unroll
   for (int k = 0; k < V; ++k) {
@@ -278,8 +323,7 @@ __device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R,
 #pragma unroll
     for (int k = 0; k < V; ++k) Klow[k] = exp_tree(p[0] + p[1] * logT[k] - p[2] * invT[k]);
     if (fs >= 0) {
-#pragma unroll
-      for (int k = 0; k < V; ++k) Cm[k] = sC[fs * TS + q + k * GS];
+      ldv<V>(sC + fs * TS + q, Cm);
     } else {
       const int *fp = rb(m.fo_ptr, tab, m.base);
       third_body<TS, V>(rb(m.fo_spc_eff, tab, m.base), rb(m.fo_alpha, tab, m.base), fp[f], fp[f + 1], q, sC, Csum, Cm);
@@ -363,22 +407,60 @@ __device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R,
       kr[k] *= w[V + k];
     }
   }
-  each_species<V, GS>(R.nr, R.r, [&](int sp) {
-    const double *cp = sC + sp * TS + q;
+  each_species(R.nr, R.r, [&](int sp) {
+    double c[V];
+    ldv<V>(sC + sp * TS + q, c);
 #pragma unroll
-    for (int k = 0; k < V; ++k) kf[k] *= cp[k * GS];
+    for (int k = 0; k < V; ++k) kf[k] *= c[k];
   });
-#pragma unroll
-  for (int k = 0; k < V; ++k) sROP[R.fwd * TS + q + k * GS] = kf[k];
+  stv<V>(sROP + R.fwd * TS + q, kf);
   if (R.rev >= 0) {
-    each_species<V, GS>(R.np, R.p, [&](int sp) {
-      const double *cp = sC + sp * TS + q;
+    each_species(R.np, R.p, [&](int sp) {
+      double c[V];
+      ldv<V>(sC + sp * TS + q, c);
 #pragma unroll
-      for (int k = 0; k < V; ++k) kr[k] *= cp[k * GS];
+      for (int k = 0; k < V; ++k) kr[k] *= c[k];
     });
-#pragma unroll
-    for (int k = 0; k < V; ++k) sROP[R.rev * TS + q + k * GS] = kr[k];
+    stv<V>(sROP + R.rev * TS + q, kr);
   }
+}
+
+// The sum of the g/RT rows over a reaction's products minus its reactants, for
+// a reverse rate from the equilibrium constant (else zero).
+template <int TS, int V>
+__device__ __forceinline__ void gibbs_from_rows(const RxnRec &R, int q, const double *__restrict__ sG,
+                                                double (&gs)[V]) {
+#pragma unroll
+  for (int k = 0; k < V; ++k) gs[k] = 0.0;
+  if (R.flags & kRevKeq) {
+    each_species(R.np, R.p, [&](int sp) {
+      double g[V];
+      ldv<V>(sG + sp * TS + q, g);
+#pragma unroll
+      for (int k = 0; k < V; ++k) gs[k] += g[k];
+    });
+    each_species(R.nr, R.r, [&](int sp) {
+      double g[V];
+      ldv<V>(sG + sp * TS + q, g);
+#pragma unroll
+      for (int k = 0; k < V; ++k) gs[k] -= g[k];
+    });
+  }
+}
+
+// The same with the g/RT rows of the species: their sum over products minus
+// reactants, then the evaluation.
+template <int TS, int V>
+__device__ __forceinline__ void reaction_item(const DevMech &m, const RxnRec &R, int q,
+                                              const double *__restrict__ sC,
+                                              const double *__restrict__ sG, double *sROP,
+                                              const double *T, const double *logT,
+                                              const double *invT,
+                                              const double *Csum, double lim,
+                                              const double *lim_step = nullptr, const char *tab = nullptr) {
+  double gs[V];
+  gibbs_from_rows<TS, V>(R, q, sG, gs);
+  reaction_eval<TS, V>(m, R, q, sC, gs, sROP, T, logT, invT, Csum, lim, lim_step, tab);
 }
 
 __device__ __forceinline__ double clamp_mass_fraction(double y, double mmf) {

@@ -14,6 +14,8 @@
 // (rate_const.cpp:548-567).
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 #include "devmech.h"
 #include "kinetics.h"
 #include "kinetics_dev.cuh"
@@ -29,27 +31,38 @@ __global__ void __launch_bounds__(256, MINB) rates_tc_kernel(DevMech m, int n, i
                                                       double *__restrict__ net,
                                                       double *__restrict__ cre_out,
                                                       double *__restrict__ des_out,
-                                                      double *__restrict__ rop_out) {
+                                                      double *__restrict__ rop_out, int vec) {
   constexpr int GS = TS / V;
-  extern __shared__ double smem_dyn[];
+  extern __shared__ __align__(16) double smem_dyn[];
   const int S = m.nsp, N = m.nstep;
   const int NW = blockDim.x >> 5, NG = blockDim.x / GS;
-  const int g = threadIdx.x / GS, q = threadIdx.x % GS, w = threadIdx.x >> 5;
+  const int g = threadIdx.x / GS, q = threadIdx.x % GS * V, w = threadIdx.x >> 5;
   const bool wlead = (threadIdx.x & 31) < GS;
   double *sC = smem_dyn, *sG = sC + S * TS, *sROP = sG + S * TS, *sPart = sROP + (size_t)N * TS;
 #define FORV _Pragma("unroll") for (int k = 0; k < V; ++k)
   const int ntiles = (n + TS - 1) / TS;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    int st[V];
+    const int st0 = tile * TS + q;
     bool valid[V];
-    double T[V], logT[V], invT[V], lprt[V], Csum[V];
+    FORV valid[k] = st0 + k < n;
+    const bool wide = V > 1 && vec && valid[V - 1];  // 16-byte global accesses
+    auto put = [&](double *row, const double (&x)[V]) {
+      double *p = row + st0;
+      if (wide) {
+        if constexpr (V > 1) {
+#pragma unroll
+          for (int k = 0; k < V; k += 2)
+            __stcs(reinterpret_cast<double2 *>(p + k), make_double2(x[k], x[k + 1]));
+        }
+      } else {
+        FORV if (valid[k]) __stcs(p + k, x[k]);
+      }
+    };
+    double T[V], logT[V], invT[V], Csum[V];
     FORV {
-      st[k] = tile * TS + q + k * GS;
-      valid[k] = st[k] < n;
-      T[k] = valid[k] ? Tin[st[k]] : 1000.0;
+      T[k] = valid[k] ? Tin[st0 + k] : 1000.0;
       logT[k] = log(T[k]);
       invT[k] = 1.0 / T[k];
-      lprt[k] = log(kPatmD / (kRuD * T[k]));
     }
     // concentrations and g/RT; partial concentration sums per warp
     {
@@ -57,57 +70,61 @@ __global__ void __launch_bounds__(256, MINB) rates_tc_kernel(DevMech m, int n, i
       FORV pc[k] = 0.0;
       for (int s = g; s < S; s += NG) {
         const double *th = m.thermo + 16 * s;
+        double c[V], gg[V];
+        const double *p = Cin + (size_t)s * ld + st0;
+        if (wide) ldv<V>(p, c);
+        else FORV c[k] = valid[k] ? p[k] : 0.0;
         FORV {
-          const double c = valid[k] ? Cin[(size_t)s * ld + st[k]] : 0.0;
-          sC[s * TS + q + k * GS] = c;
-          double cp, h, gg;
-          nasa_cp_h_g(th, T[k], logT[k], &cp, &h, &gg);
-          sG[s * TS + q + k * GS] = gg;
-          pc[k] += c;
+          double cp, h;
+          nasa_cp_h_g(th, T[k], logT[k], &cp, &h, &gg[k]);
+          pc[k] += c[k];
         }
+        stv<V>(sC + s * TS + q, c);
+        stv<V>(sG + s * TS + q, gg);
       }
-#pragma unroll
-      for (int o = GS; o < 32; o <<= 1) FORV pc[k] += __shfl_xor_sync(0xffffffffu, pc[k], o);
-      if (wlead) FORV sPart[w * TS + q + k * GS] = pc[k];
+      FORV pc[k] = warp_group_sum<GS>(pc[k]);
+      if (wlead) stv<V>(sPart + w * TS + q, pc);
     }
     __syncthreads();
-    FORV {
-      double cs = 0.0;
-      for (int ww = 0; ww < NW; ++ww) cs += sPart[ww * TS + q + k * GS];
-      Csum[k] = cs;
+    FORV Csum[k] = 0.0;
+    for (int ww = 0; ww < NW; ++ww) {
+      double x[V];
+      ldv<V>(sPart + ww * TS + q, x);
+      FORV Csum[k] += x[k];
     }
-    // reactions: both steps of each reaction, the cost-sorted records dealt
-    // to the groups in snake order (round r gives group g the record at
-    // r*NG + g, or r*NG + NG-1-g for odd r) so every group's work is close
-    // to the mean
+    // reactions: both steps of each reaction, the records (sorted by kind and
+    // cost) dealt to the groups in snake order (round r gives group g the
+    // record at r*NG + g, or r*NG + NG-1-g for odd r) so every group's work is
+    // close to the mean; the next one on its way to L1
     for (int rr = 0; rr * NG < m.nrxn; ++rr) {
-      const int rp = rr * NG + ((rr & 1) ? NG - 1 - g : g);
+      const int rp = rr * NG + ((rr & 1) ? NG - 1 - g : g), nx = (rr + 1) * NG + ((rr & 1) ? g : NG - 1 - g);
+      if (nx < m.nrxn) asm volatile("prefetch.global.L1 [%0];" ::"l"(m.rxn_by_cost + nx));
       if (rp < m.nrxn)
-        reaction_item<TS, V>(m, load_rxn(m.rxn_by_cost + rp), q, sC, sG, sROP, T, logT, invT, lprt, Csum,
-                             0.0, lim_step);
+        reaction_item<TS, V>(m, load_rxn(m.rxn_by_cost + rp), q, sC, sG, sROP, T, logT, invT, Csum, 0.0,
+                             lim_step);
     }
     __syncthreads();
-    // destruction and creation in ascending step order, net = create - destroy
-    for (int s = g; s < S; s += NG) {
-      double des[V], cre[V];
+    // destruction and creation in ascending step order, net = create - destroy;
+    // the longest lists first, in snake order
+    for (int rr = 0; rr * NG < S; ++rr) {
+      const int sp = rr * NG + ((rr & 1) ? NG - 1 - g : g);
+      if (sp >= S) continue;
+      const int s = m.spc_order[sp];
+      double des[V], cre[V], d[V];
       FORV des[k] = cre[k] = 0.0;
-      for (int i = m.sd_ptr[s]; i < m.sd_ptr[s + 1]; ++i) {
-        const double *rp = sROP + m.sd_step[i] * TS + q;
-        FORV des[k] += rp[k * GS];
-      }
-      for (int i = m.sc_ptr[s]; i < m.sc_ptr[s + 1]; ++i) {
-        const double *rp = sROP + m.sc_step[i] * TS + q;
-        FORV cre[k] += rp[k * GS];
-      }
-      FORV if (valid[k]) {
-        const size_t o = (size_t)s * ld + st[k];
-        if (net) net[o] = cre[k] - des[k];
-        if (cre_out) cre_out[o] = cre[k];
-        if (des_out) des_out[o] = des[k];
-      }
+      gather_rop<TS, V>(sROP, m.sd_step, m.sd_ptr[s], m.sd_ptr[s + 1], q, des);
+      gather_rop<TS, V>(sROP, m.sc_step, m.sc_ptr[s], m.sc_ptr[s + 1], q, cre);
+      FORV d[k] = cre[k] - des[k];
+      if (net) put(net + (size_t)s * ld, d);
+      if (cre_out) put(cre_out + (size_t)s * ld, cre);
+      if (des_out) put(des_out + (size_t)s * ld, des);
     }
     if (rop_out)
-      for (int j = g; j < N; j += NG) FORV if (valid[k]) rop_out[(size_t)j * ld + st[k]] = sROP[j * TS + q + k * GS];
+      for (int j = g; j < N; j += NG) {
+        double r[V];
+        ldv<V>(sROP + j * TS + q, r);
+        put(rop_out + (size_t)j * ld, r);
+      }
     __syncthreads();  // the next tile reuses the workspace
   }
 #undef FORV
@@ -125,8 +142,10 @@ cudaError_t launch_tv(const DevMech &m, const RatesTCArgs &a, int threads, cudaS
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int ntiles = (a.n + TS - 1) / TS;
   const int grid = ntiles < 8 * sms ? ntiles : 8 * sms;
+  const auto al16 = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
+  const int vec = a.ld % 2 == 0 && al16(a.C) && al16(a.net) && al16(a.create) && al16(a.destroy) && al16(a.rop);
   rates_tc_kernel<TS, V, MINB><<<grid, threads, bytes, stream>>>(m, a.n, a.ld, a.T, a.C, a.lim_step,
-                                                          a.net, a.create, a.destroy, a.rop);
+                                                          a.net, a.create, a.destroy, a.rop, vec);
   return cudaGetLastError();
 }
 
