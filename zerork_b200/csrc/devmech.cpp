@@ -232,6 +232,13 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
       slots.push_back(none);
     }
   }
+  std::vector<int4> slot_parts(slots.size() * 6);
+  for (size_t i = 0; i < slots.size(); ++i)
+    for (int c = 0; c < 6; ++c)
+      std::memcpy(&slot_parts[(i / 32 * 6 + c) * 32 + i % 32], (const char *)&slots[i] + 16 * c, 16);
+  std::vector<double> thermo_t(16 * (size_t)ns);
+  for (int j = 0; j < ns; ++j)
+    for (int c = 0; c < 16; ++c) thermo_t[(size_t)c * ns + j] = t.thermo[16 * (size_t)j + c];
   Blob b;
   const size_t h = 16;
   size_t o_rbc = b.add(rec_by_cost, h);
@@ -249,7 +256,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   size_t o_cp = b.add(p.col_ptr, h), o_ri = b.add(p.row_idx, h);
   size_t o_jit = b.add(jit, h), o_jext = b.add(jext, h), o_jc = b.add(jcost, h), o_jf = b.add(jf_ptr, h);
   const size_t hot = (b.bytes.size() + 15) & ~size_t(15);
-  size_t o_rec = b.add(rec), o_slot = b.add(slots);
+  size_t o_rec = b.add(rec), o_slot = b.add(slot_parts), o_tht = b.add(thermo_t);
   size_t o_jw = b.add(jw), o_jt = b.add(jt), o_jtp = b.add(jt_ptr);
   size_t o_jfc = b.add(jf_col);
   size_t o_snp = b.add(sn_ptr), o_sns = b.add(sn_step);
@@ -320,7 +327,8 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.spc_order = (const int *)P(o_so);
   view_.col_order = (const int *)P(o_co);
   view_.rxn_by_cost = (const RxnRec *)P(o_rbc);
-  view_.rxn_slots = (const RxnRec *)P(o_slot);
+  view_.rxn_slots = (const int4 *)P(o_slot);
+  view_.thermo_t = (const double *)P(o_tht);
   view_.nblocks = (int)(slots.size() / 32);
 }
 

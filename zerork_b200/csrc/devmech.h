@@ -44,6 +44,7 @@ struct DevMech {
   int nsp, nrxn, nstep, nnz;
   int max_list;  // unused by kernels, kept for diagnostics
   const double *mw, *inv_mw, *ru_inv_mw, *thermo;  // thermo: [nsp*16]
+  const double *thermo_t;  // the same, coefficient by coefficient: [16][nsp]
   const RxnRec *rxn;
   const int *tb_ptr, *tb_spc;
   const double *tb_alpha;
@@ -92,8 +93,10 @@ struct DevMech {
   // The same records for one reactor per CTA, a reaction a lane: grouped by
   // kind (PLOG, falloff, third body, the rest) in blocks of 32 of one kind,
   // padded with kNoRxn records, so that a warp runs one kind's code and the
-  // long falloff chains run beside the others instead of after them.
-  const RxnRec *rxn_slots;
+  // long falloff chains run beside the others instead of after them.  The six
+  // 16-byte parts of a block's records are stored part by part ([block][6][32]),
+  // so that a warp reads each in one piece.
+  const int4 *rxn_slots;
   int nblocks;
   // The tables the rates kernel reads form the first hot_bytes bytes of the
   // allocation at base (16-byte aligned), so a CTA can stage them in shared

@@ -14,6 +14,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "integrator.h"
 #include "kinetics_dev.cuh"
 #include "reactor_src.cuh"
@@ -28,6 +30,7 @@ constexpr double kMaxFactor = 10.0;
 constexpr double kEtaKeep = 1.5;
 constexpr int kMaxl = 10;  // Krylov dimension (no restarts)
 constexpr int kPanelMax = 8;  // widest panel of the inversion
+constexpr size_t kStateBytes = 1600;  // KernelState
 constexpr int kPredBuf = 256;  // widest predictor layer (padded)
 
 struct Smem {
@@ -50,6 +53,13 @@ struct Smem {
   // d = dT*/dY, w = (I - c J)^-1 g of the current factor
   double *r1g, *r1d, *r1w;
 };
+
+// Doubles of the region that the pivot rows and the predictor share with the
+// rates workspace and six vectors.
+__host__ __device__ inline size_t dense_rows_doubles(int nsp) {
+  const size_t d = 9 * (size_t)nsp + 6;
+  return d > kPredBuf ? d : kPredBuf;
+}
 
 // What one right-hand-side evaluation used: mixture heat capacity (c_v, or
 // c_p for constant pressure), temperature and inverse density.
@@ -110,7 +120,7 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
   const int lane = tid & 31, w = tid >> 5, nw = nt >> 5;
   RxnRec R;
   R.flags = kNoRxn;
-  if (w < m.nblocks) R = load_rxn(m.rxn_slots + w * 32 + lane);
+  if (w < m.nblocks) R = load_slot(m.rxn_slots, w, lane);
   const double logT = log(T), invT = 1.0 / T;
   const double dens = 1.0 / v;
   const double ush = o.cp ? 0.0 : 1.0;  // h/RT - 1 = u/RT; c_p/R - 1 = c_v/R
@@ -121,7 +131,7 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
     const double c = dens * m.inv_mw[k] * ys;
     s.C[k] = c;
     double cp, h, g;
-    nasa_cp_h_g(m.thermo + 16 * k, T, logT, &cp, &h, &g);
+    nasa_cp_h_g(m.thermo_t + k, T, logT, &cp, &h, &g, S);
     s.G[k] = g;
     s.U[k] = h - ush;
     pc += c;
@@ -136,7 +146,7 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
     const RxnRec cur = R;
     const int nb = (rr + 1) * nw + ((rr & 1) ? w : nw - 1 - w);
     R.flags = kNoRxn;
-    if (nb < m.nblocks) R = load_rxn(m.rxn_slots + nb * 32 + lane);
+    if (nb < m.nblocks) R = load_slot(m.rxn_slots, nb, lane);
     if (!(cur.flags & kNoRxn))
       reaction_item<1, 1>(m, cur, 0, s.C, s.G, s.ROP, &T, &logT, &invT, &Csum, o.lim);
   }
@@ -1091,52 +1101,76 @@ failed:  // D[0] holds the last accepted state (step-size changes keep it)
 
 // spill bits: 1 = rates of progress in a global slice, 2 = BDF differences
 // in a global slice (both L2-resident: one slice per resident CTA).
+// What the integrator's functions read through references, in shared memory:
+// the mechanism's table addresses, options, workspace addresses and method
+// constants.  (As kernel parameters and locals they would be copied to the
+// stack, which shares what L1 the Newton matrix leaves with the tables; each
+// use of a table then waited for its address first, often from L2.)
+struct KernelState {
+  DevMech m;
+  IntegOpts o;
+  Smem s;
+  Consts bc;
+};
+static_assert(sizeof(KernelState) <= kStateBytes, "KernelState outgrew its share of shared memory");
+
 template <class LT>
-__global__ void __launch_bounds__(512, 1) integrate_dense_kernel(DevMech m, IntegOpts o, IntegArgs a,
+__global__ void __launch_bounds__(512, 1) integrate_dense_kernel(DevMech mp, IntegOpts op, IntegArgs a,
                                                                  int lda, int spill) {
   extern __shared__ double smem_dyn[];
-  const int S = m.nsp, n = S + 1, N = m.nstep, tid = threadIdx.x, nt = blockDim.x;
-  Smem s;
-  double *p = smem_dyn;
-  double *g = a.rop_scratch + (size_t)blockIdx.x * ((size_t)N + (kMaxOrder + 6) * (size_t)n);
-  s.red = p; p += 128;
-  // pivot rows of the inversion over what is dead during one: the rates
-  // workspace and six vectors, 3 S + 6 n >= kPanelMax n doubles
-  s.rows = p;
-  s.C = p; p += S;
-  s.G = p; p += S;
-  s.U = p; p += S;
-  s.f = p; p += n;
-  s.f0 = p; p += n;
-  s.tmp = p; p += n;
-  s.yp = p; p += n;
-  s.colk = p; p += n;
-  s.bs = p; p += n;
-  if (spill & 1) { s.ROP = g; } else { s.ROP = p; p += N; }
-  if (spill & 2) { s.D = g + N; } else { s.D = p; p += (kMaxOrder + 3) * n; }
-  s.Jsm = nullptr;
-  if (spill & 4) { s.Jsm = p; p += m.nnz; }
-  s.ysrc = nullptr;
-  s.r1g = g + N + (kMaxOrder + 3) * n;
-  s.r1d = s.r1g + n;
-  s.r1w = s.r1d + n;
-  s.y = p; p += n;
-  s.ypred = p; p += n;
-  s.psi = p; p += n;
-  s.d = p; p += n;
-  s.scale = p; p += n;
-  s.wlu = p; p += n;
-  s.V = nullptr;
-  if (sizeof(LT) == sizeof(float)) {
-    s.V = p;
-    p += (kMaxl + 3) * n;
+  KernelState &ks = *reinterpret_cast<KernelState *>(smem_dyn);
+  const int S = mp.nsp, n = S + 1, N = mp.nstep, tid = threadIdx.x, nt = blockDim.x;
+  if (tid == 0) {
+    ks.m = mp;
+    ks.o = op;
+    make_consts(ks.bc);
+    Smem &s = ks.s;
+    double *p = smem_dyn + kStateBytes / sizeof(double);
+    double *g = a.rop_scratch + (size_t)blockIdx.x * ((size_t)N + (kMaxOrder + 6) * (size_t)n);
+    s.red = p; p += 128;
+    // over what is dead then: the inversion's pivot rows (kPanelMax n doubles
+    // in the 3 S + 6 n of the rates workspace and six vectors) and the learned
+    // predictor's activations
+    s.rows = p;
+    s.mlp = (float *)p;  // 2 * kPredBuf floats
+    double *const end = p + dense_rows_doubles(S);
+    s.C = p; p += S;
+    s.G = p; p += S;
+    s.U = p; p += S;
+    s.f = p; p += n;
+    s.f0 = p; p += n;
+    s.tmp = p; p += n;
+    s.yp = p; p += n;
+    s.colk = p; p += n;
+    s.bs = p;
+    p = end;
+    if (spill & 1) { s.ROP = g; } else { s.ROP = p; p += N; }
+    if (spill & 2) { s.D = g + N; } else { s.D = p; p += (kMaxOrder + 3) * n; }
+    s.Jsm = nullptr;
+    if (spill & 4) { s.Jsm = p; p += mp.nnz; }
+    s.ysrc = nullptr;
+    s.r1g = g + N + (kMaxOrder + 3) * n;
+    s.r1d = s.r1g + n;
+    s.r1w = s.r1d + n;
+    s.y = p; p += n;
+    s.ypred = p; p += n;
+    s.psi = p; p += n;
+    s.d = p; p += n;
+    s.scale = p; p += n;
+    s.wlu = p; p += n;
+    s.V = nullptr;
+    if (sizeof(LT) == sizeof(float)) {
+      s.V = p;
+      p += (kMaxl + 3) * n;
+    }
+    s.perm = (int *)p; p += (n + 1) / 2 + 1;
+    s.A = p;
   }
-  s.mlp = (float *)p;
-  p += kPredBuf;  // 2 * kPredBuf floats
-  s.perm = (int *)p; p += (n + 1) / 2 + 1;
-  s.A = p;
-  Consts bc;
-  make_consts(bc);
+  __syncthreads();
+  const DevMech &m = ks.m;
+  const IntegOpts &o = ks.o;
+  const Smem &s = ks.s;
+  const Consts &bc = ks.bc;
   __shared__ int next;
   for (;;) {
     if (tid == 0) next = atomicAdd(a.queue_head, 1);
@@ -1152,17 +1186,22 @@ __global__ void __launch_bounds__(512, 1) integrate_dense_kernel(DevMech m, Inte
     for (int k = tid; k < S; k += nt) pa += Y0[k] * m.inv_mw[k];
     const double mwmix = 1.0 / block_sum(pa, s.red);
     const double v = 1.0 / (P0 * mwmix / (kRuD * T0));
-    s.src.dpdt = a.dpdt ? a.dpdt[r] : 0.0;
-    s.src.esrc = a.esrc ? a.esrc[r] : 0.0;
-    s.src.P0 = P0;
-    s.src.ysrc = a.ysrc != nullptr;
-    s.src.fixT = !o.always_T && a.tdel_in && !(a.tdel_in[r] > 0.0);
-    s.src.T0 = T0;
-    s.src.E0 = 0.0;
-    if (s.src.esrc != 0.0 || s.src.fixT) {  // initial_energy_ (InitializeState)
+    ReactorSrc src;
+    src.dpdt = a.dpdt ? a.dpdt[r] : 0.0;
+    src.esrc = a.esrc ? a.esrc[r] : 0.0;
+    src.P0 = P0;
+    src.ysrc = a.ysrc != nullptr;
+    src.fixT = !o.always_T && a.tdel_in && !(a.tdel_in[r] > 0.0);
+    src.T0 = T0;
+    src.E0 = 0.0;
+    if (src.esrc != 0.0 || src.fixT) {  // initial_energy_ (InitializeState)
       double cx;
       mix_energy(m, o.cp != 0, false, T0, Y0, false, 0.0, tid, nt,
-                 [&](double x) { return block_sum(x, s.red); }, s.src.E0, cx);
+                 [&](double x) { return block_sum(x, s.red); }, src.E0, cx);
+    }
+    if (tid == 0) {  // (the barriers of the sum above end the last reactor's reads)
+      ks.s.src = src;
+      ks.s.ysrc = a.ysrc ? a.ysrc + (size_t)r * S : nullptr;
     }
     for (int k = tid; k < S; k += nt) s.y[k] = Y0[k];
     if (tid == 0) s.y[S] = T0 / o.Tref;
@@ -1177,7 +1216,6 @@ __global__ void __launch_bounds__(512, 1) integrate_dense_kernel(DevMech m, Inte
     // max_steps counts per attempt
     double t_left = a.dt, t_ign = -1.0;
     const double T_target = o.dT_ign > 0.0 ? T0 + o.dT_ign : -1.0;
-    s.ysrc = a.ysrc ? a.ysrc + (size_t)r * S : nullptr;
     for (int attempt = 0;; ++attempt) {
       double t_done = 0.0;
       rc = attempt_cta<LT>(m, o, bc, s, J, v, t_left, rtol, atol, rs, lda, t_done, a.dt - t_left,
@@ -1221,6 +1259,12 @@ cudaError_t launch_dense(const DevMech &m, const IntegOpts &o, const IntegArgs &
                          int ctas, int spill, size_t smem, int lda, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(integrate_dense_kernel<LT>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  // shared memory for the CTAs that can be resident (registers: 512 threads
+  // in all), the rest of the SM's 256 KB for L1, which holds the tables
+  const size_t want = (smem + 1024) * std::max(1, 512 / std::max(threads, 1));
+  const int pct = (int)std::min<size_t>(100, (100 * want + 228 * 1024 - 1) / (228 * 1024));
+  e = cudaFuncSetAttribute(integrate_dense_kernel<LT>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
   if (e != cudaSuccess) return e;
   integrate_dense_kernel<LT><<<ctas, threads, smem, stream>>>(m, o, a, lda, spill);
   return cudaGetLastError();

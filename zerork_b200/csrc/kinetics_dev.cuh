@@ -88,8 +88,9 @@ __device__ __forceinline__ const T *rb(const T *p, const char *tab, const unsign
 }
 
 // NASA-7 polynomials (src/zerork/nasa_poly.cpp:50-172), one species, one T.
+// (ld: distance between a species' coefficients)
 __device__ __forceinline__ void nasa_cp_h_g(const double *__restrict__ c, double T, double logT,
-                                            double *cp, double *h, double *g) {
+                                            double *cp, double *h, double *g, int ld = 1) {
   const double invT = 1.0 / T;
   const double m0 = T * 0.50000000000000000000;
   const double T2 = T * T, T3 = T * T2, T4 = T * T3;
@@ -102,8 +103,8 @@ __device__ __forceinline__ void nasa_cp_h_g(const double *__restrict__ c, double
   const double g3 = T3 * -0.08333333333333333333;
   const double g4 = T4 * -0.05000000000000000000;
   const int o = (T < c[0]) ? 1 : 8;
-  const double a1 = c[o], a2 = c[o + 1], a3 = c[o + 2], a4 = c[o + 3], a5 = c[o + 4],
-               a6 = c[o + 5], a7 = c[o + 6];
+  const double a1 = c[o * ld], a2 = c[(o + 1) * ld], a3 = c[(o + 2) * ld], a4 = c[(o + 3) * ld],
+               a5 = c[(o + 4) * ld], a6 = c[(o + 5) * ld], a7 = c[(o + 6) * ld];
   *cp = a1 + T * (a2 + T * (a3 + T * (a4 + T * a5)));
   *h = a1 + a2 * m0 + a3 * m1 + a4 * m2 + a5 * m3 + a6 * invT;
   *g = a1 * g0 + a2 * g1 + a3 * g2 + a4 * g3 + a5 * g4 + a6 * invT - a7;
@@ -230,6 +231,16 @@ __device__ __forceinline__ void each_species(int count, const short *spc, F f) {
     for (int i = 3; i < kMaxSide; ++i)
       if (i < count) f(spc[i]);
   }
+}
+
+// Record `lane` of a block of rxn_slots: six coalesced loads a warp.
+__device__ __forceinline__ RxnRec load_slot(const int4 *slots, int block, int lane) {
+  int4 b[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) b[i] = slots[(block * 6 + i) * 32 + lane];
+  RxnRec R;
+  memcpy(&R, b, sizeof(R));
+  return R;
 }
 
 // Third-body concentration: Csum plus the efficiency list, four entries at a
