@@ -76,9 +76,10 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
         R.flags |= kRevKeq;
       }
     }
-    R.nr = t.reac_ptr[R.fwd + 1] - t.reac_ptr[R.fwd];
-    R.np = t.prod_ptr[R.fwd + 1] - t.prod_ptr[R.fwd];
-    if (R.nr > kMaxSide || R.np > kMaxSide)
+    const int nr = t.reac_ptr[R.fwd + 1] - t.reac_ptr[R.fwd], np = t.prod_ptr[R.fwd + 1] - t.prod_ptr[R.fwd];
+    R.nr = (short)nr;
+    R.np = (short)np;
+    if (nr > kMaxSide || np > kMaxSide)
       throw std::runtime_error("reaction " + std::to_string(j) + " has more than 6 species on a side");
     for (int k = 0; k < R.nr; ++k) R.r[k] = (short)t.reac_spc[t.reac_ptr[R.fwd] + k];
     for (int k = 0; k < R.np; ++k) R.p[k] = (short)t.prod_spc[t.prod_ptr[R.fwd] + k];
@@ -87,15 +88,23 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     int j = t.step_rxn[t.keq_fwd[k]];
     rec[j].lnA_r = t.keq_dn[k];  // dn stored in the reverse slot
   }
+  std::vector<Eff> eff;
+  auto list = [&](RxnRec &R, int b, int e, const std::vector<int> &spc, const std::vector<double> &alpha) {
+    if (e - b > 0x7fff) throw std::runtime_error("efficiency list too long");
+    R.e0 = (int)eff.size();
+    R.ne = (short)(e - b);
+    for (; b < e; ++b) eff.push_back(Eff{alpha[b], spc[b], 0});
+  };
   for (size_t k = 0; k < t.tb_fwd.size(); ++k) {
     int j = t.step_rxn[t.tb_fwd[k]];
     rec[j].flags |= kThirdBody;
-    rec[j].aux = (int)k;
+    list(rec[j], t.tb_ptr[k], t.tb_ptr[k + 1], t.tb_spc, t.tb_alpha);
   }
   for (size_t k = 0; k < t.fo_fwd.size(); ++k) {
     int j = t.step_rxn[t.fo_fwd[k]];
     rec[j].flags |= kFalloff;
     rec[j].aux = (int)k;
+    if (t.fo_spc[k] < 0) list(rec[j], t.fo_ptr[k], t.fo_ptr[k + 1], t.fo_eff_spc, t.fo_alpha);
   }
   // species gather lists, ascending step order (perf_net.cpp:257-267 sum order)
   std::vector<std::vector<int>> sd(ns), sc(ns);
@@ -192,8 +201,8 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     const RxnRec &R = rec[j];
     double c = 1.0 + 0.1 * (R.nr + R.np);
     if (R.flags & (kRevKeq | kRevArr)) c += 1.0;
-    if (R.flags & kThirdBody) c += 0.5 + 0.1 * (t.tb_ptr[R.aux + 1] - t.tb_ptr[R.aux]);
-    if (R.flags & kFalloff) c += 3.0 + 0.1 * (t.fo_ptr[R.aux + 1] - t.fo_ptr[R.aux]);
+    if (R.flags & kThirdBody) c += 0.5 + 0.1 * R.ne;
+    if (R.flags & kFalloff) c += 3.0 + 0.1 * R.ne;
     if (R.flags & kPlog) {
       const int q0 = t.plog_pt_ptr[R.aux], q1 = t.plog_pt_ptr[R.aux + 1];
       c += 2.0 + 0.5 * (t.plog_ln_ptr[q1] - t.plog_ln_ptr[q0]);
@@ -239,14 +248,15 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   std::vector<double> thermo_t(16 * (size_t)ns);
   for (int j = 0; j < ns; ++j)
     for (int c = 0; c < 16; ++c) thermo_t[(size_t)c * ns + j] = t.thermo[16 * (size_t)j + c];
+  std::vector<int4> sn_rec;
+  for (int j : spc_order) sn_rec.push_back(make_int4(j, sn_ptr[j], sn_ptr[j + 1], 0));
   Blob b;
   const size_t h = 16;
   size_t o_rbc = b.add(rec_by_cost, h);
   size_t o_mw = b.add(t.mw, h), o_imw = b.add(inv_mw, h), o_rimw = b.add(ru_inv_mw, h),
          o_th = b.add(t.thermo, h);
-  size_t o_tbp = b.add(t.tb_ptr, h), o_tbs = b.add(t.tb_spc, h), o_tba = b.add(t.tb_alpha, h);
-  size_t o_fop = b.add(t.fo_ptr, h), o_foe = b.add(t.fo_eff_spc, h), o_fot = b.add(t.fo_type, h),
-         o_fos = b.add(t.fo_spc, h), o_foa = b.add(t.fo_alpha, h), o_fopar = b.add(t.fo_par, h);
+  size_t o_eff = b.add(eff, h), o_fot = b.add(t.fo_type, h), o_fos = b.add(t.fo_spc, h),
+         o_fopar = b.add(t.fo_par, h);
   size_t o_plpp = b.add(t.plog_pt_ptr, h), o_pllp = b.add(t.plog_ln_ptr, h), o_plp = b.add(t.plog_p, h),
          o_pllnp = b.add(t.plog_lnp, h), o_pla = b.add(t.plog_lnA, h), o_pls = b.add(t.plog_sgn, h),
          o_pln = b.add(t.plog_n, h), o_plt = b.add(t.plog_Ta, h);
@@ -259,7 +269,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   size_t o_rec = b.add(rec), o_slot = b.add(slot_parts), o_tht = b.add(thermo_t);
   size_t o_jw = b.add(jw), o_jt = b.add(jt), o_jtp = b.add(jt_ptr);
   size_t o_jfc = b.add(jf_col);
-  size_t o_snp = b.add(sn_ptr), o_sns = b.add(sn_step);
+  size_t o_snr = b.add(sn_rec), o_sns = b.add(sn_step);
   size_t o_lr = b.add(p.last_row);
   size_t o_ndp = b.add(nzd_ptr), o_nds = b.add(nzd_step), o_ncp = b.add(nzc_ptr), o_ncs = b.add(nzc_step);
   size_t o_jrp = b.add(jr_ptr), o_jrk = b.add(jr_kk), o_jrc = b.add(jr_col);
@@ -280,14 +290,9 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.ru_inv_mw = (const double *)P(o_rimw);
   view_.thermo = (const double *)P(o_th);
   view_.rxn = (const RxnRec *)P(o_rec);
-  view_.tb_ptr = (const int *)P(o_tbp);
-  view_.tb_spc = (const int *)P(o_tbs);
-  view_.tb_alpha = (const double *)P(o_tba);
-  view_.fo_ptr = (const int *)P(o_fop);
-  view_.fo_spc_eff = (const int *)P(o_foe);
+  view_.eff = (const Eff *)P(o_eff);
   view_.fo_type = (const int *)P(o_fot);
   view_.fo_spc = (const int *)P(o_fos);
-  view_.fo_alpha = (const double *)P(o_foa);
   view_.fo_par = (const double *)P(o_fopar);
   view_.plog_pt_ptr = (const int *)P(o_plpp);
   view_.plog_ln_ptr = (const int *)P(o_pllp);
@@ -301,7 +306,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.sd_step = (const int *)P(o_sds);
   view_.sc_ptr = (const int *)P(o_scp);
   view_.sc_step = (const int *)P(o_scs);
-  view_.sn_ptr = (const int *)P(o_snp);
+  view_.sn_rec = (const int4 *)P(o_snr);
   view_.sn_step = (const int *)P(o_sns);
   view_.col_ptr = (const int *)P(o_cp);
   view_.row_idx = (const int *)P(o_ri);

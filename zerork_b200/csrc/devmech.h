@@ -33,11 +33,17 @@ struct alignas(16) RxnRec {
   double lnA, n, Ta;        // forward (converted units)
   double lnA_r, n_r, Ta_r;  // explicit reverse, or dn in lnA_r for Keq
   int fwd, rev;             // step indices (rev = -1: irreversible)
-  int flags, aux;           // aux: third-body or falloff list index
-  int nr, np;
+  short flags, ne;          // ne efficiencies, from eff[e0] on
+  int aux, e0;              // aux: falloff or PLOG index
+  short nr, np;
   short r[kMaxSide], p[kMaxSide];
 };
 static_assert(sizeof(RxnRec) % 16 == 0, "RxnRec alignment");
+
+struct alignas(16) Eff {
+  double alpha;  // efficiency minus one
+  int spc, pad;
+};
 
 // Plain-pointer view of the device tables (all device addresses).
 struct DevMech {
@@ -46,18 +52,20 @@ struct DevMech {
   const double *mw, *inv_mw, *ru_inv_mw, *thermo;  // thermo: [nsp*16]
   const double *thermo_t;  // the same, coefficient by coefficient: [16][nsp]
   const RxnRec *rxn;
-  const int *tb_ptr, *tb_spc;
-  const double *tb_alpha;
-  const int *fo_ptr, *fo_spc_eff, *fo_type, *fo_spc;
-  const double *fo_alpha, *fo_par;
+  // third-body and falloff efficiencies, one 16-byte entry each
+  const Eff *eff;
+  const int *fo_type, *fo_spc;
+  const double *fo_par;
   // PLOG reactions: distinct pressures per reaction (plog_pt_ptr), Arrhenius
   // lines per pressure (plog_ln_ptr); see MechTables
   const int *plog_pt_ptr, *plog_ln_ptr;
   const double *plog_p, *plog_lnp, *plog_lnA, *plog_sgn, *plog_n, *plog_Ta;
   // species production gather lists (step indices in ascending step order)
   const int *sd_ptr, *sd_step, *sc_ptr, *sc_step;
-  // both lists of a species in one: step | 1 << 31 for a destruction term
-  const int *sn_ptr, *sn_step;
+  // both lists of a species in one, step | 1 << 31 for a destruction term, and
+  // {species, first, end, 0} by decreasing length
+  const int4 *sn_rec;
+  const int *sn_step;
   // Jacobian pattern and per-nonzero gather lists
   const int *col_ptr, *row_idx, *last_row;
   const int *nzd_ptr, *nzd_step, *nzc_ptr, *nzc_step;

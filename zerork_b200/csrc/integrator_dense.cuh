@@ -34,7 +34,8 @@ constexpr size_t kStateBytes = 1600;  // KernelState
 constexpr int kPredBuf = 256;  // widest predictor layer (padded)
 
 struct Smem {
-  double *red;  // 128 slots: block sums [0, 16), the right-hand side's [16, 64), change_D [64, 100)
+  double *red;  // 128 slots: block sums [0, 16), the right-hand side's [16, 64), change_D [64, 100),
+                // Newton norm [100, 116); all of it the inversion's candidates during one
   double *C, *G, *U, *ROP;
   double *D, *y, *f, *f0, *ypred, *psi, *d, *scale, *tmp, *yp;
   void *A;      // n x lda inverse (LT)
@@ -158,12 +159,12 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
   // in its chain)
   double pe = 0.0;
   for (int p0 = tid >> 3; p0 - (lane >> 3) < S; p0 += nt >> 3) {
-    const int k = p0 < S ? m.spc_order[p0] : -1;
+    const int4 rec = m.sn_rec[min(p0, S - 1)];
+    const int k = p0 < S ? rec.x : -1;
     double net = 0.0;
     if (k >= 0) {
-      const int e1 = m.sn_ptr[k + 1];
 #pragma unroll 4
-      for (int e = m.sn_ptr[k] + (lane & 7); e < e1; e += 8) {
+      for (int e = rec.y + (lane & 7); e < rec.z; e += 8) {
         const int st = m.sn_step[e];
         const double r = s.ROP[st & 0x7fffffff];
         net += st < 0 ? -r : r;
@@ -290,15 +291,15 @@ __device__ __noinline__ int jac_cta(const DevMech &m, const IntegOpts &o, const 
 // Blocked Gauss-Jordan in place with partial pivoting, PB columns at a time
 // (Quintana-Orti et al., SIAM J. Sci. Comput. 22 (2001) 1762, with look-ahead
 // and without moving rows):
-//   * warp 0 holds the panel of PB columns in registers (lane l the rows l,
-//     l + 32, ...) and exchanges its PB pivots with warp reductions and
-//     shuffles alone, no block barrier; the columns end as W, the panel's
-//     part of the inverse;
+//   * four warps (one, in smaller CTAs) hold the panel of PB columns in
+//     registers, a row or two a lane, and exchange its PB pivots with one
+//     barrier of their own each; the columns end as W, the panel's part of
+//     the inverse;
 //   * every other column then changes by one rank-PB product,
 //     A_ij = (i a pivot row ? 0 : A_ij) + sum_s W_is R_sj, with R the pivot
 //     rows before the update (copied to s.rows);
-//   * the next panel's columns are updated first, so warp 0 factors them
-//     while the other warps finish the rest.
+//   * the next panel's columns are updated first, so the panel's warps factor
+//     them while the other warps finish the rest.
 // Rows are never swapped: column j's pivot row is noted in perm, unknown j of
 // the inverse sits in that row and the right-hand side is gathered in that
 // order.  Pivots are the largest by the upper word of |a| (20 mantissa bits,
@@ -386,23 +387,111 @@ __device__ __forceinline__ int panel_warp(LT *A, int lda, int n, int k, int pw, 
   return 0;
 }
 
+// The same exchange by warps 0-3 (warp wp the rows 32 wp + lane, and those 128
+// further): every warp offers its largest pivot and that row's panel values in
+// shared memory (cand: 2 x 4 slots of PB + 1 doubles, used in turn), and one
+// barrier of the four warps a pivot settles which one it is.
+template <class LT, int RP, int PB>
+__device__ __forceinline__ int panel_four(LT *A, int lda, int n, int k, int pw, int *perm, unsigned &used,
+                                          double *cand) {
+  constexpr unsigned kInf = sizeof(LT) == 8 ? 0x7ff00000u : 0x7f800000u;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, row0 = threadIdx.x;
+  LT a[RP][PB];
+#pragma unroll
+  for (int r = 0; r < RP; ++r)
+#pragma unroll
+    for (int c = 0; c < PB; ++c)
+      a[r][c] = (row0 + 128 * r < n && c < pw) ? A[(row0 + 128 * r) * lda + k + c] : (LT)0;
+#pragma unroll 1
+  for (int t = 0; t < pw; ++t) {
+    unsigned key = 0, row = 0xffffffffu;
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const unsigned q = pivot_key(a[r][0]);
+      if ((!(used >> r & 1) || q >= kInf) && q > key) {  // (rows past n hold zeros)
+        key = q;
+        row = row0 + 128 * r;
+      }
+    }
+    double *slots = cand + (t & 1) * 4 * (PB + 1);
+    const unsigned wbest = __reduce_max_sync(kFull, key);
+    const unsigned wrow = __reduce_min_sync(kFull, key == wbest ? row : 0xffffffffu);
+    if (lane == 0) reinterpret_cast<uint2 *>(slots + wp * (PB + 1) + PB)[0] = make_uint2(wbest, wrow);
+#pragma unroll
+    for (int r = 0; r < RP; ++r)
+      if (row0 + 128 * r == (int)wrow)
+#pragma unroll
+        for (int c = 0; c < PB; ++c) slots[wp * (PB + 1) + c] = (double)a[r][c];
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    unsigned best = 0, p = 0xffffffffu;
+    int bw = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // rows of a warp lie between those of others: compare them too
+      const uint2 o = reinterpret_cast<const uint2 *>(slots + i * (PB + 1) + PB)[0];
+      if (o.x > best || (o.x == best && o.y < p)) {
+        best = o.x;
+        p = o.y;
+        bw = i;
+      }
+    }
+    if (best == 0 || best >= kInf) return 1;  // all four warps alike
+    LT v[PB];
+#pragma unroll
+    for (int c = 0; c < PB; ++c) v[c] = (LT)slots[bw * (PB + 1) + c];
+    v[0] = (LT)1 / v[0];
+#pragma unroll
+    for (int c = 1; c < PB; ++c) v[c] *= v[0];
+#pragma unroll
+    for (int r = 0; r < RP; ++r) {
+      const LT f = a[r][0];
+      const bool pr = row0 + 128 * r == (int)p;
+#pragma unroll
+      for (int c = 1; c < PB; ++c) {
+        const LT e = a[r][c] - f * v[c];
+        a[r][c - 1] = pr ? v[c] : e;
+      }
+      a[r][PB - 1] = pr ? v[0] : -f * v[0];
+      if (pr) {
+        used |= 1u << r;
+        reinterpret_cast<short *>(perm + k + t)[0] = (short)p;
+        reinterpret_cast<short *>(perm + p)[1] = (short)(k + t);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < PB; ++c) {
+    const int oc = c + pw - (c + pw >= PB ? PB : 0);  // the column at place c after pw rotations
+#pragma unroll
+    for (int r = 0; r < RP; ++r)
+      if (row0 + 128 * r < n && oc < pw) A[(row0 + 128 * r) * lda + k + oc] = a[r][c];
+  }
+  return 0;
+}
+
 __device__ __forceinline__ int pivot_row(const int *perm, int j) { return perm[j] & 0xffff; }
 __device__ __forceinline__ int pivot_col(const int *perm, int i) { return perm[i] >> 16; }
 
-template <class LT, int NC, int PB>
+// SH: the matrix and the pivot order are in shared memory.
+template <class LT, int NC, int PB, bool SH>
 __device__ __noinline__ int invert_cta(const DevMech &m, const Smem &s, const double *J, double c, int n,
                                        int lda) {
   LT *A = (LT *)s.A;
   LT *R = (LT *)s.rows;
+  int *perm = s.perm;
+  __builtin_assume(__isShared(R));
+  if constexpr (SH) {
+    __builtin_assume(__isShared(A));
+    __builtin_assume(__isShared(perm));
+  }
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
   for (int i = tid; i < n * lda; i += nt) A[i] = (LT)0;
   for (int i = tid; i < n; i += nt) {
     const double sc = s.scale[i];
     s.wlu[i] = sc;
     s.rows[i] = -c / sc;
-    s.perm[i] = -1;  // no pivot yet: pivot_col < 0
+    perm[i] = -1;  // no pivot yet: pivot_col < 0
   }
-  if (tid == 0) s.perm[n] = 0;
+  if (tid == 0) perm[n] = 0;
   __syncthreads();
 #pragma unroll 4
   for (int q = tid; q < m.nnz; q += nt) {
@@ -414,14 +503,21 @@ __device__ __noinline__ int invert_cta(const DevMech &m, const Smem &s, const do
   for (int i = tid; i < n; i += nt) A[i * lda + i] += (LT)1;
   __syncthreads();
   unsigned used = 0;
-  if (w == 0 && panel_warp<LT, NC, PB>(A, lda, n, 0, min(PB, n), s.perm, used)) s.perm[n] = 1;
+  const int np = nw >= 4 ? 4 : 1;  // the panel's warps
+  auto panel = [&](int k, int pw) {
+    if (w >= np) return;
+    const int bad = np == 4 ? panel_four<LT, (NC + 3) / 4, PB>(A, lda, n, k, pw, perm, used, s.red)
+                            : panel_warp<LT, NC, PB>(A, lda, n, k, pw, perm, used);
+    if (bad) perm[n] = 1;
+  };
+  panel(0, min(PB, n));
   __syncthreads();
-  for (int k = 0; k < n && !s.perm[n]; k += PB) {
+  for (int k = 0; k < n && !perm[n]; k += PB) {
     const int pw = min(PB, n - k), k2 = k + pw, pw2 = min(PB, n - k2);
-    auto in_panel = [&](int i) { return (unsigned)(pivot_col(s.perm, i) - k) < (unsigned)pw; };
+    auto in_panel = [&](int i) { return (unsigned)(pivot_col(perm, i) - k) < (unsigned)pw; };
     for (int q = tid; q < pw * n; q += nt) {  // the pivot rows before the update
       const int t = q / n, j = q - t * n;
-      R[q] = A[pivot_row(s.perm, k + t) * lda + j];
+      R[q] = A[pivot_row(perm, k + t) * lda + j];
     }
     __syncthreads();
     if (pw2 > 0) {
@@ -437,9 +533,10 @@ __device__ __noinline__ int invert_cta(const DevMech &m, const Smem &s, const do
       __syncthreads();
     }
     const bool ahead = pw2 > 0;
-    if (ahead && w == 0 && panel_warp<LT, NC, PB>(A, lda, n, k2, pw2, s.perm, used)) s.perm[n] = 1;
-    if (!ahead || w > 0 || nw == 1) {  // the remaining columns, three 32-wide chunks at a time
-      const int i0 = (ahead && nw > 1) ? w - 1 : w, di = (ahead && nw > 1) ? nw - 1 : nw;
+    if (ahead) panel(k2, pw2);
+    const bool apart = ahead && nw > np;
+    if (!apart || w >= np) {  // the remaining columns, three 32-wide chunks at a time
+      const int i0 = apart ? w - np : w, di = apart ? nw - np : nw;
       constexpr int CH = NC < 3 ? NC : 3;
       for (int c0 = 0; c0 < NC; c0 += CH) {
         LT r[PB][CH];
@@ -474,38 +571,38 @@ __device__ __noinline__ int invert_cta(const DevMech &m, const Smem &s, const do
     }
     __syncthreads();
   }
-  return __syncthreads_or(s.perm[n]);
+  return __syncthreads_or(perm[n]);
 }
 
 // invert_cta for the register-chunk count nc = ceil(n / 32) (1..8).
-template <class LT>
+template <class LT, bool SH>
 __device__ __forceinline__ int invert_any(int nc, const DevMech &m, const Smem &s, const double *J,
                                           double c, int n, int lda) {
   constexpr bool F64 = sizeof(LT) == 8;
   switch (nc) {
-    case 1: return invert_cta<LT, 1, 8>(m, s, J, c, n, lda);
-    case 2: return invert_cta<LT, 2, 8>(m, s, J, c, n, lda);
-    case 3: return invert_cta<LT, 3, 8>(m, s, J, c, n, lda);
-    case 4: return invert_cta<LT, 4, 8>(m, s, J, c, n, lda);
+    case 1: return invert_cta<LT, 1, 8, SH>(m, s, J, c, n, lda);
+    case 2: return invert_cta<LT, 2, 8, SH>(m, s, J, c, n, lda);
+    case 3: return invert_cta<LT, 3, 8, SH>(m, s, J, c, n, lda);
+    case 4: return invert_cta<LT, 4, 8, SH>(m, s, J, c, n, lda);
     case 5:
-    case 6: return invert_cta<LT, 6, F64 ? 6 : 8>(m, s, J, c, n, lda);
-    default: return invert_cta<LT, 8, F64 ? 4 : 8>(m, s, J, c, n, lda);
+    case 6: return invert_cta<LT, 6, F64 ? 6 : 8, SH>(m, s, J, c, n, lda);
+    default: return invert_cta<LT, 8, F64 ? 4 : 8, SH>(m, s, J, c, n, lda);
   }
 }
 
-// x = (I - c_lu J)^{-1} b with the stored inverse: x = W A (pivot order of
-// W^-1 b), the rows of A in pivot order.  Eight lanes a row, each a contiguous
-// share of its columns, and up to three rows a thread that share every
-// right-hand-side load; a share of 2 (mod 4) columns and the odd row stride
-// put the lanes of two neighbouring rows in different banks.
-template <class LT>
-__device__ void apply_inverse(const Smem &s, int n, int lda, const double *b, double *x) {
+// y = A bs with the stored inverse (rows in pivot order), put(k, y_k) called by
+// one thread for each unknown k.  Eight lanes a row, each a contiguous share of
+// its columns, and up to three rows a thread that share every right-hand-side
+// load; a share of 2 (mod 4) columns and the odd row stride put the lanes of
+// two neighbouring rows in different banks.  The caller's barrier precedes it.
+template <class LT, class F>
+__device__ __forceinline__ void inverse_times_bs(const Smem &s, int n, int lda, F put) {
   const LT *A = (const LT *)s.A;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int pi = pivot_row(s.perm, i);
-    s.bs[i] = b[pi] / s.wlu[pi];
-  }
-  __syncthreads();
+  const double *bs = s.bs;
+  const int *perm = s.perm;
+  __builtin_assume(__isShared(A));
+  __builtin_assume(__isShared(bs));
+  __builtin_assume(__isShared(perm));
   int share = (n + 7) >> 3;
   share += (6 - (share & 3)) & 3;  // the next 2 (mod 4)
   const int g = threadIdx.x & 7, nr = blockDim.x >> 3;
@@ -517,9 +614,9 @@ __device__ void apply_inverse(const Smem &s, int n, int lda, const double *b, do
     const LT *row[3];
 #pragma unroll
     for (int e = 0; e < 3; ++e) row[e] = A + min(p[e], n - 1) * lda;
-#pragma unroll 2
+#pragma unroll 4
     for (int j = j0; j < j1; ++j) {
-      const double v = s.bs[j];
+      const double v = bs[j];
 #pragma unroll
       for (int e = 0; e < 3; ++e) acc[e] += (double)row[e][j] * v;
     }
@@ -527,14 +624,19 @@ __device__ void apply_inverse(const Smem &s, int n, int lda, const double *b, do
     for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
       for (int e = 0; e < 3; ++e) acc[e] += __shfl_xor_sync(kFull, acc[e], o);
-    if (g == 0)
 #pragma unroll
-      for (int e = 0; e < 3; ++e)
-        if (p[e] < n) {
-          const int k = pivot_col(s.perm, p[e]);
-          x[k] = acc[e] * s.wlu[k];
-        }
+    for (int e = 0; e < 3; ++e)
+      if (g == e && p[e] < n) put(pivot_col(perm, p[e]), acc[e]);
   }
+}
+
+// x = (I - c_lu J)^{-1} b with the stored inverse: x = W A (pivot order of
+// W^-1 b).
+template <class LT>
+__device__ void apply_inverse(const Smem &s, int n, int lda, const double *b, double *x) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s.bs[pivot_col(s.perm, i)] = b[i] / s.wlu[i];
+  __syncthreads();
+  inverse_times_bs<LT>(s, n, lda, [&](int k, double y) { x[k] = y * s.wlu[k]; });
   __syncthreads();
 }
 
@@ -861,7 +963,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
   st.njac++;
   if (jac_cta(m, o, s, v, t_off, s.y, s.f0, J)) { rc = -2; goto failed; }
   st.nlu++;
-  if (invert_any<LT>(nc, m, s, J, c_lu, n, lda)) { rc = -3; goto failed; }
+  if (invert_any<LT, true>(nc, m, s, J, c_lu, n, lda)) { rc = -3; goto failed; }
   rank1_setup(c_lu);
   while (t < t_end) {
     if (nsteps >= o.max_steps) { rc = -4; goto failed; }
@@ -885,9 +987,15 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
       if (!(t + h > t)) { rc = -5; goto failed; }
       const double t_new = t + h;
       for (int i = tid; i < n; i += nt) {
-        double a = 0.0, ps = 0.0;
-        for (int k = 0; k <= q; ++k) a += s.D[k * n + i];
-        for (int k = 1; k <= q; ++k) ps += bc.gam[k] * s.D[k * n + i];
+        double a = 0.0, ps = 0.0, dk[kMaxOrder + 1];
+#pragma unroll
+        for (int k = 0; k <= kMaxOrder; ++k) dk[k] = k <= q ? s.D[k * n + i] : 0.0;  // loads together
+#pragma unroll
+        for (int k = 0; k <= kMaxOrder; ++k)
+          if (k <= q) {
+            a += dk[k];
+            if (k > 0) ps += bc.gam[k] * dk[k];
+          }
         s.ypred[i] = a;
         s.psi[i] = ps / bc.alp[q];
         s.scale[i] = atol_of(i) + rtol * fabs(a);
@@ -904,7 +1012,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
         st.nlu++;
         c_lu = c;
         crate = 1.0;
-        if (invert_any<LT>(nc, m, s, J, c, n, lda)) { rc = -3; goto failed; }
+        if (invert_any<LT, true>(nc, m, s, J, c, n, lda)) { rc = -3; goto failed; }
         rank1_setup(c);
       }
       const double gscale = (c == c_lu) ? 1.0 : 2.0 / (1.0 + c / c_lu);
@@ -914,16 +1022,36 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
       for (it = 0; it < kNewtonMaxIter; ++it) {
         st.nrhs++;
         if (rhs_cta(m, o, s, v, t_off + t_new, s.y, s.f, false, nullptr)) break;
+        // residual c f - psi - d; on the FP64 path straight into the inverse's
+        // order, and the correction goes from the product to the iterate and
+        // its norm without a pass of its own
+        constexpr bool kDirect = sizeof(LT) == sizeof(double);
         int bad = 0;
-        for (int i = tid; i < n; i += nt) bad |= !isfinite(s.f[i]);
+        for (int i = tid; i < n; i += nt) {
+          const double f = s.f[i], r = c * f - s.psi[i] - s.d[i];
+          bad |= !isfinite(f);
+          s.tmp[i] = r;
+          if (kDirect) s.bs[pivot_col(s.perm, i)] = r / s.wlu[i];
+        }
         if (__syncthreads_or(bad)) break;
-        if (it == 0)
-          for (int i = tid; i < n; i += nt) s.f0[i] = s.f[i];
         st.nnewt++;
-        for (int i = tid; i < n; i += nt) s.tmp[i] = c * s.f[i] - s.psi[i] - s.d[i];
-        __syncthreads();
-        double gs = gscale;
-        if constexpr (sizeof(LT) == sizeof(float)) {
+        double a = 0.0;
+        auto correct = [&](int i, double dy) {
+          s.y[i] += dy;
+          s.d[i] += dy;
+          const double tt = dy / s.scale[i];
+          a += tt * tt;
+        };
+        if constexpr (kDirect) {
+          if (s.src.esrc == 0.0) {
+            inverse_times_bs<LT>(s, n, lda, [&](int k, double y) { correct(k, y * s.wlu[k] * gscale); });
+          } else {
+            inverse_times_bs<LT>(s, n, lda, [&](int k, double y) { s.yp[k] = y * s.wlu[k]; });
+            __syncthreads();
+            rank1_fix(s, n, r1k, s.yp);
+            for (int i = tid; i < n; i += nt) correct(i, s.yp[i] * gscale);
+          }
+        } else {
           // Krylov tolerance eps_lin * nlscoef / error constant (WRMS), as a
           // weighted 2-norm.  Unlike CVODE, which accepts a reduced but
           // unconverged residual on the first Newton iteration, every solve
@@ -932,20 +1060,10 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
           // and a failure here costs only a Jacobian update or a step cut.
           const double delta = o.eps_lin * o.nlscoef / bc.econ[q] * sqrt((double)n);
           if (gmres_cta<LT>(m, s, J, c, n, lda, delta, s.tmp, s.yp, st.nkry, r1k) != 0) break;
-          gs = 1.0;  // the Krylov solve uses the current c exactly
-        } else {
-          apply_inverse<LT>(s, n, lda, s.tmp, s.yp);
-          if (s.src.esrc != 0.0) rank1_fix(s, n, r1k, s.yp);
+          // (the Krylov solve uses the current c exactly)
+          for (int i = tid; i < n; i += nt) correct(i, s.yp[i]);
         }
-        double a = 0.0;
-        for (int i = tid; i < n; i += nt) {
-          const double dy = s.yp[i] * gs;
-          s.y[i] += dy;
-          s.d[i] += dy;
-          const double tt = dy / s.scale[i];
-          a += tt * tt;
-        }
-        const double dn = sqrt(block_sum(a, s.red) / n);
+        const double dn = sqrt(block_sum_at(a, s.red + 100) / n);
         if (dnorm_old > 0.0) crate = fmax(0.3 * crate, dn / dnorm_old);
         // from a learned starting iterate, convergence is only declared on
         // the last correction itself (two iterations at least): neither the
@@ -975,7 +1093,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
           st.nlu++;
           c_lu = c;
           crate = 1.0;
-          if (invert_any<LT>(nc, m, s, J, c, n, lda)) { rc = -3; goto failed; }
+          if (invert_any<LT, true>(nc, m, s, J, c, n, lda)) { rc = -3; goto failed; }
           rank1_setup(c);
           continue;
         }
@@ -1028,9 +1146,18 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
     for (int i = tid; i < n; i += nt) {
       if (keep_prev) s.tmp[i] = s.D[i];  // the previous accepted state
       const double di = s.d[i];
+      double dk[kMaxOrder + 1];
+#pragma unroll
+      for (int k = 0; k <= kMaxOrder; ++k) dk[k] = k <= q ? s.D[k * n + i] : 0.0;
       s.D[(q + 2) * n + i] = di - s.D[(q + 1) * n + i];
       s.D[(q + 1) * n + i] = di;
-      for (int k = q; k >= 0; --k) s.D[k * n + i] += s.D[(k + 1) * n + i];
+      double up = di;
+#pragma unroll
+      for (int k = kMaxOrder; k >= 0; --k)
+        if (k <= q) {
+          up += dk[k];
+          s.D[k * n + i] = up;
+        }
     }
     __syncthreads();
     if (T_target > 0.0) {  // first crossing of T0 + dT_ign, linear between accepted steps

@@ -144,7 +144,7 @@ __device__ int factor_g(const GroupKArgs &k, Bound &b, double c, double *smem_A)
   const int n = k.m.nsp + 1, nc = (n + 31) / 32;
   Smem s = b.s;
   if (smem_A) s.A = smem_A;
-  const int bad = invert_any<double>(nc, k.m, s, b.J, c, n, k.lda);
+  const int bad = invert_any<double, false>(nc, k.m, s, b.J, c, n, k.lda);
   if (smem_A && !bad) {
     for (int i = threadIdx.x; i < n * k.lda; i += blockDim.x) b.A[i] = smem_A[i];
     __syncthreads();

@@ -243,33 +243,27 @@ __device__ __forceinline__ RxnRec load_slot(const int4 *slots, int block, int la
   return R;
 }
 
-// Third-body concentration: Csum plus the efficiency list, four entries at a
-// time (the table loads are independent of the sums, which keep the list
-// order).
+// Third-body concentration: Csum plus the record's efficiency list, four
+// entries at a time (the table loads are independent of the sums, which keep
+// the list order).
 template <int TS, int V>
-__device__ __forceinline__ void third_body(const int *__restrict__ spc, const double *__restrict__ alpha, int e0, int e1,
-                                           int q, const double *__restrict__ sC, const double *Csum, double *Cm) {
+__device__ __forceinline__ void third_body(const Eff *__restrict__ eff, int ne, int q, const double *__restrict__ sC,
+                                           const double *Csum, double *Cm) {
 #pragma unroll
   for (int k = 0; k < V; ++k) Cm[k] = Csum[k];
-  int e = e0;
-  for (; e + 3 < e1; e += 4) {
+  for (int e = 0; e < ne; e += 4) {
     double a[4], c[4][V];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      a[i] = alpha[e + i];
-      ldv<V>(sC + spc[e + i] * TS + q, c[i]);
+      const Eff f = eff[min(e + i, ne - 1)];
+      a[i] = e + i < ne ? f.alpha : 0.0;
+      ldv<V>(sC + f.spc * TS + q, c[i]);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
+      if (e + i < ne)
 #pragma unroll
-      for (int k = 0; k < V; ++k) Cm[k] += c[i][k] * a[i];
-  }
-  for (; e < e1; ++e) {
-    const double a = alpha[e];
-    double c[V];
-    ldv<V>(sC + spc[e] * TS + q, c);
-#pragma unroll
-    for (int k = 0; k < V; ++k) Cm[k] += c[k] * a;
+        for (int k = 0; k < V; ++k) Cm[k] += c[i][k] * a[i];
   }
 }
 
@@ -316,8 +310,7 @@ __device__ __forceinline__ void reaction_eval(const DevMech &m, const RxnRec &R,
   }
   if (R.flags & kThirdBody) {
     double Cm[V];
-    const int *tp = rb(m.tb_ptr, tab, m.base);
-    third_body<TS, V>(rb(m.tb_spc, tab, m.base), rb(m.tb_alpha, tab, m.base), tp[R.aux], tp[R.aux + 1], q, sC, Csum, Cm);
+    third_body<TS, V>(rb(m.eff, tab, m.base) + R.e0, R.ne, q, sC, Csum, Cm);
 #pragma unroll
     for (int k = 0; k < V; ++k) {
       kf[k] *= Cm[k];
@@ -336,8 +329,7 @@ __device__ __forceinline__ void reaction_eval(const DevMech &m, const RxnRec &R,
     if (fs >= 0) {
       ldv<V>(sC + fs * TS + q, Cm);
     } else {
-      const int *fp = rb(m.fo_ptr, tab, m.base);
-      third_body<TS, V>(rb(m.fo_spc_eff, tab, m.base), rb(m.fo_alpha, tab, m.base), fp[f], fp[f + 1], q, sC, Csum, Cm);
+      third_body<TS, V>(rb(m.eff, tab, m.base) + R.e0, R.ne, q, sC, Csum, Cm);
     }
     double Pr[V], fT[V];
 #pragma unroll
