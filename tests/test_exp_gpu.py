@@ -1,8 +1,9 @@
-"""The kernels' branch-free exponential and interleaved quotients
+"""The kernels' interleaved exponentials, logarithms and quotients
 (zerork_b200/csrc/kinetics_dev.cuh) against extended precision.
 
 Bounds: the exponential's polynomial is truncated at 4e-18, its argument
 reduction and the last two roundings cost at most one unit in the last place;
+a logarithm's three roundings of its leading parts at most two;
 a quotient corrected by its residual is within one unit, and outside the fast
 range it is the language's division, bit for bit.
 """
@@ -19,17 +20,20 @@ pytestmark = pytest.mark.gpu
 
 SRC = r"""
 #include "kinetics_dev.cuh"
-__global__ void k(int n, const double *a, const double *d, double *e, double *q) {
+__global__ void k(int n, const double *a, const double *d, double *e, double *q, double *l) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  e[i] = zrk::exp_tree(a[i]);
   const double x[1] = {a[i]}, y[1] = {d[i]};
   double z[1];
+  zrk::exps<1>(x, z);
+  e[i] = z[0];
   zrk::quotients<1>(x, y, z);
   q[i] = z[0];
+  zrk::logs<1>(x, z);
+  l[i] = z[0];
 }
-extern "C" int run(int n, const double *a, const double *d, double *e, double *q) {
-  k<<<(n + 255) / 256, 256>>>(n, a, d, e, q);
+extern "C" int run(int n, const double *a, const double *d, double *e, double *q, double *l) {
+  k<<<(n + 255) / 256, 256>>>(n, a, d, e, q, l);
   return (int)cudaDeviceSynchronize();
 }
 """
@@ -49,9 +53,9 @@ def probe(tmp_path_factory):
     lib = C.CDLL(so)
 
     def run(a, den):
-        t = [torch.from_numpy(np.ascontiguousarray(x, np.float64)).cuda() for x in (a, den, a, a)]
+        t = [torch.from_numpy(np.ascontiguousarray(x, np.float64)).cuda() for x in (a, den, a, a, a)]
         assert lib.run(len(a), *[C.c_void_p(x.data_ptr()) for x in t]) == 0
-        return t[2].cpu().numpy(), t[3].cpu().numpy()
+        return [x.cpu().numpy() for x in t[2:]]
 
     return run
 
@@ -63,13 +67,13 @@ def _ulps(x, exact):
 @pytest.mark.parametrize("lo,hi", [(-1e-6, 1e-6), (-1.0, 1.0), (-50.0, 50.0), (-700.0, 709.0)])
 def test_exp(probe, lo, hi):
     x = np.random.default_rng(1).uniform(lo, hi, 200001)
-    e, _ = probe(x, np.ones_like(x))
+    e, _, _ = probe(x, np.ones_like(x))
     assert _ulps(e, np.exp(x.astype(np.longdouble))) <= 1.0
 
 
 def test_exp_ends(probe):
     x = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 709.78, 709.79, 1e300, -1e300, -745.0, -746.0, -720.0, 750.0])
-    e, _ = probe(x, np.ones_like(x))
+    e, _, _ = probe(x, np.ones_like(x))
     with np.errstate(over="ignore", under="ignore"):
         r = np.exp(x)
     assert np.array_equal(np.isnan(e), np.isnan(r)) and np.array_equal(np.isinf(e), np.isinf(r))
@@ -77,15 +81,27 @@ def test_exp_ends(probe):
     assert np.all(np.abs(e[ok] - r[ok]) <= np.maximum(np.spacing(r[ok]), 5e-324))
 
 
+def test_logs(probe):
+    r = np.random.default_rng(3)
+    x = np.concatenate([2.0 ** r.uniform(-1020, 1020, 100001), r.uniform(0.4, 2.5, 100001), 1.0 + r.uniform(-1e-6, 1e-6, 9999)])
+    _, _, l = probe(x, np.ones_like(x))
+    assert _ulps(l, np.log(x.astype(np.longdouble))) <= 2.0
+    x = np.array([1.0, 0.0, -1.0, np.inf, np.nan, 5e-324, 1e-310])
+    _, _, l = probe(x, np.ones_like(x))
+    with np.errstate(all="ignore"):
+        assert np.allclose(l, np.log(x), rtol=4e-16, atol=0.0, equal_nan=True)
+
+
 def test_quotients(probe):
     r = np.random.default_rng(2)
     a = r.choice([-1.0, 1.0], 200001) * 2.0 ** r.uniform(-700, 700, 200001)
     d = r.choice([-1.0, 1.0], 200001) * 2.0 ** r.uniform(-700, 700, 200001)
-    d = np.where(np.abs(np.log2(np.abs(a / d))) < 1000, d, np.sign(d))
-    _, q = probe(a, d)
+    with np.errstate(all="ignore"):
+        d = np.where(np.abs(np.log2(np.abs(a / d))) < 1000, d, np.sign(d))
+    _, q, _ = probe(a, d)
     assert _ulps(q, a.astype(np.longdouble) / d.astype(np.longdouble)) <= 1.0
     ends = np.array([0.0, -0.0, 1.0, 5e-324, 1e-310, 1e-250, 1e250, 1.7e308, np.inf, -np.inf, np.nan])
     a, d = (x.ravel() for x in np.meshgrid(ends, ends))
-    _, q = probe(a, d)
+    _, q, _ = probe(a, d)
     with np.errstate(all="ignore"):
         assert np.array_equal(q, a / d, equal_nan=True)

@@ -250,13 +250,19 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     for (int c = 0; c < 16; ++c) thermo_t[(size_t)c * ns + j] = t.thermo[16 * (size_t)j + c];
   std::vector<int4> sn_rec;
   for (int j : spc_order) sn_rec.push_back(make_int4(j, sn_ptr[j], sn_ptr[j + 1], 0));
+  // Troe's -1 / T*** and -1 / T* in their places (0 where the term is absent)
+  std::vector<double> fo_par(t.fo_par);
+  for (size_t k = 0; k < t.fo_type.size(); ++k)
+    if (t.fo_type[k] == kTroe3 || t.fo_type[k] == kTroe4)
+      for (int i : {4, 5})
+        if (fo_par[8 * k + i] != 0.0) fo_par[8 * k + i] = -1.0 / fo_par[8 * k + i];
   Blob b;
   const size_t h = 16;
   size_t o_rbc = b.add(rec_by_cost, h);
   size_t o_mw = b.add(t.mw, h), o_imw = b.add(inv_mw, h), o_rimw = b.add(ru_inv_mw, h),
          o_th = b.add(t.thermo, h);
   size_t o_eff = b.add(eff, h), o_fot = b.add(t.fo_type, h), o_fos = b.add(t.fo_spc, h),
-         o_fopar = b.add(t.fo_par, h);
+         o_fopar = b.add(fo_par, h);
   size_t o_plpp = b.add(t.plog_pt_ptr, h), o_pllp = b.add(t.plog_ln_ptr, h), o_plp = b.add(t.plog_p, h),
          o_pllnp = b.add(t.plog_lnp, h), o_pla = b.add(t.plog_lnA, h), o_pls = b.add(t.plog_sgn, h),
          o_pln = b.add(t.plog_n, h), o_plt = b.add(t.plog_Ta, h);

@@ -55,7 +55,7 @@ struct DevMech {
   // third-body and falloff efficiencies, one 16-byte entry each
   const Eff *eff;
   const int *fo_type, *fo_spc;
-  const double *fo_par;
+  const double *fo_par;  // 8 a reaction: the loader's, with -1 / T for Troe's T*** and T*
   // PLOG reactions: distinct pressures per reaction (plog_pt_ptr), Arrhenius
   // lines per pressure (plog_ln_ptr); see MechTables
   const int *plog_pt_ptr, *plog_ln_ptr;

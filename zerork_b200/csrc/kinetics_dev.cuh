@@ -14,62 +14,109 @@ constexpr double kPatmD = 1.01325e5;    // src/zerork/constants.h:12
 
 constexpr double kLnPatmRu = 2.50033668997960945;  // ln(kPatmD / kRuD)
 
-// exp(x) without branches, so that the calls of independent states and steps
-// interleave (the library's function ends in a branch, behind which the next
-// call's chain of some twenty dependent operations has to wait): Cody and
-// Waite's reduction by ln 2 in two parts (Software Manual for the Elementary
-// Functions, 1980), the Taylor polynomial of degree 13 on |r| <= ln 2 / 2
-// (remainder 4e-18) summed as a tree, and 2^n in two factors, which covers
-// overflow to infinity and gradual underflow.  NaN passes through.  Within one
-// ulp of the correctly rounded value (tests/test_exp_gpu.py).
-__device__ __forceinline__ double exp_tree(double x) {
-  x = x > 720.0 ? 720.0 : x;    // infinity from 710 on
-  x = x < -760.0 ? -760.0 : x;  // zero below -746
-  const double big = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
-  const double t = fma(x, 1.4426950408889634074, big), k = t - big;
-  const int n = __double2loint(t), n1 = n >> 1;
-  double r = fma(k, -0.69314718055994530942, x);
-  r = fma(k, -2.3190468138462995584e-17, r);  // ln 2 minus its nearest double
-  const double r2 = r * r, r4 = r2 * r2, r8 = r4 * r4;
-  const double a = fma(1.0 / 6.0, r, 0.5), b = fma(1.0 / 120.0, r, 1.0 / 24.0);
-  const double c = fma(1.0 / 5040.0, r, 1.0 / 720.0), d = fma(1.0 / 362880.0, r, 1.0 / 40320.0);
-  const double e = fma(1.0 / 39916800.0, r, 1.0 / 3628800.0), f = fma(1.0 / 6227020800.0, r, 1.0 / 479001600.0);
-  const double lo = fma(b, r2, a), mid = fma(d, r2, c), hi = fma(f, r2, e);
-  const double q = fma(hi, r8, fma(mid, r4, lo));
-  const double p = 1.0 + fma(r2, q, r);
-  return p * __hiloint2double((n1 + 1023) << 20, 0) * __hiloint2double((n - n1 + 1023) << 20, 0);
-}
+// Transcendental functions and divisions of K independent arguments side by
+// side.  The library's functions and the language's division end in a branch,
+// behind which the next call's chain of some twenty dependent operations has
+// to wait; here one test covers all K arguments, the chains behind it have no
+// branch and interleave, and arguments out of the fast range take the library's
+// way.
 
-// q[i] = a[i] / d[i].  When every operand is well inside the range of
-// doubles: a reciprocal from the hardware's approximation by one cubic
-// iteration, and the quotient corrected by its residual (Markstein, IA-64 and
-// Elementary Functions, 2000), all K interleaved; otherwise the language's
-// division.
+// Reciprocal of a mid-range number to some 39 bits: the hardware's approximation
+// and one cubic iteration.  A quotient corrected once by its residual is then
+// good to the last place (Markstein, IA-64 and Elementary Functions, 2000).
+__device__ __forceinline__ double recip(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
 __device__ __forceinline__ bool mid_range(double x) {
   return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 300u < 1440u;  // 2^-723 <= |x| < 2^717
 }
+__device__ __forceinline__ bool not_huge(double x) {
+  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) < 1740u;  // |x| < 2^717, not NaN
+}
+
+// q[i] = a[i] / d[i]: the quotient corrected by its residual (Markstein).
 template <int K>
 __device__ __forceinline__ void quotients(const double (&a)[K], const double (&d)[K], double (&q)[K]) {
   bool ok = true;
 #pragma unroll
-  for (int i = 0; i < K; ++i) ok = ok && mid_range(a[i]) && mid_range(d[i]);
+  for (int i = 0; i < K; ++i) ok = ok && not_huge(a[i]) && mid_range(d[i]);
   if (ok) {
-    double y[K];
-#pragma unroll
-    for (int i = 0; i < K; ++i) asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y[i]) : "d"(d[i]));
 #pragma unroll
     for (int i = 0; i < K; ++i) {
-      const double e = fma(-d[i], y[i], 1.0);
-      y[i] = fma(y[i], fma(e, e, e), y[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      const double g = a[i] * y[i];
-      q[i] = fma(fma(-d[i], g, a[i]), y[i], g);
+      const double y = recip(d[i]), g = a[i] * y;
+      q[i] = fma(fma(-d[i], g, a[i]), y, g);
     }
   } else {
 #pragma unroll
     for (int i = 0; i < K; ++i) q[i] = a[i] / d[i];
+  }
+}
+
+// y[i] = exp(x[i]), fast for |x| < 700: Cody and Waite's reduction by ln 2 in
+// two parts (Software Manual for the Elementary Functions, 1980), the Taylor
+// polynomial of degree 13 on |r| <= ln 2 / 2 (remainder 4e-18) summed as a
+// tree, and the exponent added.  Within an ulp (tests/test_exp_gpu.py).
+static __device__ __noinline__ double exp_any(double x) { return exp(x); }
+
+template <int K>
+__device__ __forceinline__ void exps(const double (&x)[K], double (&y)[K]) {
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < K; ++i) ok = ok && (__double2hiint(x[i]) & 0x7fffffff) < 0x4085e000;  // 700
+  if (ok) {
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const double big = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
+      const double t = fma(x[i], 1.4426950408889634074, big), k = t - big;
+      double r = fma(k, -0.69314718055994530942, x[i]);
+      r = fma(k, -2.3190468138462995584e-17, r);  // ln 2 minus its nearest double
+      const double r2 = r * r, r4 = r2 * r2, r8 = r4 * r4;
+      const double a = fma(1.0 / 6.0, r, 0.5), b = fma(1.0 / 120.0, r, 1.0 / 24.0);
+      const double c = fma(1.0 / 5040.0, r, 1.0 / 720.0), d = fma(1.0 / 362880.0, r, 1.0 / 40320.0);
+      const double e = fma(1.0 / 39916800.0, r, 1.0 / 3628800.0);
+      const double f = fma(1.0 / 6227020800.0, r, 1.0 / 479001600.0);
+      const double lo = fma(b, r2, a), mid = fma(d, r2, c), hi = fma(f, r2, e);
+      const double p = 1.0 + fma(r2, fma(hi, r8, fma(mid, r4, lo)), r);
+      y[i] = __hiloint2double(__double2hiint(p) + (__double2loint(t) << 20), __double2loint(p));
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < K; ++i) y[i] = exp_any(x[i]);
+  }
+}
+
+// y[i] = ln(x[i]), fast for positive normal numbers: x = 2^k m with m in
+// [sqrt(1/2), sqrt 2), ln m = 2 atanh(s) with s = (m - 1) / (m + 1), eleven
+// terms of its series (z = s^2 <= 0.0295, remainder 6e-19).
+static __device__ __noinline__ double log_any(double x) { return log(x); }
+
+template <int K>
+__device__ __forceinline__ void logs(const double (&x)[K], double (&y)[K]) {
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < K; ++i) ok = ok && (unsigned)(__double2hiint(x[i]) - 0x00100000) < 0x7fe00000u;
+  if (ok) {
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const int hi = __double2hiint(x[i]), k = (hi - 0x3fe6a09e) >> 20;  // sqrt(1/2)
+      const double m = __hiloint2double(hi - (k << 20), __double2loint(x[i]));
+      const double f = m - 1.0, d = m + 1.0, w = recip(d);
+      double s = f * w;
+      s = fma(fma(-d, s, f), w, s);
+      const double z = s * s, z2 = z * z, z4 = z2 * z2, z8 = z4 * z4, s2 = s + s;
+      const double p0 = fma(1.0 / 5.0, z, 1.0 / 3.0), p1 = fma(1.0 / 9.0, z, 1.0 / 7.0);
+      const double p2 = fma(1.0 / 13.0, z, 1.0 / 11.0), p3 = fma(1.0 / 17.0, z, 1.0 / 15.0);
+      const double p4 = fma(1.0 / 21.0, z, 1.0 / 19.0);
+      const double p = fma(p4, z8, fma(fma(p3, z2, p2), z4, fma(p1, z2, p0)));
+      const double kd = (double)k;
+      y[i] = fma(kd, 0.69314718055994530942, s2 + fma(s2 * z, p, kd * 2.3190468138462995584e-17));
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < K; ++i) y[i] = log_any(x[i]);
   }
 }
 
@@ -270,10 +317,12 @@ __device__ __forceinline__ void third_body(const Eff *__restrict__ eff, int ne, 
 // One reaction (both steps) for the V states a thread owns (states q .. q +
 // V - 1 of the tile): rate constants, third body, falloff, step limiter
 // (one scalar for all steps, or one per step when lim_step is given) and
-// concentration products.  The V independent chains, and the forward and
-// reverse exponentials of each, give the scheduler instruction-level
-// parallelism: the exponentials and the limiter's quotients are branch-free
-// and run side by side.  gs: the sum of g/RT over products minus reactants.
+// concentration products.  gs: the sum of g/RT over products minus reactants.
+// The V states and the forward and reverse sides run side by side.  The
+// reduced pressure comes from the difference of the two limits' exponents,
+// Pr = exp(a_low - a_high) [M], which needs no division; a falloff reaction's
+// five or six exponentials, its two logarithms and its quotients then form one
+// chain of a few interleaved groups.
 template <int TS, int V>
 __device__ __forceinline__ void reaction_eval(const DevMech &m, const RxnRec &R, int q,
                                               const double *__restrict__ sC,
@@ -282,104 +331,127 @@ __device__ __forceinline__ void reaction_eval(const DevMech &m, const RxnRec &R,
                                               const double *invT,
                                               const double *Csum, double lim,
                                               const double *lim_step = nullptr, const char *tab = nullptr) {
-  double kf[V], kr[V];
-  // exponents first, then the exponentials together
-  double ar[V];
-#pragma unroll
-  for (int k = 0; k < V; ++k) ar[k] = 0.0;
-  if (R.flags & kRevArr) {
-#pragma unroll
-    for (int k = 0; k < V; ++k) ar[k] = R.lnA_r + R.n_r * logT[k] - R.Ta_r * invT[k];
-  } else if (R.flags & kRevKeq) {
-#pragma unroll
-    for (int k = 0; k < V; ++k) ar[k] = gs[k] - R.lnA_r * (kLnPatmRu - logT[k]);
+  const bool falloff = (R.flags & kFalloff) != 0;
+  double Cm[V];
+  if (R.flags & (kThirdBody | kFalloff)) {
+    const int fs = falloff ? rb(m.fo_spc, tab, m.base)[R.aux] : -1;
+    if (fs >= 0) ldv<V>(sC + fs * TS + q, Cm);
+    else third_body<TS, V>(rb(m.eff, tab, m.base) + R.e0, R.ne, q, sC, Csum, Cm);
   }
+  // exponents first, then the exponentials together: forward, reverse
+  double x[2 * V], kk[2 * V];
 #pragma unroll
   for (int k = 0; k < V; ++k) {
-    kf[k] = exp_tree(R.lnA + R.n * logT[k] - R.Ta * invT[k]);
-    kr[k] = exp_tree(ar[k]);
+    x[k] = R.lnA + R.n * logT[k] - R.Ta * invT[k];
+    x[V + k] = 0.0;
   }
+  if (R.flags & kRevArr) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) x[V + k] = R.lnA_r + R.n_r * logT[k] - R.Ta_r * invT[k];
+  } else if (R.flags & kRevKeq) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) x[V + k] = gs[k] - R.lnA_r * (kLnPatmRu - logT[k]);
+  }
+  exps<2 * V>(x, kk);
+  double kf[V], kr[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) kf[k] = kk[k];
   if (R.flags & kPlog) {  // at the pressure of the concentrations, Csum Ru T (rate_const.cpp:548-567)
 #pragma unroll
     for (int k = 0; k < V; ++k) kf[k] = plog_rate(m, R.aux, T[k], invT[k], logT[k], Csum[k] * kRuD * T[k], tab);
   }
-  if (!(R.flags & kRevArr)) {
+  if (R.flags & kRevArr) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) kr[k] = kk[V + k];
+  } else {
     const bool keq = (R.flags & kRevKeq) != 0;
 #pragma unroll
-    for (int k = 0; k < V; ++k) kr[k] = keq ? kr[k] * kf[k] : 0.0;
+    for (int k = 0; k < V; ++k) kr[k] = keq ? kk[V + k] * kf[k] : 0.0;
   }
   if (R.flags & kThirdBody) {
-    double Cm[V];
-    third_body<TS, V>(rb(m.eff, tab, m.base) + R.e0, R.ne, q, sC, Csum, Cm);
 #pragma unroll
     for (int k = 0; k < V; ++k) {
       kf[k] *= Cm[k];
       kr[k] *= Cm[k];
     }
   }
-  if (R.flags & kFalloff) {
-    const int f = R.aux;
-    const double *p = rb(m.fo_par, tab, m.base) + 8 * f;
-    const int fs = rb(m.fo_spc, tab, m.base)[f];
-    const int ty = rb(m.fo_type, tab, m.base)[f];
-    const double p3 = p[3], p4 = p[4], p5 = p[5], p6 = p[6];
-    double Klow[V], Cm[V];
+  if (falloff) {
+    const double *p = rb(m.fo_par, tab, m.base) + 8 * R.aux;
+    const int ty = rb(m.fo_type, tab, m.base)[R.aux];
+    double Pr[V], fT[V], t[V];
 #pragma unroll
-    for (int k = 0; k < V; ++k) Klow[k] = exp_tree(p[0] + p[1] * logT[k] - p[2] * invT[k]);
-    if (fs >= 0) {
-      ldv<V>(sC + fs * TS + q, Cm);
-    } else {
-      third_body<TS, V>(rb(m.eff, tab, m.base) + R.e0, R.ne, q, sC, Csum, Cm);
-    }
-    double Pr[V], fT[V];
+    for (int k = 0; k < V; ++k) t[k] = (p[0] + p[1] * logT[k] - p[2] * invT[k]) - x[k];
+    exps<V>(t, Pr);
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      Klow[k] *= Cm[k];
+      Pr[k] *= Cm[k];
+      if (Pr[k] < 1.0e-300) Pr[k] = 1.0e-300;
       fT[k] = 1.0;
     }
-    quotients<V>(Klow, kf, Pr);
-#pragma unroll
-    for (int k = 0; k < V; ++k)
-      if (Pr[k] < 1.0e-300) Pr[k] = 1.0e-300;
     if (ty == kTroe3 || ty == kTroe4) {
-      double e1[V], e2[V], e3[V];
+      const double p3 = p[3], p4 = p[4], p5 = p[5], p6 = p[6];  // p4, p5: -1 / T***, -1 / T*, or 0
+      double u[3 * V], e[3 * V];
 #pragma unroll
       for (int k = 0; k < V; ++k) {
-        e1[k] = exp_tree(p4 != 0.0 ? -T[k] / p4 : 0.0);
-        e2[k] = exp_tree(p5 != 0.0 ? -T[k] / p5 : 0.0);
-        e3[k] = exp_tree(-p6 * invT[k]);
+        u[k] = T[k] * p4;
+        u[V + k] = T[k] * p5;
+        u[2 * V + k] = ty == kTroe4 ? -p6 * invT[k] : 0.0;
       }
+      exps<3 * V>(u, e);
+      double w[2 * V], l[2 * V];
 #pragma unroll
       for (int k = 0; k < V; ++k) {
         double Fc = 0.0;
-        if (p4 != 0.0) Fc += (1.0 - p3) * e1[k];
-        if (p5 != 0.0) Fc += p3 * e2[k];
-        if (ty == kTroe4) Fc += e3[k];
+        if (p4 != 0.0) Fc += (1.0 - p3) * e[k];
+        if (p5 != 0.0) Fc += p3 * e[V + k];
+        if (ty == kTroe4) Fc += e[2 * V + k];
         if (Fc < 1.0e-300) Fc = 1.0e-300;
-        const double lF = log10(Fc);
-        const double nT = 0.75 - 1.27 * lF;
-        double x = log10(Pr[k]) - (0.4 + 0.67 * lF);
-        x = x / (nT - 0.14 * x);
-        x *= x;
-        fT[k] = exp_tree(lF / (1.0 + x) * 2.30258509299404568402);  // 10^
+        w[k] = Fc;
+        w[V + k] = Pr[k];
       }
+      logs<2 * V>(w, l);
+      const double ln10 = 2.30258509299404568402, ilog = 0.43429448190325182765;  // log10 = ln / ln 10
+      double a[V], d[V], r[V];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const double lF = l[k] * ilog;
+        a[k] = l[V + k] * ilog - (0.4 + 0.67 * lF);
+        d[k] = (0.75 - 1.27 * lF) - 0.14 * a[k];
+      }
+      quotients<V>(a, d, r);
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        a[k] = l[k] * ilog;
+        d[k] = 1.0 + r[k] * r[k];
+      }
+      quotients<V>(a, d, r);
+#pragma unroll
+      for (int k = 0; k < V; ++k) r[k] *= ln10;
+      exps<V>(r, fT);
     } else if (ty == kSRI) {
+      const double p3 = p[3], p4 = p[4], p5 = p[5], p6 = p[6];
 #pragma unroll
       for (int k = 0; k < V; ++k) {
         const double lPr = log10(Pr[k]);
         const double xp = 1.0 / (1.0 + lPr * lPr);
-        double t = p3 * exp_tree(-p4 * invT[k]);
-        if (p5 > 0) t += exp_tree(-T[k] * p5);
-        t = pow(t, xp);
-        t *= p6;
-        fT[k] = t * pow(T[k], p[7]);
+        double s = p3 * exp(-p4 * invT[k]);
+        if (p5 > 0) s += exp(-T[k] * p5);
+        s = pow(s, xp);
+        s *= p6;
+        fT[k] = s * pow(T[k], p[7]);
       }
     }
+    double d[V];
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      const double Pc = fT[k] * Pr[k] / (1.0 + Pr[k]);
-      kf[k] *= Pc;
-      kr[k] *= Pc;
+      t[k] = fT[k] * Pr[k];
+      d[k] = 1.0 + Pr[k];
+    }
+    quotients<V>(t, d, fT);
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      kf[k] *= fT[k];
+      kr[k] *= fT[k];
     }
   }
   if (lim_step) {  // one limit per step (perf_net.cpp:213-224)
