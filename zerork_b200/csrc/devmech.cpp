@@ -248,6 +248,19 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   std::vector<double> thermo_t(16 * (size_t)ns);
   for (int j = 0; j < ns; ++j)
     for (int c = 0; c < 16; ++c) thermo_t[(size_t)c * ns + j] = t.thermo[16 * (size_t)j + c];
+  std::vector<int4> sq_rec;
+  std::vector<int2> sq_step;
+  for (int j : spc_order) {
+    std::vector<int> all(sd[j]);
+    all.insert(all.end(), sc[j].begin(), sc[j].end());
+    sq_rec.push_back(make_int4(j, (int)all.size(), (int)sq_step.size(), (int)sd[j].size()));
+    for (size_t i = 0; i < all.size(); i += 4) {
+      unsigned u[4];
+      for (int e = 0; e < 4; ++e) u[e] = (unsigned)all[std::min(i + e, all.size() - 1)];
+      sq_step.push_back(make_int2((int)(u[0] | u[1] << 16), (int)(u[2] | u[3] << 16)));
+    }
+  }
+  sq_step.push_back(make_int2(0, 0));  // the record fetched past the end
   std::vector<int4> sn_rec;
   for (int j : spc_order) sn_rec.push_back(make_int4(j, sn_ptr[j], sn_ptr[j + 1], 0));
   // Troe's -1 / T*** and -1 / T* in their places (0 where the term is absent)
@@ -261,6 +274,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   size_t o_rbc = b.add(rec_by_cost, h);
   size_t o_mw = b.add(t.mw, h), o_imw = b.add(inv_mw, h), o_rimw = b.add(ru_inv_mw, h),
          o_th = b.add(t.thermo, h);
+  const size_t spc_end = (b.bytes.size() + 15) & ~size_t(15);
   size_t o_eff = b.add(eff, h), o_fot = b.add(t.fo_type, h), o_fos = b.add(t.fo_spc, h),
          o_fopar = b.add(fo_par, h);
   size_t o_plpp = b.add(t.plog_pt_ptr, h), o_pllp = b.add(t.plog_ln_ptr, h), o_plp = b.add(t.plog_p, h),
@@ -268,7 +282,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
          o_pln = b.add(t.plog_n, h), o_plt = b.add(t.plog_Ta, h);
   size_t o_sdp = b.add(sd_ptr, h), o_sds = b.add(sd_step, h), o_scp = b.add(sc_ptr, h),
          o_scs = b.add(sc_step, h);
-  size_t o_so = b.add(spc_order, h);
+  size_t o_so = b.add(spc_order, h), o_sqr = b.add(sq_rec, h), o_sqs = b.add(sq_step, h);
   size_t o_cp = b.add(p.col_ptr, h), o_ri = b.add(p.row_idx, h);
   size_t o_jit = b.add(jit, h), o_jext = b.add(jext, h), o_jc = b.add(jcost, h), o_jf = b.add(jf_ptr, h);
   const size_t hot = (b.bytes.size() + 15) & ~size_t(15);
@@ -287,6 +301,9 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   auto P = [&](size_t off) { return (const void *)((const unsigned char *)blob_ + off); };
   view_.base = (const unsigned char *)blob_;
   view_.hot_bytes = (int)hot;
+  view_.spc_bytes = (int)(spc_end - o_mw);
+  view_.sq_rec = (const int4 *)P(o_sqr);
+  view_.sq_step = (const int2 *)P(o_sqs);
   view_.nsp = ns;
   view_.nrxn = t.nrxn;
   view_.nstep = t.nstep;

@@ -66,6 +66,11 @@ struct DevMech {
   // {species, first, end, 0} by decreasing length
   const int4 *sn_rec;
   const int *sn_step;
+  // both lists of a species for the rates kernel, longest first: {species,
+  // number of terms, first record, number of destruction terms} and records of
+  // four 16-bit steps, destruction first (unused places repeat the last step)
+  const int4 *sq_rec;
+  const int2 *sq_step;
   // Jacobian pattern and per-nonzero gather lists
   const int *col_ptr, *row_idx, *last_row;
   const int *nzd_ptr, *nzd_step, *nzc_ptr, *nzc_step;
@@ -111,6 +116,8 @@ struct DevMech {
   // memory and address them at a fixed offset from their global copies.
   const unsigned char *base;
   int hot_bytes;
+  // molecular weights, their reciprocals and the thermodynamic fits: bytes from mw on
+  int spc_bytes;
 };
 
 // Host-side builder; owns the device allocation.

@@ -58,8 +58,11 @@ cudaError_t launch_rates_tc(const DevMech &m, const RatesTCArgs &a, cudaStream_t
 int rates_jac_part_rows(const DevMech &m, const LaunchCfg &cfg);
 // The whole workspace of a tile.
 size_t rates_jac_ws_bytes(const DevMech &m, const LaunchCfg &cfg);
+// Whether the species tables (molecular weights, fits) fit in shared memory
+// beside the workspace; they are then read from there.
+bool rates_jac_species_fit(const DevMech &m, const LaunchCfg &cfg);
 // Dynamic shared memory of a launch: the workspace (unless global) plus the
-// staged tables (cfg.stage).
+// staged tables (cfg.stage) or the species tables.
 size_t rates_jac_smem_bytes(const DevMech &m, const LaunchCfg &cfg);
 bool rates_jac_mapping_ok(const LaunchCfg &cfg);
 cudaError_t launch_rates_jac(const DevMech &m, const RatesJacArgs &a, const KinParams &kp,

@@ -137,8 +137,8 @@ __device__ __forceinline__ bool rop_change(const RxnRec &R, int q, const double 
 // The sum of g/RT over a reaction's products minus its reactants from the
 // species' fits at T (where the g/RT rows hold something else).
 template <int V>
-__device__ __forceinline__ void gibbs_from_fits(const DevMech &m, const RxnRec &R, const double *T, const double *logT,
-                                                double (&gs)[V], const char *tab) {
+__device__ __forceinline__ void gibbs_from_fits(const double *thermo, const RxnRec &R, const double *T,
+                                                const double *logT, double (&gs)[V]) {
 #pragma unroll
   for (int k = 0; k < V; ++k) gs[k] = 0.0;
 #pragma unroll 1
@@ -150,7 +150,7 @@ __device__ __forceinline__ void gibbs_from_fits(const DevMech &m, const RxnRec &
       if (prod && e == i) sp = R.p[e];
       if (!prod && e == i - R.np) sp = R.r[e];
     }
-    const double *th = rb(m.thermo, tab, m.base) + 16 * sp;
+    const double *th = thermo + 16 * sp;
 #pragma unroll
     for (int k = 0; k < V; ++k) {
       double cp, h, g;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
     DevMech m, int n, int ld, const double *__restrict__ Tin, const double *__restrict__ Pin,
     const double *__restrict__ Y, double *__restrict__ wdot, double *__restrict__ jac,
     double *__restrict__ ydot, KinParams kp, double *__restrict__ gscratch, int slice_doubles,
-    int stage_bytes, int part_rows, int vec) {
+    int stage_bytes, int spc_bytes, int part_rows, int vec) {
   constexpr int GS = TS / V;
   extern __shared__ __align__(16) double smem_dyn[];
   const int S = m.nsp, N = m.nstep;
@@ -188,21 +188,27 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
     __syncthreads();
     tab = reinterpret_cast<const char *>(dst);
   }
+  // the species tables after the workspace, when they fit: every phase reads
+  // them once or more per item, and what L1 the workspace leaves is the lists'
+  const char *stab = nullptr;
+  if (!STAGE && spc_bytes) {
+    int4 *dst = reinterpret_cast<int4 *>(smem_dyn + (GLOBAL ? 0 : (size_t)L.rows * TS));
+    const int4 *src = reinterpret_cast<const int4 *>(m.mw);
+    for (int i = threadIdx.x; i < spc_bytes / 16; i += blockDim.x) dst[i] = src[i];
+    __syncthreads();
+    stab = reinterpret_cast<const char *>(dst);
+  }
 #define TB(f) rb(m.f, tab, m.base)
+#define SB(f) (STAGE ? TB(f) : rb(m.f, stab, (const unsigned char *)m.mw))
   double *sC = ws + L.rC * TS, *sU = ws + L.rU * TS, *sG = ws + L.rG * TS;
   double *sPart = ws + L.rPart * TS, *sStash = ws + L.rStash * TS;
   double *sROP = ws + L.rROP * TS;
 #define PT(a, ww, k) sPart[((a) * NW + (ww)) * TS + q + (k)]
 #define FORV _Pragma("unroll") for (int k = 0; k < V; ++k)
-// Items of a cost-sorted work list in snake order: round r gives group g the
-// item at r*NG + g (r even) or r*NG + NG-1-g (r odd), so the costliest items
-// spread over the groups and every group's total is close to the mean.
-#define SNAKE(var, list, count)                                      \
-  for (int snake_r = 0, var = 0; snake_r * NG < (count); ++snake_r)  \
-    if (const int snake_p = snake_r * NG + ((snake_r & 1) ? NG - 1 - g : g); \
-        snake_p < (count) && ((var = (list)[snake_p]), true))
-  // All reactions in snake order, the next record on its way to L1 during
-  // this one: body(record)
+  // All reactions in snake order (round r gives group g the record at r*NG + g,
+  // or at r*NG + NG-1-g for odd r, so that the costliest spread over the groups
+  // and every group's total is close to the mean), the next record on its way
+  // to L1 during this one: body(record)
   auto each_reaction = [&](auto body) {
     const RxnRec *recs = TB(rxn_by_cost);
 #pragma unroll 1
@@ -248,13 +254,17 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
     if (const long nt = (long)(tile + gridDim.x) * TS; nt < n) {
       for (int i = threadIdx.x; i < S; i += blockDim.x)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(Y + (size_t)i * ld + nt));
+      if (threadIdx.x == 0) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(Tin + nt));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(Pin + nt));
+      }
     }
     // ---- mixture molecular weight partials
     {
       double pa[V];
       FORV pa[k] = 0.0;
       for (int s = g; s < S; s += NG) {
-        const double iw = TB(inv_mw)[s];
+        const double iw = SB(inv_mw)[s];
         double y[V];
         yload(s, y);
         FORV pa[k] += y[k] * iw;
@@ -309,8 +319,8 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
         double pc[V], pcv[V];
         FORV pc[k] = pcv[k] = 0.0;
         for (int s = g; s < S; s += NG) {
-          const double *th = TB(thermo) + 16 * s;
-          const double iw = TB(inv_mw)[s], riw = TB(ru_inv_mw)[s];
+          const double *th = SB(thermo) + 16 * s;
+          const double iw = SB(inv_mw)[s], riw = SB(ru_inv_mw)[s];
           double y[V], c[V], gg[V], u[V];
           yload(s, y);
           FORV {
@@ -374,7 +384,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
           if (R.rev >= 0) ldv<V>(sROP + R.rev * TS + q, r0);
         }
         double gs[V];
-        if (pass == 1 && (R.flags & kRevKeq)) gibbs_from_fits<V>(m, R, Tq, lq, gs, tab);
+        if (pass == 1 && (R.flags & kRevKeq)) gibbs_from_fits<V>(SB(thermo), R, Tq, lq, gs);
         else gibbs_from_rows<TS, V>(R, q, sG, gs);
         reaction_eval<TS, V>(m, R, q, sC, gs, sROP, Tq, lq, iq, Csum, kp.lim, nullptr, tab);
         if (pass == 1) {
@@ -394,15 +404,35 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
       {
         double pe[V];
         FORV pe[k] = 0.0;
-        SNAKE(s, TB(spc_order), S) {
-          double des[V], net[V], u[V], out[V];
-          FORV des[k] = net[k] = 0.0;
-          gather_rop<TS, V>(sROP, TB(sd_step), TB(sd_ptr)[s], TB(sd_ptr)[s + 1], q, des);
-          gather_rop<TS, V>(sROP, TB(sc_step), TB(sc_ptr)[s], TB(sc_ptr)[s + 1], q, net);
-          const double mws = TB(mw)[s];
-          FORV net[k] -= des[k];
+        // every species' terms four a record, the next record in flight during
+        // this one; the longest lists first, in snake order
+        for (int r = 0; r * NG < S; ++r) {
+          const int sp = r * NG + ((r & 1) ? NG - 1 - g : g);
+          if (sp >= S) continue;
+          const int4 rec = TB(sq_rec)[sp];
+          const int s = rec.x, nd = rec.w;
+          const int2 *steps = TB(sq_step) + rec.z;
+          double net[V], u[V], out[V];
+          FORV net[k] = 0.0;
+          int2 nx = steps[0];
+          for (int pos = 0; pos < rec.y; pos += 4) {
+            const int2 it = nx;
+            nx = *++steps;
+            double x[4][V];
+            ldv<V>(sROP + (it.x & 0xffff) * TS + q, x[0]);
+            ldv<V>(sROP + (int)((unsigned)it.x >> 16) * TS + q, x[1]);
+            ldv<V>(sROP + (it.y & 0xffff) * TS + q, x[2]);
+            ldv<V>(sROP + (int)((unsigned)it.y >> 16) * TS + q, x[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (pos + e < rec.y) {
+                const double sg = pos + e < nd ? -1.0 : 1.0;
+                FORV net[k] = fma(sg, x[e][k], net[k]);
+              }
+          }
+          const double mws = SB(mw)[s];
           if (pass == 1) {
-            const double *th = TB(thermo) + 16 * s, *wd = wdot + (size_t)s * ld + st0;
+            const double *th = SB(thermo) + 16 * s, *wd = wdot + (size_t)s * ld + st0;
             FORV {
               const double mult = 1.0 / ((yS[k] + yS[k] * kp.sqrt_ur) - yS[k]);
               out[k] = net[k] * mws * v[k] * mult;
@@ -483,8 +513,8 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
             }
             double t2[V], trow[V], wcol = 0.0;
             auto column = [&]() {
-              wcol = TB(inv_mw)[j];
-              const double mj = TB(mw)[j];
+              wcol = SB(inv_mw)[j];
+              const double mj = SB(mw)[j];
               double y[V];
               yload(j, y);
               FORV {
@@ -508,7 +538,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
                   column();
                 }
                 const int row = it.x & 0xffff, nd = (int)((unsigned)it.x >> 16);
-                const double conv = TB(mw)[row] * wcol;
+                const double conv = SB(mw)[row] * wcol;
                 double r[4][V], u[V], val[V];
                 ldv<V>(sROP + (it.y & 0xffff) * TS + q, r[0]);
                 ldv<V>(sROP + (int)((unsigned)it.y >> 16) * TS + q, r[1]);
@@ -560,14 +590,14 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
             ldv<V>(sTP + (j + gg) * TS + q, t);
             FORV tp[k] += t[k];
           }
-          const double *th = TB(thermo) + 16 * j;
+          const double *th = SB(thermo) + 16 * j;
           ldv<V>(sStash + q, sd);
           ldv<V>(sStash + TS + q, sc);
           FORV {
-            const double cvj = (nasa_cp(th, Tr[k]) - 1.0) * TB(ru_inv_mw)[j];
+            const double cvj = (nasa_cp(th, Tr[k]) - 1.0) * SB(ru_inv_mw)[j];
             double tr = tp[k] * (kRu * yS[k]);
-            tr += sd[k] * cvj * TB(mw)[j];
-            tr *= TB(inv_mw)[j] * (-1.0 / sc[k]);
+            tr += sd[k] * cvj * SB(mw)[j];
+            tr *= SB(inv_mw)[j] * (-1.0 / sc[k]);
             t[k] = tr;
           }
           put(jac + (size_t)(TB(jf_ptr)[j + 1] + j) * ld, t);
@@ -578,8 +608,8 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
   }
 #undef PT
 #undef TB
+#undef SB
 #undef FORV
-#undef SNAKE
 }
 
 template <int TS, int V, bool GLOBAL, int MAXT, bool STAGE, int MINB>
@@ -617,7 +647,8 @@ cudaError_t launch_one(const DevMech &m, const RatesJacArgs &a, const KinParams 
   const auto al16 = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
   const int vec = V > 1 && a.ld % 2 == 0 && al16(a.Y) && al16(a.wdot) && al16(a.jac) && al16(a.ydot);
   kern<<<grid, threads, smem, stream>>>(m, a.n, a.ld, a.T, a.P, a.Y, a.wdot, a.jac, a.ydot, kp, a.scratch,
-                                        (int)(slice / sizeof(double)), stage_bytes, rates_jac_part_rows(m, cfg), vec);
+                                        (int)(slice / sizeof(double)), stage_bytes,
+                                        rates_jac_species_fit(m, cfg) ? m.spc_bytes : 0, rates_jac_part_rows(m, cfg), vec);
   return cudaGetLastError();
 }
 
