@@ -110,6 +110,7 @@ LaunchCfg MechHandle::launch_for(int n, bool jac) const {
 MechHandle::~MechHandle() {
   if (scratch) cudaFree(scratch);
   if (pipe) cudaFree(pipe);
+  if (pinned) cudaFreeHost(pinned);
   for (auto &s : pipe_stream)
     if (s) cudaStreamDestroy(s);
   for (void *p : host_bufs) cudaFree(p);
@@ -126,6 +127,11 @@ cudaError_t MechHandle::ensure_pipe(size_t bytes) {
   e = cudaMalloc(&pipe, bytes);
   if (e == cudaSuccess) pipe_bytes = bytes;
   return e;
+}
+
+cudaError_t MechHandle::ensure_pinned() {
+  if (pinned) return cudaSuccess;
+  return cudaHostAlloc(&pinned, kPinnedBytes, cudaHostAllocMapped);
 }
 
 cudaError_t MechHandle::ensure_scratch(size_t bytes) {
@@ -444,6 +450,38 @@ int zrk_rates_tc_host(zrk_mech_t m, int n, const double *T, const double *C,
   double *dT = (double *)h->pipe, *dC = dT + n, *dL = dC + S * n, *dN = dL + N, *dCr = dN + S * n,
          *dDe = dCr + S * n, *dR = dDe + S * n;
   cudaStream_t st = h->pipe_stream[0];
+  if (doubles * dp <= MechHandle::kPinnedBytes) {
+    // A few states: seven copies of a few KB, most of them waited for by the
+    // driver because user memory is pageable, cost several times the kernel
+    // (one 53-species state 104 us).  The inputs go over in one copy from
+    // pinned staging and the kernel writes its results there.
+    if ((e = h->ensure_pinned()) != cudaSuccess) return cuda_error(e, "pinned staging");
+    double *host = (double *)h->pinned, *hdev = nullptr;
+    if ((e = cudaHostGetDevicePointer((void **)&hdev, host, 0)) != cudaSuccess) return cuda_error(e, "pinned staging");
+    std::memcpy(host, T, n * dp);
+    std::memcpy(host + n, C, S * n * dp);
+    if (step_limiter) std::memcpy(host + n + S * n, step_limiter, N * dp);
+    const size_t in = n + S * n + (step_limiter ? N : 0), on = n + S * n + N;  // outputs start at `on`
+    if ((e = cudaMemcpyAsync(dT, host, in * dp, cudaMemcpyHostToDevice, st)) != cudaSuccess)
+      return cuda_error(e, "copy in");
+    RatesTCArgs a;
+    a.n = n;
+    a.ld = n;
+    a.T = dT;
+    a.C = dC;
+    a.lim_step = step_limiter ? dL : nullptr;
+    a.net = net ? hdev + on : nullptr;
+    a.create = create ? hdev + on + S * n : nullptr;
+    a.destroy = destroy ? hdev + on + 2 * S * n : nullptr;
+    a.rop = rop ? hdev + on + 3 * S * n : nullptr;
+    if ((e = launch_rates_tc(h->dev->view(), a, st)) != cudaSuccess) return cuda_error(e, "rates_tc launch");
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_error(e, "rates_tc");
+    if (net) std::memcpy(net, host + on, S * n * dp);
+    if (create) std::memcpy(create, host + on + S * n, S * n * dp);
+    if (destroy) std::memcpy(destroy, host + on + 2 * S * n, S * n * dp);
+    if (rop) std::memcpy(rop, host + on + 3 * S * n, N * n * dp);
+    return ZRK_OK;
+  }
   if ((e = cudaMemcpyAsync(dT, T, n * dp, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
       (e = cudaMemcpyAsync(dC, C, S * n * dp, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
       (step_limiter &&

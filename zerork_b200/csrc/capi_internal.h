@@ -24,11 +24,14 @@ struct MechHandle {
   std::vector<void *> host_bufs;
   void *pipe = nullptr;  // host-entry pipeline slots (device)
   size_t pipe_bytes = 0;
+  void *pinned = nullptr;  // staging of small host calls, kPinnedBytes, mapped for the device
+  static constexpr size_t kPinnedBytes = 256 << 10;
   cudaStream_t pipe_stream[2] = {nullptr, nullptr};
   ~MechHandle();
   LaunchCfg launch_for(int n, bool jac) const;
   cudaError_t ensure_scratch(size_t bytes);
   cudaError_t ensure_pipe(size_t bytes);
+  cudaError_t ensure_pinned();
 };
 
 int set_error(int code, const std::string &msg);

@@ -161,6 +161,12 @@ cudaError_t launch_rates_tc(const DevMech &m, const RatesTCArgs &a, cudaStream_t
   // states per tile where two workspaces fit in shared memory; else one CTA
   // per SM with the largest tile that fits
   const size_t kMax = 227 * 1024, kSm = 228 * 1024;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // up to one state per SM: a CTA a state and a reaction a thread (two rounds
+  // of 325 reactions instead of eleven in a 16-state tile of mostly idle lanes)
+  if (a.n <= sms && rates_tc_smem_bytes(m, 1, 256) <= kMax) return launch_tv<1, 1, 2>(m, a, 256, stream);
   if (2 * (rates_tc_smem_bytes(m, 16, 256) + 1024) <= kSm) return launch_tv<16, 2, 2>(m, a, 256, stream);
   if (rates_tc_smem_bytes(m, 32, 256) <= kMax) return launch_tv<32, 2, 1>(m, a, 256, stream);
   if (rates_tc_smem_bytes(m, 16, 256) <= kMax) return launch_tv<16, 1, 1>(m, a, 256, stream);
