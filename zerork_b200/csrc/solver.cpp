@@ -282,6 +282,23 @@ cudaError_t ReactorSolver::solve_with_callback(int method, const IntegOpts &io, 
   return cudaSuccess;
 }
 
+// Threads of the dense integrator.  A call lasts as long as its slowest
+// reactor, so a reactor gets a warp for each of its blocks of 32 reactions
+// (devmech.h rxn_slots), 12 when that would be 13 to 16 (barriers then cost what
+// the warps give: 13 blocks, 1000 cells: 72.9 ms with 384 threads, 75.1 with
+// 416, 94.9 with 256) and 16 beyond (900 reactions: 399 ms with 512, 447 with
+// 384).  27 reactions, 64 reactors: 41.1 ms with 96 threads, 45.2 with 64, 52.5
+// with 32; with more small reactors than the SMs hold side by side their
+// number counts instead (1000 reactors: 127 ms with 96, 101 with 32), and the
+// unknowns decide.
+static int dense_threads(const DevMech &m, int n, int sms) {
+  const int work = std::max(m.nsp + 1, m.nrxn / 2);
+  int threads = 32;
+  while (threads < work && threads < 512) threads *= 2;
+  const int warps = m.nblocks > 16 ? 16 : std::min(m.nblocks, 12);
+  return n <= 4 * sms || m.nblocks > 8 ? std::max(threads, 32 * warps) : threads;
+}
+
 int ReactorSolver::solve(const SolveOptions &o, int n, double dt, double *T, double *P, double *mf,
                          int stride, double *cost, double *gpu_time, double *temp_delta,
                          double temp_threshold, std::vector<ReactorStats> *stats,
@@ -356,11 +373,7 @@ int ReactorSolver::solve(const SolveOptions &o, int n, double dt, double *T, dou
   int dthreads = o.threads;
   int dctas = ctas;
   if (method == 1) {
-    if (dthreads <= 0) {
-      const int work = std::max(m.nsp + 1, m.nrxn / 2);
-      dthreads = 32;
-      while (dthreads < work && dthreads < 512) dthreads *= 2;
-    }
+    if (dthreads <= 0) dthreads = dense_threads(m, n, ctas);
     const size_t sm = dense_smem_bytes(m, o.lu_fp32, nullptr, spill);
     int per_sm = (int)std::min<size_t>(kSmemMax / sm, (size_t)(2048 / dthreads));
     per_sm = std::max(1, std::min(per_sm, 65536 / (dthreads * 128)));
