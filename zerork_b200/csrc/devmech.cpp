@@ -119,11 +119,39 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     sc_step.insert(sc_step.end(), sc[j].begin(), sc[j].end());
     sc_ptr.push_back((int)sc_step.size());
   }
-  std::vector<int> sn_ptr(1, 0), sn_step;
+  // one flat list of all species' terms in equal chunks (devmech.h net_ent)
+  std::vector<unsigned> flat;
+  std::vector<int> owner;
   for (int j = 0; j < ns; ++j) {
-    for (int st : sd[j]) sn_step.push_back((int)(st | 0x80000000u));
-    sn_step.insert(sn_step.end(), sc[j].begin(), sc[j].end());
-    sn_ptr.push_back((int)sn_step.size());
+    for (int st : sd[j]) flat.push_back((unsigned)st | 0x80000000u);
+    for (int st : sc[j]) flat.push_back((unsigned)st);
+    owner.resize(flat.size(), j);
+  }
+  int net_quads = 2;
+  auto chunks_of = [&](int quads) { return ((int)flat.size() + 4 * quads - 1) / (4 * quads); };
+  while (chunks_of(net_quads) > std::min(416, 3 * ns + 2)) ++net_quads;
+  const int net_chunks = chunks_of(net_quads), net_len = 4 * net_quads;
+  std::vector<int> net_slot, net_ptr(ns + 1, 0);
+  std::vector<int4> net_ent((size_t)(net_chunks + 31) / 32 * net_quads * 32, make_int4(0, 0, 0, 0));
+  {
+    int slot = 0, done = 0;  // species up to `done` have their first slot noted
+    for (int c = 0; c < net_chunks; ++c) {
+      net_slot.push_back(slot);
+      for (int e = 0; e < net_len; ++e) {
+        const size_t i = (size_t)c * net_len + e;
+        unsigned w = 0;
+        if (i < flat.size()) {
+          while (done <= owner[i]) net_ptr[done++] = slot;
+          w = flat[i];
+          if (e + 1 == net_len || i + 1 == flat.size() || owner[i + 1] != owner[i]) {
+            w |= 0x40000000u;
+            ++slot;
+          }
+        }
+        (&net_ent[((size_t)c / 32 * net_quads + e / 4) * 32 + c % 32].x)[e % 4] = (int)w;
+      }
+    }
+    while (done <= ns) net_ptr[done++] = slot;
   }
   // Jacobian per-nonzero gather lists, in term-list order
   // (reactor_nvector_serial.cpp:659-673: all destruction terms, then creation)
@@ -241,6 +269,14 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
       slots.push_back(none);
     }
   }
+  std::vector<int4> sn_rec;
+  std::vector<int> sn_step;
+  for (int j : spc_order) {
+    const int first = (int)sn_step.size();
+    for (int st : sd[j]) sn_step.push_back((int)(st | 0x80000000u));
+    sn_step.insert(sn_step.end(), sc[j].begin(), sc[j].end());
+    sn_rec.push_back(make_int4(j, first, (int)sn_step.size(), 0));
+  }
   std::vector<int4> slot_parts(slots.size() * 6);
   for (size_t i = 0; i < slots.size(); ++i)
     for (int c = 0; c < 6; ++c)
@@ -261,8 +297,6 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     }
   }
   sq_step.push_back(make_int2(0, 0));  // the record fetched past the end
-  std::vector<int4> sn_rec;
-  for (int j : spc_order) sn_rec.push_back(make_int4(j, sn_ptr[j], sn_ptr[j + 1], 0));
   // Troe's -1 / T*** and -1 / T* in their places (0 where the term is absent)
   std::vector<double> fo_par(t.fo_par);
   for (size_t k = 0; k < t.fo_type.size(); ++k)
@@ -289,7 +323,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   size_t o_rec = b.add(rec), o_slot = b.add(slot_parts), o_tht = b.add(thermo_t);
   size_t o_jw = b.add(jw), o_jt = b.add(jt), o_jtp = b.add(jt_ptr);
   size_t o_jfc = b.add(jf_col);
-  size_t o_snr = b.add(sn_rec), o_sns = b.add(sn_step);
+  size_t o_snr = b.add(sn_rec), o_sns = b.add(sn_step), o_ne = b.add(net_ent), o_ns = b.add(net_slot), o_np = b.add(net_ptr);
   size_t o_lr = b.add(p.last_row);
   size_t o_ndp = b.add(nzd_ptr), o_nds = b.add(nzd_step), o_ncp = b.add(nzc_ptr), o_ncs = b.add(nzc_step);
   size_t o_jrp = b.add(jr_ptr), o_jrk = b.add(jr_kk), o_jrc = b.add(jr_col);
@@ -331,6 +365,11 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.sc_step = (const int *)P(o_scs);
   view_.sn_rec = (const int4 *)P(o_snr);
   view_.sn_step = (const int *)P(o_sns);
+  view_.net_chunks = slots.size() / 32 > kFewBlocks ? net_chunks : 0;
+  view_.net_quads = net_quads;
+  view_.net_ent = (const int4 *)P(o_ne);
+  view_.net_slot = (const int *)P(o_ns);
+  view_.net_ptr = (const int *)P(o_np);
   view_.col_ptr = (const int *)P(o_cp);
   view_.row_idx = (const int *)P(o_ri);
   view_.last_row = (const int *)P(o_lr);

@@ -62,10 +62,20 @@ struct DevMech {
   const double *plog_p, *plog_lnp, *plog_lnA, *plog_sgn, *plog_n, *plog_Ta;
   // species production gather lists (step indices in ascending step order)
   const int *sd_ptr, *sd_step, *sc_ptr, *sc_step;
-  // both lists of a species in one, step | 1 << 31 for a destruction term, and
-  // {species, first, end, 0} by decreasing length
+  // Both lists of all species as one list for one reactor per CTA, cut into
+  // net_chunks equal chunks of net_quads * 4 entries whatever species they
+  // belong to: step | 1 << 31 for a destruction term | 1 << 30 where a partial
+  // sum ends (a species' or the chunk's last term).  Chunk c's partial sums go
+  // to the slots from net_slot[c] on, and species k's net rate is the sum of
+  // the slots [net_ptr[k], net_ptr[k + 1]).  Stored quad by quad in blocks of 32
+  // chunks ([block][net_quads][32]).
+  // For mechanisms of up to kFewBlocks blocks of reactions instead: {species,
+  // first, end, 0} by decreasing length, and the terms (net_chunks = 0 then).
   const int4 *sn_rec;
   const int *sn_step;
+  int net_chunks, net_quads;
+  const int4 *net_ent;
+  const int *net_slot, *net_ptr;
   // both lists of a species for the rates kernel, longest first: {species,
   // number of terms, first record, number of destruction terms} and records of
   // four 16-bit steps, destruction first (unused places repeat the last step)
@@ -119,6 +129,12 @@ struct DevMech {
   // molecular weights, their reciprocals and the thermodynamic fits: bytes from mw on
   int spc_bytes;
 };
+
+constexpr int kFewBlocks = 4;
+
+// Doubles of the partial sums of net_ent's chunks: at most 3 nsp + 2 chunks,
+// and a species boundary each.
+__host__ __device__ inline int net_slots(int nsp) { return 4 * nsp + 2; }
 
 // Host-side builder; owns the device allocation.
 class DeviceMechanism {

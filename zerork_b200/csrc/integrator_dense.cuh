@@ -40,6 +40,7 @@ struct Smem {
   double *D, *y, *f, *f0, *ypred, *psi, *d, *scale, *tmp, *yp;
   void *A;      // n x lda inverse (LT)
   double *rows; // kPanelMax x n pivot rows of the inversion: overlays vectors that are dead then
+  double *part; // net_slots partial sums of the net rates: overlays what the reactions leave unread
   int *perm;    // n + 1: low half of entry j the pivot row of column j, high half of entry i
                 // the column that row i was the pivot of; entry n the singular flag
   double *colk; // n: operator product of the Krylov path
@@ -116,12 +117,14 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
   double v = v0;
   if (o.cp || s.src.dpdt != 0.0 || s.src.esrc != 0.0)
     source_cta(m, o, s, t, y, clamp, v0, T_force, T, v);
-  // this warp's first block of reactions: its records arrive during the
+  // this warp's first block of reactions (3 KB) on its way to L1 during the
   // species pass
   const int lane = tid & 31, w = tid >> 5, nw = nt >> 5;
-  RxnRec R;
-  R.flags = kNoRxn;
-  if (w < m.nblocks) R = load_slot(m.rxn_slots, w, lane);
+  auto fetch_block = [&](int b) {
+    if (b < m.nblocks && lane < 24)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(m.rxn_slots + (size_t)b * 192 + lane * 8));
+  };
+  fetch_block(w);
   const double logT = log(T), invT = 1.0 / T;
   const double dens = 1.0 / v;
   const double ush = o.cp ? 0.0 : 1.0;  // h/RT - 1 = u/RT; c_p/R - 1 = c_v/R
@@ -144,43 +147,86 @@ __device__ __noinline__ int rhs_cta(const DevMech &m, const IntegOpts &o, const 
   const double Csum = block_sum_at(pc, s.red + 16);
   // blocks of reactions in snake order over the warps
   for (int rr = 0; rr * nw < m.nblocks; ++rr) {
-    const RxnRec cur = R;
-    const int nb = (rr + 1) * nw + ((rr & 1) ? w : nw - 1 - w);
-    R.flags = kNoRxn;
-    if (nb < m.nblocks) R = load_slot(m.rxn_slots, nb, lane);
+    const int b = rr * nw + ((rr & 1) ? nw - 1 - w : w);
+    fetch_block((rr + 1) * nw + ((rr & 1) ? w : nw - 1 - w));
+    if (b >= m.nblocks) continue;
+    const RxnRec cur = load_slot(m.rxn_slots, b, lane);
     if (!(cur.flags & kNoRxn))
       reaction_item<1, 1>(m, cur, 0, s.C, s.G, s.ROP, &T, &logT, &invT, &Csum, o.lim);
   }
   double cv = 0.0;
   for (int i = 0; i < nw; ++i) cv += s.red[32 + i];
   __syncthreads();
-  // net production rates: eight lanes a species, the longest lists first (a
-  // thread a species walked lists of hundreds of steps with the index loads
-  // in its chain)
+  // Net production rates from equal chunks of the flat list: a chunk's entries
+  // and then its rates arrive together, partial sums go to s.part, and a thread
+  // a species adds those of its species.  (Eight lanes a species walked lists
+  // of very different lengths, some of hundreds of steps, through their
+  // pointers: 12.6 K of the
+  // right-hand side's 40 K cycles with 160 species.  With few reactions, whose
+  // tables L1 holds, that is still the shorter way: 1000 reactors of 27
+  // reactions 99 ms, 120 with chunks.)
   double pe = 0.0;
-  for (int p0 = tid >> 3; p0 - (lane >> 3) < S; p0 += nt >> 3) {
-    const int4 rec = m.sn_rec[min(p0, S - 1)];
-    const int k = p0 < S ? rec.x : -1;
-    double net = 0.0;
-    if (k >= 0) {
+  auto finish = [&](int k, double net) {
+    if (s.ysrc) {  // reactor_constant_volume_cpu.cpp:108-113
+      const double ys = s.ysrc[k];
+      ydot[k] = net * m.mw[k] * v + ys;
+      pe += s.U[k] * (net * v + ys * m.inv_mw[k]);
+    } else {
+      ydot[k] = net * m.mw[k] * v;
+      pe += s.U[k] * net * v;
+    }
+  };
+  if (m.net_chunks > 0) {
+    const int k0 = min(tid, S - 1), pb = m.net_ptr[k0], pend = m.net_ptr[k0 + 1];
+    for (int ch = tid; ch < m.net_chunks; ch += nt) {
+      const int4 *ent = m.net_ent + (size_t)(ch >> 5) * m.net_quads * 32 + (ch & 31);
+      double *out = s.part + m.net_slot[ch];
+      double acc = 0.0;
+      for (int q0 = 0; q0 < m.net_quads; q0 += 4) {
+        int w[16];
+        double r[16];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int4 e = ent[min(q0 + u, m.net_quads - 1) * 32];
+          w[4 * u] = e.x;
+          w[4 * u + 1] = e.y;
+          w[4 * u + 2] = e.z;
+          w[4 * u + 3] = e.w;
+        }
+#pragma unroll
+        for (int u = 0; u < 16; ++u) r[u] = s.ROP[w[u] & 0x3fffffff];
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+          if (q0 + u / 4 < m.net_quads) {
+            acc += w[u] < 0 ? -r[u] : r[u];
+            if (w[u] & 0x40000000) {
+              *out++ = acc;
+              acc = 0.0;
+            }
+          }
+      }
+    }
+    __syncthreads();
+    for (int k = tid; k < S; k += nt) {
+      const int b = k == tid ? pb : m.net_ptr[k], e = k == tid ? pend : m.net_ptr[k + 1];
+      double net = 0.0;
+#pragma unroll 4
+      for (int i = b; i < e; ++i) net += s.part[i];
+      finish(k, net);
+    }
+  } else {  // few reactions: eight lanes a species, no second barrier
+    for (int p0 = tid >> 3; p0 - (lane >> 3) < S; p0 += nt >> 3) {
+      const int4 rec = m.sn_rec[min(p0, S - 1)];
+      double net = 0.0;
 #pragma unroll 4
       for (int e = rec.y + (lane & 7); e < rec.z; e += 8) {
         const int st = m.sn_step[e];
         const double r = s.ROP[st & 0x7fffffff];
         net += st < 0 ? -r : r;
       }
-    }
 #pragma unroll
-    for (int off = 1; off < 8; off <<= 1) net += __shfl_xor_sync(kFull, net, off);
-    if (k >= 0 && (lane & 7) == 0) {
-      if (s.ysrc) {  // reactor_constant_volume_cpu.cpp:108-113
-        const double ys = s.ysrc[k];
-        ydot[k] = net * m.mw[k] * v + ys;
-        pe += s.U[k] * (net * v + ys * m.inv_mw[k]);
-      } else {
-        ydot[k] = net * m.mw[k] * v;
-        pe += s.U[k] * net * v;
-      }
+      for (int off = 1; off < 8; off <<= 1) net += __shfl_xor_sync(kFull, net, off);
+      if (p0 < S && (lane & 7) == 0) finish(rec.x, net);
     }
   }
   const double es = block_sum_at(pe, s.red + 48);
@@ -309,8 +355,9 @@ __device__ __noinline__ int jac_cta(const DevMech &m, const IntegOpts &o, const 
 // once per pair (162 passes of shared memory at n = 161) with four block
 // barriers each.  Panel width: what the registers of the panel warp hold,
 // NC x PB values (128 registers a thread at 512 threads).
-//   n = 161 FP64 (160 species)  1,410 K cycles before, 577 K now
-//   n = 80 FP64                   407 K cycles before, 172 K now
+//   n = 161 FP64 (160 species)  1,410 K cycles before, 577 K with one panel warp,
+//                                434 K with four, the rest in batches of rows on top
+//   n = 80 FP64                   407 K cycles before, 172 K, 102 K
 template <class LT>
 __device__ __forceinline__ unsigned pivot_key(LT a) {
   if constexpr (sizeof(LT) == 8) return (unsigned)__double2hiint(a) & 0x7fffffffu;
@@ -548,24 +595,38 @@ __device__ __noinline__ int invert_cta(const DevMech &m, const Smem &s, const do
 #pragma unroll
           for (int u = 0; u < PB; ++u) r[u][t] = (on[t] && u < pw) ? R[u * n + j] : (LT)0;
         }
-#pragma unroll 2
-        for (int i = i0; i < n; i += di) {
-          LT *row = A + i * lda;
-          // (the pivots of the next panel may be noted meanwhile, in entries
-          // that this test reads as outside [k, k2))
-          const bool piv = in_panel(i);
-          LT a[CH], wv[PB];
+        // a batch of rows at a time, every load before the stores (the compiler
+        // must keep the order of accesses to A)
+        constexpr int RB = sizeof(LT) == 8 && PB * CH >= 24 ? 2 : 3;
+        for (int ib = i0; ib < n; ib += RB * di) {
+          LT a[RB][CH], wv[RB][PB];
 #pragma unroll
-          for (int u = 0; u < PB; ++u) wv[u] = u < pw ? row[k + u] : (LT)0;
+          for (int e = 0; e < RB; ++e) {
+            const int i = min(ib + e * di, n - 1);
+            const LT *row = A + i * lda;
+            // (the pivots of the next panel may be noted meanwhile, in entries
+            // that this test reads as outside [k, k2))
+            const bool piv = in_panel(i);
 #pragma unroll
-          for (int t = 0; t < CH; ++t) a[t] = (on[t] && !piv) ? row[lane + 32 * (c0 + t)] : (LT)0;
+            for (int u = 0; u < PB; ++u) wv[e][u] = u < pw ? row[k + u] : (LT)0;
+#pragma unroll
+            for (int t = 0; t < CH; ++t) {
+              const LT x = on[t] ? row[lane + 32 * (c0 + t)] : (LT)0;
+              a[e][t] = piv ? (LT)0 : x;
+            }
+          }
 #pragma unroll
           for (int u = 0; u < PB; ++u)
 #pragma unroll
-            for (int t = 0; t < CH; ++t) a[t] += wv[u] * r[u][t];
+            for (int e = 0; e < RB; ++e)
 #pragma unroll
-          for (int t = 0; t < CH; ++t)
-            if (on[t]) row[lane + 32 * (c0 + t)] = a[t];
+              for (int t = 0; t < CH; ++t) a[e][t] += wv[e][u] * r[u][t];
+#pragma unroll
+          for (int e = 0; e < RB; ++e)
+            if (ib + e * di < n)
+#pragma unroll
+              for (int t = 0; t < CH; ++t)
+                if (on[t]) A[(ib + e * di) * lda + lane + 32 * (c0 + t)] = a[e][t];
         }
       }
     }
@@ -991,7 +1052,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
 #pragma unroll
         for (int k = 0; k <= kMaxOrder; ++k) dk[k] = k <= q ? s.D[k * n + i] : 0.0;  // loads together
 #pragma unroll
-        for (int k = 0; k <= kMaxOrder; ++k)
+        for (int k = kMaxOrder; k >= 0; --k)  // the high differences first: they are the smallest
           if (k <= q) {
             a += dk[k];
             if (k > 0) ps += bc.gam[k] * dk[k];
@@ -1028,7 +1089,7 @@ __device__ __forceinline__ int attempt_cta(const DevMech &m, const IntegOpts &o,
         constexpr bool kDirect = sizeof(LT) == sizeof(double);
         int bad = 0;
         for (int i = tid; i < n; i += nt) {
-          const double f = s.f[i], r = c * f - s.psi[i] - s.d[i];
+          const double f = s.f[i], r = c * f - (s.psi[i] + s.d[i]);
           bad |= !isfinite(f);
           s.tmp[i] = r;
           if (kDirect) s.bs[pivot_col(s.perm, i)] = r / s.wlu[i];
@@ -1261,13 +1322,14 @@ __global__ void __launch_bounds__(512, 1) integrate_dense_kernel(DevMech mp, Int
     s.rows = p;
     s.mlp = (float *)p;  // 2 * kPredBuf floats
     double *const end = p + dense_rows_doubles(S);
-    s.C = p; p += S;
-    s.G = p; p += S;
     s.U = p; p += S;
     s.f = p; p += n;
     s.f0 = p; p += n;
     s.tmp = p; p += n;
     s.yp = p; p += n;
+    s.part = p;  // C, G, colk and bs: 4 S + 2 doubles, dead while the net rates are summed
+    s.C = p; p += S;
+    s.G = p; p += S;
     s.colk = p; p += n;
     s.bs = p;
     p = end;

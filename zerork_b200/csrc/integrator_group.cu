@@ -80,6 +80,7 @@ __device__ Bound bind(const GroupKArgs &k, double *smem) {
   s.G = p; p += S;
   s.U = p; p += S;
   s.ROP = p; p += m.nstep;
+  s.part = p; p += net_slots(S);
   s.mlp = nullptr;
   s.Jsm = nullptr;
   s.V = nullptr;
@@ -667,7 +668,7 @@ cudaError_t integrate_group(const DevMech &m, const IntegOpts &o, const IntegArg
   drv.part_h = part_host;
   make_consts(drv.bc);
   // reduction slots, then the rates workspace or the inversion's pivot rows
-  const size_t ws = std::max(3 * (size_t)S + m.nstep, (size_t)kPanelMax * n);
+  const size_t ws = std::max(3 * (size_t)S + m.nstep + net_slots(S), (size_t)kPanelMax * n);
   drv.k.ws_doubles = (int)(128 + ws);
   drv.smem = (128 + ws) * sizeof(double);
   const size_t kSmemMax = 227 * 1024;

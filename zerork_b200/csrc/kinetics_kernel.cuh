@@ -94,7 +94,7 @@ __device__ __forceinline__ bool rop_change(const RxnRec &R, int q, const double 
 #pragma unroll
     for (int k = 0; k < V; ++k) xr[k] = R.n_r * dlogT[k] - R.Ta_r * dinvT[k];
   } else if (R.flags & kRevKeq) {
-    gibbs_from_rows<TS, V>(R, q, sdG, xr);
+    gibbs_from_rows<TS, V, false>(R, q, sdG, xr);
 #pragma unroll
     for (int k = 0; k < V; ++k) xr[k] += xf[k] + R.lnA_r * dlogT[k];
   }
@@ -112,9 +112,7 @@ __device__ __forceinline__ bool rop_change(const RxnRec &R, int q, const double 
       c[k] = 1.0;
     }
     if (limited) {
-      each_species(count, spc, [&](int sp) {
-        double y[V];
-        ldv<V>(sC + sp * TS + q, y);
+      each_row<TS, V, false>(sC, q, count, spc, [&](const double (&y)[V]) {
 #pragma unroll
         for (int k = 0; k < V; ++k) c[k] *= y[k];
       });
@@ -385,8 +383,8 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
         }
         double gs[V];
         if (pass == 1 && (R.flags & kRevKeq)) gibbs_from_fits<V>(SB(thermo), R, Tq, lq, gs);
-        else gibbs_from_rows<TS, V>(R, q, sG, gs);
-        reaction_eval<TS, V>(m, R, q, sC, gs, sROP, Tq, lq, iq, Csum, kp.lim, nullptr, tab);
+        else gibbs_from_rows<TS, V, false>(R, q, sG, gs);
+        reaction_eval<TS, V, false>(m, R, q, sC, gs, sROP, Tq, lq, iq, Csum, kp.lim, nullptr, tab);
         if (pass == 1) {
           double x[V];
           ldv<V>(sROP + R.fwd * TS + q, x);
