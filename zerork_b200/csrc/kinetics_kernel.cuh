@@ -416,6 +416,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
           for (int pos = 0; pos < rec.y; pos += 4) {
             const int2 it = nx;
             nx = *++steps;
+            if (!STAGE && (pos & 63) == 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(steps + 16));
             double x[4][V];
             ldv<V>(sROP + (it.x & 0xffff) * TS + q, x[0]);
             ldv<V>(sROP + (int)((unsigned)it.x >> 16) * TS + q, x[1]);
@@ -526,9 +527,18 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
               int jend = TB(jf_ptr)[j + 1];
               const int4 *items = TB(jit);
               int4 nx = items[f0];
+              // list records of this and the next items on their way to L1, a
+              // line of each ahead
+              auto ahead = [&](const void *p) {
+                if constexpr (!STAGE) asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+              };
+              const int2 *ext = TB(jext);
+              ahead(items + min(f0 + 8, m.nj));
+              ahead(ext + nx.w);
               for (int f = f0; f < f1; ++f) {
                 const int4 it = nx;
                 nx = items[f + 1];  // in flight during this item (the list ends in a sentinel)
+                if ((f & 7) == 0) ahead(items + min(f + 16, m.nj));
                 while (f == jend) {  // column j ends inside this share
                   stv<V>(sTP + (j + g) * TS + q, trow);
                   ++j;
@@ -537,32 +547,40 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
                 }
                 const int row = it.x & 0xffff, nd = (int)((unsigned)it.x >> 16);
                 const double conv = SB(mw)[row] * wcol;
-                double r[4][V], u[V], val[V];
-                ldv<V>(sROP + (it.y & 0xffff) * TS + q, r[0]);
-                ldv<V>(sROP + (int)((unsigned)it.y >> 16) * TS + q, r[1]);
-                ldv<V>(sROP + (it.z & 0xffff) * TS + q, r[2]);
-                ldv<V>(sROP + (int)((unsigned)it.z >> 16) * TS + q, r[3]);
+                double r[4][V], u[V], val[V], odd[V];
+                auto rows = [&](int a, int b) {
+                  ldv<V>(sROP + (a & 0xffff) * TS + q, r[0]);
+                  ldv<V>(sROP + (int)((unsigned)a >> 16) * TS + q, r[1]);
+                  ldv<V>(sROP + (b & 0xffff) * TS + q, r[2]);
+                  ldv<V>(sROP + (int)((unsigned)b >> 16) * TS + q, r[3]);
+                };
+                rows(it.y, it.z);
                 ldv<V>(sU + row * TS + q, u);
-                FORV val[k] = 0.0;
-                // destruction terms first, then creation (SetupJacobianSparse order)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const double sg = e < nd ? -1.0 : 1.0;
-                  FORV val[k] = fma(sg, r[e][k], val[k]);
-                }
-                int pos = 4;
-                for (int c = it.w; c < nx.w; ++c, pos += 4) {  // further terms, four a record
-                  const int2 more = TB(jext)[c];
-                  ldv<V>(sROP + (more.x & 0xffff) * TS + q, r[0]);
-                  ldv<V>(sROP + (int)((unsigned)more.x >> 16) * TS + q, r[1]);
-                  ldv<V>(sROP + (more.y & 0xffff) * TS + q, r[2]);
-                  ldv<V>(sROP + (int)((unsigned)more.y >> 16) * TS + q, r[3]);
+                FORV val[k] = odd[k] = 0.0;
+                // destruction terms negative; two chains
+                auto add = [&](int pos) {
 #pragma unroll
                   for (int e = 0; e < 4; ++e) {
                     const double sg = pos + e < nd ? -1.0 : 1.0;
-                    FORV val[k] = fma(sg, r[e][k], val[k]);
+                    FORV {
+                      if (e & 1) odd[k] = fma(sg, r[e][k], odd[k]);
+                      else val[k] = fma(sg, r[e][k], val[k]);
+                    }
                   }
+                };
+                add(0);
+                if (it.w < nx.w) {  // further terms, four a record, the next one in flight
+                  int2 more = ext[it.w];
+                  for (int c = it.w; c < nx.w; ++c) {
+                    const int2 cur = more;
+                    more = ext[min(c + 1, nx.w - 1)];
+                    if ((c & 15) == 0) ahead(ext + c + 16);
+                    rows(cur.x, cur.y);
+                    add(4 * (c - it.w + 1));
+                  }
+                  ahead(ext + nx.w);
                 }
+                FORV val[k] += odd[k];
                 FORV {
                   val[k] *= t2[k];
                   trow[k] += val[k] * u[k];
