@@ -77,7 +77,10 @@ int zrk_mech_get_double_option(zrk_mech_t m, const char *name, double *value);
  * the workspace (rejected when the two do not fit), bit 2
  * (ZRK_LAUNCH_TWO_CTAS, up to 8 warps and 16 states per tile, tables not
  * staged) compiles the kernel for two resident CTAs per SM (at most 128
- * registers per thread).  ts = 0 restores the default mapping. */
+ * registers per thread).  ts = 0 restores the default: every call takes the
+ * tile size from its number of states (a set or tuned mapping serves all
+ * sizes); zrk_mech_get_launch then reports the mapping that
+ * zrk_rates_jac_dev_noalloc uses. */
 #define ZRK_LAUNCH_GLOBAL_WS 1
 #define ZRK_LAUNCH_STAGE_TABLES 2
 #define ZRK_LAUNCH_TWO_CTAS 4

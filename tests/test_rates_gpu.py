@@ -309,3 +309,60 @@ def test_rates_tc_per_step_limiter(torch, mech, therm):
     hn, hc, hd, hr = pm.rates_tc_host(T, np.ascontiguousarray(Cc.T), lim)
     dn, dc, dd, dr = _tc_run(torch, pm, T, Cc, lim)
     assert np.array_equal(hn.T, dn) and np.array_equal(hr.T, dr)
+
+
+@pytest.mark.parametrize("jac", [True, False])
+def test_default_mapping_edges(torch, jac, mech_dir):
+    """The mapping that a call takes from its size gives the results of a fixed
+    one at the edges of every rule (tile remainders, waves of 148 tiles, two
+    CTAs per SM), with odd and even leading dimensions (16-byte accesses or
+    not) and with clamped states (zero mass fractions) among the others.
+    Bound: both are within TOL of the oracle's rounding scale elsewhere; here
+    net rates against the largest rate of the state, entries against the
+    largest of their column."""
+    import zerork_b200 as zb
+    from zerork_b200 import mechgen
+    g, (m, t) = synth("c2_53", mech_dir)
+    auto, fixed = zb.Mechanism(m, t), zb.Mechanism(m, t)
+    fixed.set_launch(8, 1, 8)
+    T, P, Y = mechgen.rate_states(g, 4740, seed=17)
+    Y[5::7, 3:20] = 0.0
+    for n, ld in ((1, 1), (7, 9), (9, 10), (1184, 1184), (1185, 1187), (2369, 2370), (4735, 4735), (4736, 4738)):
+        dev = [torch.from_numpy(a[:n].copy()).cuda() for a in (T, P)]
+        Yd = torch.zeros((auto.nsp, ld), dtype=torch.float64, device="cuda")
+        Yd[:, :n] = torch.from_numpy(np.ascontiguousarray(Y[:n].T)).cuda()
+        out = []
+        for pm in (auto, fixed):
+            W = torch.zeros((pm.nsp, ld), dtype=torch.float64, device="cuda")
+            J = torch.zeros((pm.nnz, ld), dtype=torch.float64, device="cuda") if jac else None
+            D = torch.zeros((pm.nsp + 1, ld), dtype=torch.float64, device="cuda")
+            pm.rates_jac(dev[0], dev[1], Yd, W, J, D, n=n)
+            out.append([x.cpu().numpy() for x in (W, J, D) if x is not None])
+        for a, b in zip(*out):
+            assert np.all(a[:, n:] == 0.0)
+            assert np.all(np.abs(a - b) <= 1e-9 * np.abs(b).max(axis=0, keepdims=True)), n
+
+
+def test_small_rate_calls(torch, mech_dir):
+    """Rates from (T, C) at the edges of the small paths (a state per CTA up to
+    one per SM, pinned staging up to 256 KB: 40 states of this mechanism)
+    against the general path's tiles; the same operations per state, summed in
+    the same order."""
+    import zerork_b200 as zb
+    from zerork_b200 import mechgen
+    g, (m, t) = synth("c2_53", mech_dir)
+    pm = zb.Mechanism(m, t)
+    T, P, Y = mechgen.rate_states(g, 300, seed=19)
+    iw = 1.0 / pm.table("mw")
+    C = np.ascontiguousarray((Y * iw * (P / (8314.462618 * T) / (Y * iw).sum(1))[:, None]).T)
+    lim = np.full(pm.nstep, 1e22)
+    ref = [x.cpu().numpy() for x in pm.rates_tc(torch.from_numpy(T).cuda(), torch.from_numpy(C).cuda(),
+                                                torch.from_numpy(lim).cuda())]
+    for n in (1, 2, 39, 40, 41, 148, 149):
+        got = pm.rates_tc_host(T[:n], np.ascontiguousarray(C[:, :n]), lim)
+        dev = pm.rates_tc(torch.from_numpy(T[:n].copy()).cuda(), torch.from_numpy(np.ascontiguousarray(C[:, :n])).cuda(),
+                          torch.from_numpy(lim).cuda())
+        for a, d, r in zip(got, dev, ref):
+            scale = np.abs(ref[1][:, :n]).max(axis=0) + np.abs(ref[2][:, :n]).max(axis=0)
+            assert np.all(np.abs(a - r[:, :n]) <= 1e-12 * np.maximum(scale, np.abs(r[:, :n])))
+            assert np.array_equal(a, d.cpu().numpy())
