@@ -43,7 +43,6 @@ struct Smem {
   double *part; // net_slots partial sums of the net rates: overlays what the reactions leave unread
   int *perm;    // n + 1: low half of entry j the pivot row of column j, high half of entry i
                 // the column that row i was the pivot of; entry n the singular flag
-  double *colk; // n: operator product of the Krylov path
   double *wlu;  // n: error-weight scale the stored inverse was formed with
   double *bs;   // n: scaled right-hand side
   double *V;    // FP32 path: (kMaxl + 1) Krylov vectors, then 2 work vectors
@@ -1341,10 +1340,10 @@ __global__ void __launch_bounds__(512, 1) integrate_dense_kernel(DevMech mp, Int
     s.f0 = p; p += n;
     s.tmp = p; p += n;
     s.yp = p; p += n;
-    s.part = p;  // C, G, colk and bs: 4 S + 2 doubles, dead while the net rates are summed
+    s.part = p;  // C, G, n doubles and bs: 4 S + 2, dead while the net rates are summed
     s.C = p; p += S;
     s.G = p; p += S;
-    s.colk = p; p += n;
+    p += n;
     s.bs = p;
     p = end;
     if (spill & 1) { s.ROP = g; } else { s.ROP = p; p += N; }

@@ -95,7 +95,7 @@ __device__ Bound bind(const GroupKArgs &k, double *smem) {
   s.scale = g; g += n;
   s.tmp = g; g += n;
   s.yp = g; g += n;
-  s.colk = g; g += n;
+  g += n;
   s.wlu = g; g += n;
   s.bs = g; g += n;
   s.r1g = g; g += n;
