@@ -132,6 +132,66 @@ def test_gpu_tiles_and_slices(torch, n_in, hidden, layers, n_out, batch, rows):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n_in,hidden,layers,n_out,batch", [
+    (3, 16, 1, 2, 2048), (17, 100, 2, 65, 80), (163, 256, 3, 128, 4096)])
+def test_gpu_sums_run_over_the_batch_in_order(torch, n_in, hidden, layers, n_out, batch):
+    """Gradients are one sum over the rows in order and the loss a fixed tree,
+    so training repeats bit for bit whatever tiles and slices a version uses.
+    Exact: the bias gradient of the output layer and the loss (up to 128
+    outputs: one column a thread) from the outputs, in FP32, in that order."""
+    from zerork_b200.predictor import Mlp
+    rng = np.random.default_rng(7)
+    net = Mlp(n_in, n_out, hidden, layers, seed=3)
+    d, w, b = _net(rng, n_in, hidden, layers, n_out)
+    net.set_params(w, b)
+    x = torch.from_numpy(rng.standard_normal((batch, n_in)).astype(np.float32)).cuda()
+    t = rng.standard_normal((batch, n_out)).astype(np.float32)
+    loss = torch.zeros(1, dtype=torch.float32, device="cuda")
+    net.gradients(x, torch.from_numpy(t).cuda(), loss)
+    e = net.forward(x).cpu().numpy() - t
+    scale = np.float32(2.0) / (np.float32(batch) * np.float32(n_out))
+    gb = net.grads()[1][-d[-1]:][:n_out]
+    assert np.array_equal(gb, np.add.accumulate(scale * e, axis=0, dtype=np.float32)[-1])
+
+    def tree(v):  # 32 lanes, halving distances
+        for o in (16, 8, 4, 2, 1):
+            v = v + v[..., np.arange(32) ^ o]
+        return v[..., 0]
+
+    def in_order(v):
+        return np.add.accumulate(v, axis=-1, dtype=np.float32)[..., -1]
+
+    sq = np.zeros((batch, 128), np.float32)
+    sq[:, :n_out] = e * e
+    rows = np.zeros(-(-batch // 256) * 256, np.float32)
+    rows[:batch] = in_order(tree(sq.reshape(batch, 4, 32)))
+    assert loss.item() == in_order(tree(in_order(rows.reshape(-1, 256).T).reshape(8, 32)))
+
+
+@pytest.mark.gpu
+def test_gpu_weight_gradient_is_one_chain(torch):
+    """A weight gradient adds the batch rows 16 at a time to one accumulator:
+    with a first row of 1 and one row of 1.5 * 2^-26 in each following 16, every
+    addition is below half a unit of the accumulator and is lost, while partial
+    sums of any four of them would not be."""
+    from zerork_b200.predictor import Mlp
+    net = Mlp(1, 2, 1, 1, seed=3)
+    d = mo.dims(1, 1, 1, 2)
+    w, b = np.zeros(net.nw, np.float32), np.zeros(net.nb, np.float32)
+    b[0] = 1.0  # hidden activation silu(1) in every row, outputs 0
+    net.set_params(w, b)
+    n = 2048
+    t = np.zeros((n, 2), np.float32)
+    t[16::16, 0] = -1.5 * 2.0 ** -26
+    t[0, 0] = -1.0
+    loss = torch.zeros(1, dtype=torch.float32, device="cuda")
+    net.gradients(torch.zeros((n, 1), device="cuda"), torch.from_numpy(t).cuda(), loss)
+    gw, _ = net.grads()
+    silu1 = mo.bf16(np.float32(1.0 / (1.0 + np.exp(-1.0))))
+    assert mo.unpack(gw, np.zeros(net.nb, np.float32), d)[0][1][0, 0] == silu1 * np.float32(2.0 / (2 * n))
+
+
+@pytest.mark.gpu
 def test_gpu_training_reduces_loss(torch):
     from zerork_b200.predictor import train
     rng = np.random.default_rng(4)

@@ -16,18 +16,22 @@
 //     cp.async pipeline of 32-deep slices, ldmatrix and m16n8k16 products with
 //     FP32 accumulators; transposed operands (X^T dZ, dZ W^T) are read in
 //     place and transposed by ldmatrix;
-//   * bias, SiLU, its derivative, the loss gradient and the bias-gradient
-//     column sums work on the accumulators, so no pass re-reads an output;
-//   * the weight gradient, whose output has only 16 tiles, is split over the
-//     batch rows into partial sums that one kernel adds in a fixed order, and
-//     shares its launch with the input gradient of the same layer.
+//   * bias, SiLU, its derivative and the loss gradient work on the accumulators;
+//   * the weight gradients and bias gradients of all layers form one launch
+//     after the input gradients.  Each is one sum over the batch rows in order,
+//     not a sum of slices, so a training run repeats bit for bit whatever the
+//     tiling; 32 x 64 tiles of every layer run side by side (112 of the network
+//     below, on 148 SMs) and last as long as one chain of 4096 / 16 products.
+//     (Deeper pipelines, 60 KB in flight instead of 24, changed nothing.  Sums
+//     of slices of the batch took 1.11 ms where this takes 1.19.)
 // 163-256-256-256-161 on a B200: eight training steps at batch 4096, a forward
-// pass of 5,001 rows and the copy of the parameters to the host took 15.3 ms
+// pass of 5,001 rows and the copy of the parameters to the host took 15.2 ms
 // with a kernel for each elementwise pass, products straight from global
-// memory and one block per weight-gradient tile, and take 1.11 ms now.
+// memory and one block per weight-gradient tile, and take 1.19 ms now.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -59,9 +63,9 @@ __global__ void input_to_bf16(int rows, int n_in, int K0, const float *__restric
 }
 
 constexpr int kBM = 64, kBN = 64, kBK = 32, kStages = 3;
-constexpr int kPadK = kBK + 8, kPadM = kBM + 8;  // padded rows: ldmatrix without bank conflicts
-constexpr int kTileElems = kBM * kPadK;          // >= kBK * kPadM
-static_assert(kBK * kPadM <= kTileElems && kBM == kBN, "operand tile size");
+// Elements of an operand tile of R (the output dimension) x BK in either layout;
+// rows padded by 16 bytes: ldmatrix without bank conflicts.
+constexpr int tile_elems(int R, int BK, bool mk) { return mk ? R * (BK + 8) : BK * (R + 8); }
 
 __device__ __forceinline__ void cp16(void *dst, const void *src, bool on) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -80,79 +84,81 @@ __device__ __forceinline__ void ldsm4(unsigned (&r)[4], const bf16 *p) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
 
-// One operand tile of 64 (the output dimension) x kBK.  MK: memory rows run
+// One operand tile of R (the output dimension) x BK.  MK: memory rows run
 // along the output dimension (row stride ld, k contiguous), kept as
-// [64][kPadK]; otherwise memory rows run along k, kept as [kBK][kPadM].
+// [R][BK + 8]; otherwise memory rows run along k, kept as [BK][R + 8].
 // Everything outside (lim, klim) reads as zero; both are multiples of 8.
-template <bool MK>
+template <int R, int BK, bool MK>
 __device__ __forceinline__ void load_tile(bf16 *t, const bf16 *__restrict__ g, int ld, int r0, int lim, int k0,
                                           int klim) {
 #pragma unroll
-  for (int i = 0; i < kBM * kBK / 8 / 128; ++i) {
+  for (int i = 0; i < R * BK / 8 / 128; ++i) {
     const int c = threadIdx.x + i * 128;
     if constexpr (MK) {
-      const int r = c / (kBK / 8), k = c % (kBK / 8) * 8;
+      const int r = c / (BK / 8), k = c % (BK / 8) * 8;
       const bool on = r0 + r < lim && k0 + k < klim;
-      cp16(t + r * kPadK + k, on ? g + (size_t)(r0 + r) * ld + k0 + k : g, on);
+      cp16(t + r * (BK + 8) + k, on ? g + (size_t)(r0 + r) * ld + k0 + k : g, on);
     } else {
-      const int k = c / (kBM / 8), r = c % (kBM / 8) * 8;
+      const int k = c / (R / 8), r = c % (R / 8) * 8;
       const bool on = r0 + r < lim && k0 + k < klim;
-      cp16(t + k * kPadM + r, on ? g + (size_t)(k0 + k) * ld + r0 + r : g, on);
+      cp16(t + k * (R + 8) + r, on ? g + (size_t)(k0 + k) * ld + r0 + r : g, on);
     }
   }
 }
 
-// acc = A B over k in [k0, k1) for the 64 x 64 tile at (m0, n0): warp (wm, wn)
-// owns 32 x 32 as 2 x 4 fragments of 16 x 8.  TA: A is stored [K x M]; TB: B
-// is stored [N x K].
-template <bool TA, bool TB>
-__device__ __forceinline__ void tile_product(bf16 *sm, float (&acc)[2][4][4], int M, int N, int m0, int n0, int k0,
-                                             int k1, const bf16 *__restrict__ A, int lda,
+// acc = A B over all K for the 32 FM x 64 tile at (m0, n0), one chain of k in
+// ascending steps of 16: warp (wm, wn) owns 16 FM x 32 as FM x 4 fragments of
+// 16 x 8.  TA: A is stored [K x M]; TB: B is stored [N x K].  ST slices of BK
+// in shared memory.
+template <int FM, int BK, int ST, bool TA, bool TB>
+__device__ __forceinline__ void tile_product(bf16 *sm, float (&acc)[FM][4][4], int M, int N, int m0, int n0, int K,
+                                             const bf16 *__restrict__ A, int lda,
                                              const bf16 *__restrict__ B, int ldb) {
+  constexpr int BM = 32 * FM, EA = tile_elems(BM, BK, !TA), EB = tile_elems(kBN, BK, TB);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+  const int wm = (warp >> 1) * 16 * FM, wn = (warp & 1) * 32;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < FM; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0f;
-  const int nk = (k1 - k0 + kBK - 1) / kBK;
+  const int nk = (K + BK - 1) / BK;
   auto fetch = [&](int it) {
     if (it < nk) {
-      bf16 *t = sm + (it % kStages) * 2 * kTileElems;
-      load_tile<!TA>(t, A, lda, m0, M, k0 + it * kBK, k1);
-      load_tile<TB>(t + kTileElems, B, ldb, n0, N, k0 + it * kBK, k1);
+      bf16 *t = sm + (it % ST) * (EA + EB);
+      load_tile<BM, BK, !TA>(t, A, lda, m0, M, it * BK, K);
+      load_tile<kBN, BK, TB>(t + EA, B, ldb, n0, N, it * BK, K);
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
 #pragma unroll
-  for (int i = 0; i < kStages - 1; ++i) fetch(i);
+  for (int i = 0; i < ST - 1; ++i) fetch(i);
   for (int it = 0; it < nk; ++it) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2) : "memory");
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");
     __syncthreads();  // slice `it` has arrived, and everyone is done with slice it - 1
-    fetch(it + kStages - 1);
-    const bf16 *ta = sm + (it % kStages) * 2 * kTileElems, *tb = ta + kTileElems;
+    fetch(it + ST - 1);
+    const bf16 *ta = sm + (it % ST) * (EA + EB), *tb = ta + EA;
 #pragma unroll
-    for (int kk = 0; kk < kBK; kk += 16) {
-      unsigned a[2][4], b[2][4];
+    for (int kk = 0; kk < BK; kk += 16) {
+      unsigned a[FM][4], b[2][4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < FM; ++i) {
         // lanes 0-15 address rows 0-15 at k, lanes 16-31 the same rows at k + 8
         if constexpr (!TA)
-          ldsm4<false>(a[i], ta + (wm + 16 * i + (lane & 15)) * kPadK + kk + (lane >> 4) * 8);
+          ldsm4<false>(a[i], ta + (wm + 16 * i + (lane & 15)) * (BK + 8) + kk + (lane >> 4) * 8);
         else
-          ldsm4<true>(a[i], ta + (kk + (lane & 7) + (lane >> 4) * 8) * kPadM + wm + 16 * i + ((lane >> 3) & 1) * 8);
+          ldsm4<true>(a[i], ta + (kk + (lane & 7) + (lane >> 4) * 8) * (BM + 8) + wm + 16 * i + ((lane >> 3) & 1) * 8);
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {  // 16 columns: two 8-wide fragments of (k, k + 8)
         if constexpr (!TB)
-          ldsm4<true>(b[j], tb + (kk + (lane & 15)) * kPadM + wn + 16 * j + (lane >> 4) * 8);
+          ldsm4<true>(b[j], tb + (kk + (lane & 15)) * (kBN + 8) + wn + 16 * j + (lane >> 4) * 8);
         else
-          ldsm4<false>(b[j], tb + (wn + 16 * j + (lane & 7) + (lane >> 4) * 8) * kPadK + kk + ((lane >> 3) & 1) * 8);
+          ldsm4<false>(b[j], tb + (wn + 16 * j + (lane & 7) + (lane >> 4) * 8) * (BK + 8) + kk + ((lane >> 3) & 1) * 8);
       }
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < FM; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           float *c = acc[i][j];
@@ -166,205 +172,213 @@ __device__ __forceinline__ void tile_product(bf16 *sm, float (&acc)[2][4][4], in
     }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();  // the caller may reuse the operand slices
 }
 
 // The accumulator pairs of this thread: f(row, col, i, j, h) for elements
 // (row, col) and (row, col + 1), which are acc[i][j][2 h] and [2 h + 1].
-template <class F>
+template <int FM, class F>
 __device__ __forceinline__ void for_pairs(int m0, int n0, F f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < FM; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        f(m0 + (warp >> 1) * 32 + 16 * i + 8 * h + (lane >> 2), n0 + (warp & 1) * 32 + 8 * j + (lane & 3) * 2, i, j, h);
-}
-
-// Column sums of the tile (its rows are the batch rows m0 .. m0 + 63) into
-// part[blockrow][N]: over the fragments of a thread, the eight row lanes, the
-// two warps of a column half, always in that order.
-__device__ __forceinline__ void tile_colsum(float *sm, const float (&v)[2][4][4], int N, int n0, float *part) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float s = (v[0][j][e] + v[0][j][e + 2]) + (v[1][j][e] + v[1][j][e + 2]);
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane < 4) sm[(warp >> 1) * kBN + (warp & 1) * 32 + 8 * j + lane * 2 + e] = s;
-    }
-  __syncthreads();
-  if (threadIdx.x < kBN && n0 + (int)threadIdx.x < N) part[n0 + threadIdx.x] = sm[threadIdx.x] + sm[kBN + threadIdx.x];
+        f(m0 + (warp >> 1) * 16 * FM + 16 * i + 8 * h + (lane >> 2), n0 + (warp & 1) * 32 + 8 * j + (lane & 3) * 2, i, j, h);
 }
 
 // Forward layer, output Z = X W + b.  MODE 0: hidden layer, X' = bf16(silu(Z))
 // and Z kept when the backward pass will want it (Zout not null); 1: output
 // layer of an evaluation, y on the valid rows and columns; 2: output layer of
-// a training step, the gradient of the mean squared error 2 (y - t) / (rows
-// n_out) as bf16 (zero on padding columns), its column sums (the bias
-// gradient of this block of rows) and this tile's squared error.
+// a training step, the errors y - t (Zout) and the gradient of the mean squared
+// error 2 (y - t) / (rows n_out) as bf16, both zero on padding columns.
 template <int MODE>
 __global__ void __launch_bounds__(128) layer_forward(int M, int N, int K, const bf16 *__restrict__ X,
                                                      const bf16 *__restrict__ W, const float *__restrict__ bias,
                                                      float *__restrict__ Zout, bf16 *__restrict__ Xout, int n,
-                                                     int n_out, const float *__restrict__ t, float *__restrict__ y,
-                                                     float *__restrict__ db_part, float *__restrict__ loss_part) {
-  __shared__ __align__(16) bf16 sm[kStages * 2 * kTileElems];
+                                                     int n_out, const float *__restrict__ t, float *__restrict__ y) {
+  __shared__ __align__(16) bf16 sm[kStages * (tile_elems(kBM, kBK, true) + tile_elems(kBN, kBK, false))];
   const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
   float acc[2][4][4];
-  tile_product<false, false>(sm, acc, M, N, m0, n0, 0, K, X, K, W, N);
-  float sq = 0.0f;
+  tile_product<2, kBK, kStages, false, false>(sm, acc, M, N, m0, n0, K, X, K, W, N);
   const float scale = MODE == 2 ? 2.0f / ((float)n * (float)n_out) : 0.0f;
-  for_pairs(m0, n0, [&](int r, int c, int i, int j, int h) {
-    float z[2] = {0.0f, 0.0f};
-    const bool on = r < M && c < N;
-    if (on) {
-      z[0] = acc[i][j][2 * h] + bias[c];
-      z[1] = acc[i][j][2 * h + 1] + bias[c + 1];
-    }
+  for_pairs<2>(m0, n0, [&](int r, int c, int i, int j, int h) {
+    if (r >= M || c >= N) return;
+    float z[2] = {acc[i][j][2 * h] + bias[c], acc[i][j][2 * h + 1] + bias[c + 1]};
     if constexpr (MODE == 0) {
-      if (on) {
-        if (Zout) *reinterpret_cast<float2 *>(Zout + (size_t)r * N + c) = make_float2(z[0], z[1]);
-        *reinterpret_cast<__nv_bfloat162 *>(Xout + (size_t)r * N + c) =
-            __halves2bfloat162(__float2bfloat16(silu(z[0])), __float2bfloat16(silu(z[1])));
-      }
+      if (Zout) *reinterpret_cast<float2 *>(Zout + (size_t)r * N + c) = make_float2(z[0], z[1]);
+      *reinterpret_cast<__nv_bfloat162 *>(Xout + (size_t)r * N + c) =
+          __halves2bfloat162(__float2bfloat16(silu(z[0])), __float2bfloat16(silu(z[1])));
     } else if constexpr (MODE == 1) {
 #pragma unroll
       for (int e = 0; e < 2; ++e)
         if (r < n && c + e < n_out) y[(size_t)r * n_out + c + e] = z[e];
     } else {
-      float g[2] = {0.0f, 0.0f};
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-        if (on && c + e < n_out) {
-          const float d = z[e] - t[(size_t)r * n_out + c + e];
-          sq += d * d;
-          g[e] = scale * d;
-        }
-      if (on)
-        *reinterpret_cast<__nv_bfloat162 *>(Xout + (size_t)r * N + c) =
-            __halves2bfloat162(__float2bfloat16(g[0]), __float2bfloat16(g[1]));
-      acc[i][j][2 * h] = g[0];
-      acc[i][j][2 * h + 1] = g[1];
+      for (int e = 0; e < 2; ++e) z[e] = c + e < n_out ? z[e] - t[(size_t)r * n_out + c + e] : 0.0f;
+      *reinterpret_cast<float2 *>(Zout + (size_t)r * N + c) = make_float2(z[0], z[1]);
+      *reinterpret_cast<__nv_bfloat162 *>(Xout + (size_t)r * N + c) =
+          __halves2bfloat162(__float2bfloat16(scale * z[0]), __float2bfloat16(scale * z[1]));
     }
   });
-  if constexpr (MODE == 2) {
-    float *red = reinterpret_cast<float *>(sm);
-    tile_colsum(red, acc, N, n0, db_part + (size_t)blockIdx.y * N);
+}
+
+// A row's squared error, as 128 threads sum it: thread c the columns c, c + 128,
+// ..., the 32 threads of each of four warps in a tree, the warps in order.
+__device__ __forceinline__ float row_error(const float *__restrict__ e, int n_out) {
+  const int lane = threadIdx.x & 31;
+  float s = 0.0f;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    float sq = 0.0f;
+    for (int c = 32 * w + lane; c < n_out; c += 128) sq = fmaf(e[c], e[c], sq);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if ((threadIdx.x & 31) == 0) red[2 * kBN + (threadIdx.x >> 5)] = sq;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      loss_part[blockIdx.y * gridDim.x + blockIdx.x] =
-          (red[2 * kBN] + red[2 * kBN + 1]) + (red[2 * kBN + 2] + red[2 * kBN + 3]);
+    s += sq;
   }
+  return s;
 }
 
-// Backward layer l: the first nw blocks form the partial weight gradients
-// X^T dZ (K x N) over slices of `chunk` batch rows, the rest the input
-// gradient dZ W^T (M x K) times silu'(Z) of the layer below, with its column
-// sums.  Both only read dZ, so they run side by side in one launch.
-__global__ void __launch_bounds__(128) layer_backward(int M, int N, int K, int nw, int chunk,
-                                                      const bf16 *__restrict__ X, const bf16 *__restrict__ dZ,
-                                                      float *__restrict__ dW_part, const bf16 *__restrict__ W,
-                                                      const float *__restrict__ Zin, bf16 *__restrict__ dZin,
-                                                      float *__restrict__ db_part) {
-  __shared__ __align__(16) bf16 sm[kStages * 2 * kTileElems];
-  float acc[2][4][4];
-  if ((int)blockIdx.x < nw) {
-    const int tn = (N + kBN - 1) / kBN, tk = (K + kBM - 1) / kBM;
-    const int slice = blockIdx.x / (tn * tk), rest = blockIdx.x % (tn * tk);
-    const int k0 = rest / tn * kBM, n0 = rest % tn * kBN;
-    const int r0 = slice * chunk, r1 = min(M, r0 + chunk);
-    tile_product<true, false>(sm, acc, K, N, k0, n0, r0, r1, X, K, dZ, N);
-    float *out = dW_part + (size_t)slice * K * N;
-    for_pairs(k0, n0, [&](int r, int c, int i, int j, int h) {
-      if (r < K && c < N)
-        *reinterpret_cast<float2 *>(out + (size_t)r * N + c) = make_float2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
-    });
+constexpr int kErrRows = 4;  // rows of a block of row errors
+
+// Input gradient of a layer (K inputs, N outputs): dZ W^T (M x K) times
+// silu'(Z) of the layer below, as bf16 for the next products and in FP32 in
+// Z's place for the bias gradient.  With the last layer, blocks from nb on sum
+// the squared errors of kErrRows rows each.
+__global__ void __launch_bounds__(128) layer_backward(int M, int N, int K, const bf16 *__restrict__ dZ,
+                                                      const bf16 *__restrict__ W, float *__restrict__ Z,
+                                                      bf16 *__restrict__ dZin, int nb,
+                                                      const float *__restrict__ err, int n_err, int n_out,
+                                                      float *__restrict__ row_sq) {
+  __shared__ __align__(16) bf16 sm[kStages * (tile_elems(kBM, kBK, true) + tile_elems(kBN, kBK, true))];
+  if ((int)blockIdx.x >= nb) {
+    for (int i = threadIdx.x >> 5; i < kErrRows; i += 4) {
+      const int r = ((int)blockIdx.x - nb) * kErrRows + i;
+      if (r >= M) break;
+      const float s = row_error(err + (size_t)r * n_err, n_out);
+      if ((threadIdx.x & 31) == 0) row_sq[r] = s;
+    }
     return;
   }
-  const int tk = (K + kBN - 1) / kBN, b = blockIdx.x - nw;
-  const int m0 = b / tk * kBM, n0 = b % tk * kBN;
-  tile_product<false, true>(sm, acc, M, K, m0, n0, 0, N, dZ, N, W, N);
-  for_pairs(m0, n0, [&](int r, int c, int i, int j, int h) {
-    float g[2] = {0.0f, 0.0f};
-    if (r < M && c < K) {
-      const float2 z = *reinterpret_cast<const float2 *>(Zin + (size_t)r * K + c);
-      const float zz[2] = {z.x, z.y};
+  float acc[2][4][4];
+  const int tk = (K + kBN - 1) / kBN, m0 = (int)blockIdx.x / tk * kBM, n0 = (int)blockIdx.x % tk * kBN;
+  tile_product<2, kBK, kStages, false, true>(sm, acc, M, K, m0, n0, N, dZ, N, W, N);
+  for_pairs<2>(m0, n0, [&](int r, int c, int i, int j, int h) {
+    if (r >= M || c >= K) return;
+    float2 *zp = reinterpret_cast<float2 *>(Z + (size_t)r * K + c);
+    const float zz[2] = {zp->x, zp->y};
+    float g[2];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const float s = 1.0f / (1.0f + expf(-zz[e]));
-        g[e] = acc[i][j][2 * h + e] * s * (1.0f + zz[e] * (1.0f - s));
-      }
-      *reinterpret_cast<__nv_bfloat162 *>(dZin + (size_t)r * K + c) =
-          __halves2bfloat162(__float2bfloat16(g[0]), __float2bfloat16(g[1]));
+    for (int e = 0; e < 2; ++e) {
+      const float s = 1.0f / (1.0f + expf(-zz[e]));
+      g[e] = acc[i][j][2 * h + e] * s * (1.0f + zz[e] * (1.0f - s));
     }
-    acc[i][j][2 * h] = g[0];
-    acc[i][j][2 * h + 1] = g[1];
+    *zp = make_float2(g[0], g[1]);
+    *reinterpret_cast<__nv_bfloat162 *>(dZin + (size_t)r * K + c) =
+        __halves2bfloat162(__float2bfloat16(g[0]), __float2bfloat16(g[1]));
   });
-  tile_colsum(reinterpret_cast<float *>(sm), acc, K, n0, db_part + (size_t)(m0 / kBM) * K);
 }
 
-// Where the partial sums of every layer's gradient are.
-struct GradParts {
-  int layers;
-  int slices[kMlpMaxLayers];               // partial weight gradients
-  long woff[kMlpMaxLayers + 1], boff[kMlpMaxLayers + 1];
-  const float *w[kMlpMaxLayers], *b[kMlpMaxLayers];
+constexpr int kGradM = 32, kGradK = 64, kGradStages = 3;  // tiles of the weight gradients
+constexpr int kColN = 32, kColRows = 64, kColStages = 5;  // of the bias gradients
+constexpr size_t kGradBytes = std::max(
+    kGradStages * (tile_elems(kGradM, kGradK, false) + tile_elems(kBN, kGradK, false)) * sizeof(bf16),
+    kColStages * kColRows * kColN * sizeof(float));
+
+// What the gradients of every layer are summed from.
+struct GradArgs {
+  int layers, rows;
+  int first_w[kMlpMaxLayers + 1], first_b[kMlpMaxLayers + 1];  // first block of each layer
+  int K[kMlpMaxLayers], N[kMlpMaxLayers];
+  const bf16 *X[kMlpMaxLayers], *dZ[kMlpMaxLayers];
+  const float *dZf[kMlpMaxLayers];  // the last: errors, to be scaled
+  float *gw[kMlpMaxLayers], *gb[kMlpMaxLayers];
+  float scale;
+  const float *row_sq;
+  float *loss;
 };
 
-// grad = the partial sums added in slice order (weights; four at a time, the
-// layers are multiples of 256 weights) and in block-row order (biases); the
-// last block adds the loss of the tiles.
-__global__ void __launch_bounds__(256) sum_parts(GradParts p, int blockrows, long nw, long nb, float *__restrict__ grad,
-                                                 int ntiles, const float *__restrict__ loss_part,
-                                                 float *__restrict__ loss) {
-  if (blockIdx.x == gridDim.x - 1) {
-    float s = 0.0f;
-    for (int i = threadIdx.x; i < ntiles; i += 256) s += loss_part[i];
-    __shared__ float red[8];
+// Sums of kColN columns over the rows in order: a warp adds, all fetch ahead.
+__device__ __forceinline__ void column_sums(float *sm, int rows, int N, int c0, const float *__restrict__ a,
+                                            bool scaled, float scale, float *__restrict__ out) {
+  const int nt = (rows + kColRows - 1) / kColRows;
+  auto fetch = [&](int it) {
+    if (it < nt) {
+      float *t = sm + (it % kColStages) * kColRows * kColN;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+      for (int i = 0; i < kColRows * kColN / 4 / 128; ++i) {
+        const int q = threadIdx.x + i * 128, r = q / (kColN / 4), c = q % (kColN / 4) * 4;
+        const bool on = it * kColRows + r < rows && c0 + c < N;
+        cp16(t + r * kColN + c, on ? a + (size_t)(it * kColRows + r) * N + c0 + c : a, on);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < kColStages - 1; ++i) fetch(i);
+  float s = 0.0f;
+  for (int it = 0; it < nt; ++it) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kColStages - 2) : "memory");
     __syncthreads();
-    if (threadIdx.x == 0) {
+    fetch(it + kColStages - 1);
+    if (threadIdx.x < kColN) {
+      const float *t = sm + (it % kColStages) * kColRows * kColN + threadIdx.x;
+      float v[kColRows];
+#pragma unroll
+      for (int u = 0; u < kColRows; ++u) v[u] = t[u * kColN];
+#pragma unroll
+      for (int u = 0; u < kColRows; ++u) s = __fadd_rn(s, scaled ? __fmul_rn(scale, v[u]) : v[u]);  // (+ 0 past the end)
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (threadIdx.x < kColN && c0 + (int)threadIdx.x < N) out[c0 + threadIdx.x] = s;
+}
+
+// All gradients of a training step: weight gradient tiles X^T dZ of every layer
+// first (the longest), then columns of the bias gradients, and the last block
+// the loss, as 256 threads sum the rows' errors: thread i the rows i, i + 256,
+// ..., warps in trees, then in order.
+__global__ void __launch_bounds__(128) all_gradients(GradArgs p) {
+  __shared__ __align__(16) unsigned char smem[kGradBytes];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  if (b == p.first_b[p.layers]) {
+    float *red = reinterpret_cast<float *>(smem);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float s = 0.0f;
+#pragma unroll 4
+      for (int r = tid + 128 * h; r < p.rows; r += 256) s += p.row_sq[r];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((tid & 31) == 0) red[4 * h + (tid >> 5)] = s;
+    }
+    __syncthreads();
+    if (tid == 0) {
       float t = 0.0f;
       for (int w = 0; w < 8; ++w) t += red[w];
-      *loss = t;
+      *p.loss = t;
     }
     return;
   }
-  const long i = (long)blockIdx.x * 256 + threadIdx.x;
-  if (i < nw / 4) {
-    int l = 0;
-    while (l + 1 < p.layers && 4 * i >= p.woff[l + 1]) ++l;
-    const long at = 4 * i - p.woff[l], stride = p.woff[l + 1] - p.woff[l];
-    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 4
-    for (int k = 0; k < p.slices[l]; ++k) {
-      const float4 v = *reinterpret_cast<const float4 *>(p.w[l] + k * stride + at);
-      s.x += v.x;
-      s.y += v.y;
-      s.z += v.z;
-      s.w += v.w;
-    }
-    *reinterpret_cast<float4 *>(grad + 4 * i) = s;
-  } else if (i - nw / 4 < nb) {
-    const long q = i - nw / 4;
-    int l = 0;
-    while (l + 1 < p.layers && q >= p.boff[l + 1]) ++l;
-    const long at = q - p.boff[l], stride = p.boff[l + 1] - p.boff[l];
-    float s = 0.0f;
-#pragma unroll 8
-    for (int k = 0; k < blockrows; ++k) s += p.b[l][k * stride + at];
-    grad[nw + q] = s;
+  int l = 0;
+  if (b >= p.first_b[0]) {
+    while (b >= p.first_b[l + 1]) ++l;
+    column_sums(reinterpret_cast<float *>(smem), p.rows, p.N[l], (b - p.first_b[l]) * kColN, p.dZf[l],
+                l == p.layers - 1, p.scale, p.gb[l]);
+    return;
   }
+  while (b >= p.first_w[l + 1]) ++l;
+  const int K = p.K[l], N = p.N[l], tn = (N + kBN - 1) / kBN, rest = b - p.first_w[l];
+  const int k0 = rest / tn * kGradM, n0 = rest % tn * kBN;
+  float acc[1][4][4];
+  tile_product<1, kGradK, kGradStages, true, false>(reinterpret_cast<bf16 *>(smem), acc, K, N, k0, n0, p.rows, p.X[l], K,
+                                            p.dZ[l], N);
+  float *out = p.gw[l];
+  for_pairs<1>(k0, n0, [&](int r, int c, int i, int j, int h) {
+    if (r < K && c < N)
+      *reinterpret_cast<float2 *>(out + (size_t)r * N + c) = make_float2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
+  });
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master copy; refreshes the BF16 copy
@@ -390,19 +404,8 @@ __global__ void to_bf16(long n, const float *__restrict__ a, bf16 *__restrict__ 
 }
 
 inline int pad16(int x) { return (x + 15) / 16 * 16; }
-inline int tiles(int x) { return (x + kBM - 1) / kBM; }
+inline int tiles(int x, int t) { return (x + t - 1) / t; }
 
-// Slices of the batch rows for a weight gradient of K x N: enough blocks to
-// fill the chip (16 output tiles alone would leave 9 of 10 SMs idle), at
-// least 64 rows each.
-constexpr int kSplitTarget = 148;
-inline int split_rows(int rows, int K, int N, int &chunk) {
-  const int t = tiles(K) * tiles(N);
-  int s = std::min((kSplitTarget + t - 1) / t, std::max(1, rows / 64));
-  chunk = (rows + s - 1) / s;
-  chunk = (chunk + kBK - 1) / kBK * kBK;
-  return (rows + chunk - 1) / chunk;
-}
 inline unsigned blocks(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -474,12 +477,10 @@ void Mlp::get_grads(float *w, float *b) const {
 }
 
 // Workspace for `rows` rows (a multiple of 16): the bf16 input of every layer
-// and, for a training step, the pre-activations, the loss gradients of two
-// adjacent layers and the partial gradients.
+// and, for a training step, the pre-activations, the loss gradients of every
+// layer, the errors and the rows' squared errors.
 cudaError_t Mlp::carve(int rows, bool train, Work &w) {
-  const int L = (int)dims_.size() - 1, br = tiles(rows);
-  int maxd = 0;
-  for (int d : dims_) maxd = std::max(maxd, d);
+  const int L = (int)dims_.size() - 1;
   for (int pass = 0; pass < 2; ++pass) {  // sizes, then pointers
     size_t used = 0;
     auto take = [&](size_t bytes) {
@@ -489,14 +490,9 @@ cudaError_t Mlp::carve(int rows, bool train, Work &w) {
     };
     for (int l = 0; l < L; ++l) w.X[l] = (bf16 *)take((size_t)rows * dims_[l] * sizeof(bf16));
     if (train) {
-      for (int l = 1; l < L; ++l) w.Z[l] = (float *)take((size_t)rows * dims_[l] * sizeof(float));
-      for (auto &d : w.dZ) d = (bf16 *)take((size_t)rows * maxd * sizeof(bf16));
-      for (int l = 0; l < L; ++l) {
-        w.slices[l] = split_rows(rows, dims_[l], dims_[l + 1], w.chunk[l]);
-        w.dW[l] = (float *)take((size_t)w.slices[l] * dims_[l] * dims_[l + 1] * sizeof(float));
-        w.db[l] = (float *)take((size_t)br * dims_[l + 1] * sizeof(float));
-      }
-      w.loss = (float *)take((size_t)br * tiles(dims_[L]) * sizeof(float));
+      for (int l = 1; l <= L; ++l) w.Z[l] = (float *)take((size_t)rows * dims_[l] * sizeof(float));
+      for (int l = 1; l <= L; ++l) w.dZ[l] = (bf16 *)take((size_t)rows * dims_[l] * sizeof(bf16));
+      w.row_sq = (float *)take((size_t)rows * sizeof(float));
     }
     if (pass == 0 && used > ws_bytes_) {
       cudaFree(ws_);
@@ -516,10 +512,10 @@ cudaError_t Mlp::hidden_layers(int n, int rows, const float *x, const Work &w, b
   if (rows > n) cudaMemsetAsync(w.X[0] + (size_t)n * dims_[0], 0, (size_t)(rows - n) * dims_[0] * sizeof(bf16), s);
   input_to_bf16<<<blocks((long)n * dims_[0], 256), 256, 0, s>>>(n, n_in_, dims_[0], x, w.X[0]);
   for (int l = 0; l + 2 < (int)dims_.size(); ++l) {
-    const dim3 grid(tiles(dims_[l + 1]), tiles(rows));
+    const dim3 grid(tiles(dims_[l + 1], kBN), tiles(rows, kBM));
     layer_forward<0><<<grid, 128, 0, s>>>(rows, dims_[l + 1], dims_[l], w.X[l], (const bf16 *)wbf_ + woff_[l],
                                           master_ + nw_ + boff_[l], keep ? w.Z[l + 1] : nullptr, w.X[l + 1], n, 0,
-                                          nullptr, nullptr, nullptr, nullptr);
+                                          nullptr, nullptr);
   }
   return cudaGetLastError();
 }
@@ -529,9 +525,9 @@ cudaError_t Mlp::forward(int n, const float *x, float *y, cudaStream_t s) {
   Work w;
   cudaError_t e = carve(rows, false, w);
   if (e != cudaSuccess || (e = hidden_layers(n, rows, x, w, false, s)) != cudaSuccess) return e;
-  layer_forward<1><<<dim3(tiles(dims_[L]), tiles(rows)), 128, 0, s>>>(
+  layer_forward<1><<<dim3(tiles(dims_[L], kBN), tiles(rows, kBM)), 128, 0, s>>>(
       rows, dims_[L], dims_[L - 1], w.X[L - 1], (const bf16 *)wbf_ + woff_[L - 1], master_ + nw_ + boff_[L - 1],
-      nullptr, nullptr, n, n_out_, nullptr, y, nullptr, nullptr);
+      nullptr, nullptr, n, n_out_, nullptr, y);
   return cudaGetLastError();
 }
 
@@ -540,31 +536,44 @@ cudaError_t Mlp::forward(int n, const float *x, float *y, cudaStream_t s) {
 // *loss_dev (device float).
 cudaError_t Mlp::backward(int n, const float *x, const float *t, float *loss_dev, cudaStream_t s) {
   if (n % 16) return cudaErrorInvalidValue;
-  const int L = (int)dims_.size() - 1, br = tiles(n);
+  const int L = (int)dims_.size() - 1;
   Work w;
   cudaError_t e = carve(n, true, w);
   if (e != cudaSuccess || (e = hidden_layers(n, n, x, w, true, s)) != cudaSuccess) return e;
-  layer_forward<2><<<dim3(tiles(dims_[L]), br), 128, 0, s>>>(
-      n, dims_[L], dims_[L - 1], w.X[L - 1], (const bf16 *)wbf_ + woff_[L - 1], master_ + nw_ + boff_[L - 1],
-      nullptr, w.dZ[(L - 1) & 1], n, n_out_, t, nullptr, w.db[L - 1], w.loss);
-  GradParts p{};
-  p.layers = L;
-  p.woff[L] = nw_;
-  p.boff[L] = nb_;
-  for (int l = L - 1; l >= 0; --l) {
-    const int K = dims_[l], N = dims_[l + 1];
-    const int nw = w.slices[l] * tiles(K) * tiles(N), na = l > 0 ? br * tiles(K) : 0;
-    layer_backward<<<nw + na, 128, 0, s>>>(n, N, K, nw, w.chunk[l], w.X[l], w.dZ[l & 1], w.dW[l],
-                                           (const bf16 *)wbf_ + woff_[l], l > 0 ? w.Z[l] : nullptr, w.dZ[(l & 1) ^ 1],
-                                           l > 0 ? w.db[l - 1] : nullptr);
-    p.slices[l] = w.slices[l];
-    p.woff[l] = woff_[l];
-    p.boff[l] = boff_[l];
-    p.w[l] = w.dW[l];
-    p.b[l] = w.db[l];
+  layer_forward<2><<<dim3(tiles(dims_[L], kBN), tiles(n, kBM)), 128, 0, s>>>(
+      n, dims_[L], dims_[L - 1], w.X[L - 1], (const bf16 *)wbf_ + woff_[L - 1], master_ + nw_ + boff_[L - 1], w.Z[L],
+      w.dZ[L], n, n_out_, t, nullptr);
+  for (int l = L - 1; l > 0; --l) {
+    const int nb = tiles(n, kBM) * tiles(dims_[l], kBN);
+    layer_backward<<<nb + (l == L - 1 ? tiles(n, kErrRows) : 0), 128, 0, s>>>(
+        n, dims_[l + 1], dims_[l], w.dZ[l + 1], (const bf16 *)wbf_ + woff_[l], w.Z[l], w.dZ[l], nb, w.Z[L], dims_[L],
+        n_out_, w.row_sq);
   }
-  sum_parts<<<blocks(nw_ / 4 + nb_, 256) + 1, 256, 0, s>>>(p, br, nw_, nb_, grad_, br * tiles(dims_[L]), w.loss,
-                                                           loss_dev);
+  GradArgs p{};
+  p.layers = L;
+  p.rows = n;
+  p.scale = 2.0f / ((float)n * (float)n_out_);
+  p.row_sq = w.row_sq;
+  p.loss = loss_dev;
+  int block = 0;
+  for (int l = 0; l < L; ++l) {
+    p.K[l] = dims_[l];
+    p.N[l] = dims_[l + 1];
+    p.X[l] = w.X[l];
+    p.dZ[l] = w.dZ[l + 1];
+    p.dZf[l] = w.Z[l + 1];
+    p.gw[l] = grad_ + woff_[l];
+    p.gb[l] = grad_ + nw_ + boff_[l];
+    p.first_w[l] = block;
+    block += tiles(dims_[l], kGradM) * tiles(dims_[l + 1], kBN);
+  }
+  p.first_w[L] = block;
+  for (int l = 0; l < L; ++l) {
+    p.first_b[l] = block;
+    block += tiles(dims_[l + 1], kColN);
+  }
+  p.first_b[L] = block;
+  all_gradients<<<block + 1, 128, 0, s>>>(p);
   return cudaGetLastError();
 }
 

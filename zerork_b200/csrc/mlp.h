@@ -38,9 +38,8 @@ class Mlp {
 
  private:
   struct Work {  // device workspace of one call
-    __nv_bfloat16 *X[kMlpMaxLayers], *dZ[2];
-    float *Z[kMlpMaxLayers], *dW[kMlpMaxLayers], *db[kMlpMaxLayers], *loss;
-    int slices[kMlpMaxLayers], chunk[kMlpMaxLayers];
+    __nv_bfloat16 *X[kMlpMaxLayers], *dZ[kMlpMaxLayers + 1];
+    float *Z[kMlpMaxLayers + 1], *row_sq;  // Z of the output layer: the errors
   };
   cudaError_t carve(int rows, bool train, Work &w);
   cudaError_t hidden_layers(int n, int rows, const float *x, const Work &w, bool keep, cudaStream_t s);
