@@ -146,6 +146,28 @@ def test_edge_sizes_and_clamp(torch, mech_dir):
         _check(pm, ot, T[:n], P[:n], Y[:n], w, j)
 
 
+@pytest.mark.parametrize("name", ["c1_h2", "c2_53"])
+def test_limited_rates_of_trace_species(torch, name, mech_dir):
+    """At 300 K many reverse rate constants are at the step limit.  With their
+    reactants' mass fractions near 1e-163 (two: the product of concentrations
+    underflows, the rate does not) and 1e-110 (three) the temperature column
+    stays finite and the oracle's."""
+    import zerork_b200 as zb
+    from zerork_b200 import mechgen
+    g, (m, t) = synth(name, mech_dir)
+    pm = zb.Mechanism(m, t)
+    tab = pm.tables()
+    rp, rs = tab["reac_ptr"], tab["reac_spc"]
+    T, P, Y = mechgen.rate_states(g, 2 * pm.nstep, seed=29)
+    T[:], P[:] = 300.0, 101325.0
+    for st in range(pm.nstep):
+        for i, y in ((st, 3e-163), (pm.nstep + st, 1e-110)):
+            Y[i, rs[rp[st]:rp[st + 1]]] = y
+    w, j, _ = _run(torch, pm, T, P, Y)
+    assert np.isfinite(w).all() and np.isfinite(j).all()
+    _check(pm, oracle_tables(pm), T, P, Y, w, j)
+
+
 def test_ydot_matches_oracle_rhs(torch, mech_dir):
     import zerork_b200 as zb
     from zerork_b200 import mechgen

@@ -71,6 +71,18 @@ namespace {
 constexpr double kRu = kRuD;
 constexpr double kPatm = kPatmD;
 
+// r over each of a side's concentrations in turn, as r was multiplied: their
+// product alone may underflow where the rate does not.  (Out of line: rare.)
+static __device__ __noinline__ double over_each(double r, const double *y, int stride, int count, int s01, int s23,
+                                                int s45) {
+#pragma unroll 1
+  for (int i = 0; i < count; ++i) {
+    const int s = i < 2 ? s01 : i < 4 ? s23 : s45;
+    r /= y[((i & 1) ? s >> 16 : s & 0xffff) * stride];
+  }
+  return r;
+}
+
 // The rates of progress of one reaction at T become their changes to T' =
 // T + dT at the same concentrations.  A rate constant k n^T exp(-Ta/T) changes
 // by the factor 1 + e, e = expm1(n dlogT - Ta dinvT), an equilibrium constant
@@ -119,7 +131,11 @@ __device__ __forceinline__ bool rop_change(const RxnRec &R, int q, const double 
 #pragma unroll
       for (int k = 0; k < V; ++k)
         if (!(fabs(r[k]) <= fabs(c[k]) * (lim * 1e-11))) {  // w < 1e-11 changes no bit of 1 + e
-          const double w = r[k] / c[k] / lim, we = w * e[k];
+          double x = r[k] / c[k];
+          if (!(fabs(c[k]) >= 1.0e-290))
+            x = over_each(r[k], sC + q + k, TS, count, spc[0] | spc[1] << 16, spc[2] | spc[3] << 16,
+                          spc[4] | spc[5] << 16);
+          const double w = x / lim, we = w * e[k];
           e[k] = e[k] * (1.0 - w) * (1.0 - we * (1.0 - we));
         }
     }
