@@ -4,8 +4,9 @@
 Bounds: the exponential's polynomial is truncated at 4e-18, its argument
 reduction and the last two roundings cost at most one unit in the last place;
 a logarithm's three roundings of its leading parts at most two;
-a quotient corrected by its residual is within one unit, and outside the fast
-range it is the language's division, bit for bit.
+a quotient corrected by its residual is within one unit (of the smallest
+number, when it underflows), and outside the fast range it is the language's
+division, bit for bit.
 """
 import ctypes as C
 import os
@@ -32,6 +33,18 @@ __global__ void k(int n, const double *a, const double *d, double *e, double *q,
   zrk::logs<1>(x, z);
   l[i] = z[0];
 }
+__global__ void k3(int n, const double *a, const double *d, double *q) {
+  const int i = 3 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (i + 2 >= n) return;
+  const double x[3] = {a[i], a[i + 1], a[i + 2]}, y[3] = {d[i], d[i + 1], d[i + 2]};
+  double z[3];
+  zrk::quotients<3>(x, y, z);
+  for (int j = 0; j < 3; ++j) q[i + j] = z[j];
+}
+extern "C" int run3(int n, const double *a, const double *d, double *q) {
+  k3<<<(n / 3 + 255) / 256, 256>>>(n, a, d, q);
+  return (int)cudaDeviceSynchronize();
+}
 extern "C" int run(int n, const double *a, const double *d, double *e, double *q, double *l) {
   k<<<(n + 255) / 256, 256>>>(n, a, d, e, q, l);
   return (int)cudaDeviceSynchronize();
@@ -57,6 +70,12 @@ def probe(tmp_path_factory):
         assert lib.run(len(a), *[C.c_void_p(x.data_ptr()) for x in t]) == 0
         return [x.cpu().numpy() for x in t[2:]]
 
+    def three(a, den):
+        t = [torch.from_numpy(np.ascontiguousarray(x, np.float64)).cuda() for x in (a, den, a)]
+        assert lib.run3(len(a), *[C.c_void_p(x.data_ptr()) for x in t]) == 0
+        return t[2].cpu().numpy()
+
+    run.three = three
     return run
 
 
@@ -92,16 +111,30 @@ def test_logs(probe):
         assert np.allclose(l, np.log(x), rtol=4e-16, atol=0.0, equal_nan=True)
 
 
-def test_quotients(probe):
+@pytest.mark.parametrize("span", [10, 499, 720, 1020])
+def test_quotients(probe, span):
     r = np.random.default_rng(2)
-    a = r.choice([-1.0, 1.0], 200001) * 2.0 ** r.uniform(-700, 700, 200001)
-    d = r.choice([-1.0, 1.0], 200001) * 2.0 ** r.uniform(-700, 700, 200001)
+    a = r.choice([-1.0, 1.0], 200001) * 2.0 ** r.uniform(-span, span, 200001)
+    d = r.choice([-1.0, 1.0], 200001) * 2.0 ** r.uniform(-span, span, 200001)
+    exact = a.astype(np.longdouble) / d.astype(np.longdouble)
     with np.errstate(all="ignore"):
-        d = np.where(np.abs(np.log2(np.abs(a / d))) < 1000, d, np.sign(d))
-    _, q, _ = probe(a, d)
-    assert _ulps(q, a.astype(np.longdouble) / d.astype(np.longdouble)) <= 1.0
+        ref = a / d
+    over = np.isinf(ref)
+    for q in (probe(a, d)[1], probe.three(a, d)):
+        assert np.array_equal(q[over], ref[over])
+        assert np.all(np.abs(q - exact)[~over] <= np.maximum(np.spacing(np.abs(ref[~over])), 5e-324))
+
+
+def test_quotient_ends(probe):
     ends = np.array([0.0, -0.0, 1.0, 5e-324, 1e-310, 1e-250, 1e250, 1.7e308, np.inf, -np.inf, np.nan])
     a, d = (x.ravel() for x in np.meshgrid(ends, ends))
     _, q, _ = probe(a, d)
     with np.errstate(all="ignore"):
         assert np.array_equal(q, a / d, equal_nan=True)
+    # one argument out of range sends all of a group the language's way
+    mixed = np.repeat(np.array([[3.0, 7.0, 1.0]]), len(a), axis=0), np.repeat(np.array([[7.0, 3.0, 1.0]]), len(a), axis=0)
+    for j in range(3):
+        x, y = mixed[0].copy(), mixed[1].copy()
+        x[:, j], y[:, j] = a, d
+        with np.errstate(all="ignore"):
+            assert np.allclose(probe.three(x.ravel(), y.ravel()), (x / y).ravel(), rtol=2.3e-16, atol=0.0, equal_nan=True)

@@ -22,7 +22,7 @@ constexpr double kLnPatmRu = 2.50033668997960945;  // ln(kPatmD / kRuD)
 // way.
 
 // Reciprocal of a mid-range number to some 39 bits: the hardware's approximation
-// and one cubic iteration.  A quotient corrected once by its residual is then
+// (some 13 bits as measured) and one cubic iteration.  A quotient corrected once by its residual is then
 // good to the last place (Markstein, IA-64 and Elementary Functions, 2000).
 __device__ __forceinline__ double recip(double d) {
   double y;
@@ -31,13 +31,15 @@ __device__ __forceinline__ double recip(double d) {
   return fma(y, fma(e, e, e), y);
 }
 __device__ __forceinline__ bool mid_range(double x) {
-  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 300u < 1440u;  // 2^-723 <= |x| < 2^717
+  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 523u < 1000u;  // 2^-500 <= |x| < 2^500
 }
 __device__ __forceinline__ bool not_huge(double x) {
-  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) < 1740u;  // |x| < 2^717, not NaN
+  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) < 1523u;  // |x| < 2^500, not NaN
 }
 
-// q[i] = a[i] / d[i]: the quotient corrected by its residual (Markstein).
+// q[i] = a[i] / d[i]: the quotient corrected by its residual (Markstein).  In
+// the fast range no quotient overflows (its residual would be infinite and the
+// result not a number).
 template <int K>
 __device__ __forceinline__ void quotients(const double (&a)[K], const double (&d)[K], double (&q)[K]) {
   bool ok = true;
