@@ -78,7 +78,9 @@ def test_rates_jac_vs_oracle(torch, name, mech_dir):
     (32, 1, 8, False, False), (32, 2, 4, False, False), (32, 4, 8, False, False),
     (16, 2, 8, True, False), (8, 1, 16, True, False), (32, 4, 1, True, False),
     (16, 2, 16, False, True), (16, 1, 16, False, True), (8, 2, 8, False, True),
-    (16, 2, 8, True, True), (16, 2, 8, False, "two"), (8, 1, 8, False, "two"), (16, 4, 4, True, "two")])
+    (16, 2, 8, True, True), (16, 2, 8, False, "two"), (8, 1, 8, False, "two"), (16, 4, 4, True, "two"),
+    (32, 1, 32, False, False), (16, 1, 32, True, False), (8, 1, 32, False, True), (16, 1, 32, True, True),
+    (16, 2, 16, True, True), (8, 1, 2, True, "two")])
 def test_launch_mappings(torch, ts, v, warps, gws, stage, mech_dir):
     """Every tile/CTA mapping (shared or global workspace, mechanism tables
     staged in shared memory or read from global memory, one or two resident
@@ -96,6 +98,27 @@ def test_launch_mappings(torch, ts, v, warps, gws, stage, mech_dir):
     T, P, Y = mechgen.rate_states(g, 77, seed=3)
     w, j, _ = _run(torch, pm, T, P, Y, ld=80)
     _check(pm, ot, T, P, Y, w, j)
+
+
+def test_launch_flags_are_not_ignored(torch, mech_dir):
+    """Staged tables that cannot be staged are refused: with tiles of 32 states
+    at the call, with tables larger than shared memory when they are asked for,
+    whatever the workspace."""
+    import zerork_b200 as zb
+    from zerork_b200 import mechgen
+    g, (m, t) = synth("c1_h2", mech_dir)
+    pm = zb.Mechanism(m, t)
+    T, P, Y = mechgen.rate_states(g, 40, seed=3)
+    for gws in (False, True):
+        pm.set_launch(32, 1, 8, gws, grid=3 if gws else 0, stage=True)
+        with pytest.raises(zb.ZeroRKError):
+            _run(torch, pm, T, P, Y)
+    pm.set_launch(32, 1, 8)
+    w, j, _ = _run(torch, pm, T, P, Y)
+    _check(pm, oracle_tables(pm), T, P, Y, w, j)
+    _, (m, t) = synth("c3_160", mech_dir)
+    with pytest.raises(zb.ZeroRKError):
+        zb.Mechanism(m, t).set_launch(16, 2, 8, True, grid=7, stage=True)
 
 
 @pytest.mark.parametrize("name", ["c1_h2", "c2_53"])

@@ -32,16 +32,15 @@ size_t rates_jac_ws_bytes(const DevMech &m, const LaunchCfg &cfg) {
 }
 
 bool rates_jac_species_fit(const DevMech &m, const LaunchCfg &cfg) {
-  if (cfg.stage && !cfg.global_ws) return false;  // among the staged tables
+  if (cfg.stage) return false;  // among the staged tables
   const size_t ws = cfg.global_ws ? 0 : rates_jac_ws_bytes(m, cfg);
   // (two resident CTAs share the SM's 228 KB, 1 KB of it the system's for each)
   return ws + m.spc_bytes <= (cfg.minb == 2 ? 113 * 1024 : 227 * 1024);
 }
 
 size_t rates_jac_smem_bytes(const DevMech &m, const LaunchCfg &cfg) {
-  const size_t spc = rates_jac_species_fit(m, cfg) ? m.spc_bytes : 0;
-  if (cfg.global_ws) return spc;
-  return rates_jac_ws_bytes(m, cfg) + (cfg.stage ? (size_t)m.hot_bytes : spc);
+  const size_t tables = cfg.stage ? m.hot_bytes : rates_jac_species_fit(m, cfg) ? m.spc_bytes : 0;
+  return (cfg.global_ws ? 0 : rates_jac_ws_bytes(m, cfg)) + tables;
 }
 
 bool rates_jac_mapping_ok(const LaunchCfg &c) {

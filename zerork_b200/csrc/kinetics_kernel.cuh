@@ -174,9 +174,25 @@ __device__ __forceinline__ void gibbs_from_fits(const double *thermo, const RxnR
   }
 }
 
-template <int TS, int V, bool GLOBAL, int MAXT, bool STAGE, int MINB>
+// The full evaluation at T' out of line, for the kernel of more than 16 warps:
+// inlined beside the rates' own, its 64 registers a thread spilled in both.
+template <int TS>
+__device__ __noinline__ void eval_aside(const DevMech &m, const RxnRec *rec, int q, const double *sC, const double *sG,
+                                        double *sROP, double T, double logT, double invT, double Csum, double lim,
+                                        const char *tab, const double *thermo) {
+  const RxnRec R = load_rxn(rec);
+  const double t[1] = {T}, l[1] = {logT}, i[1] = {invT}, c[1] = {Csum};
+  double gs[1] = {0.0};
+  if (R.flags & kRevKeq) gibbs_from_fits<1>(thermo, R, t, l, gs);
+  reaction_eval<TS, 1, false>(m, R, q, sC, gs, sROP, t, l, i, c, lim, nullptr, tab);
+}
+
+// JAC: with the Jacobian when jac is given; without, never (a kernel of its own
+// for more than 16 warps: 65,536 53-species rates 338 us with 64 registers for
+// both, 268 so).
+template <int TS, int V, bool GLOBAL, int MAXT, bool STAGE, int MINB, bool JAC>
 __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
-    DevMech m, int n, int ld, const double *__restrict__ Tin, const double *__restrict__ Pin,
+    const __grid_constant__ DevMech m, int n, int ld, const double *__restrict__ Tin, const double *__restrict__ Pin,
     const double *__restrict__ Y, double *__restrict__ wdot, double *__restrict__ jac,
     double *__restrict__ ydot, KinParams kp, double *__restrict__ gscratch, int slice_doubles,
     int stage_bytes, int spc_bytes, int part_rows, int vec) {
@@ -196,7 +212,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
   // copy (tab) instead of global memory
   const char *tab = nullptr;
   if constexpr (STAGE) {
-    int4 *dst = reinterpret_cast<int4 *>(smem_dyn + (size_t)L.rows * TS);
+    int4 *dst = reinterpret_cast<int4 *>(smem_dyn + (GLOBAL ? 0 : (size_t)L.rows * TS));
     const int4 *src = reinterpret_cast<const int4 *>(m.base);
     for (int i = threadIdx.x; i < stage_bytes / 16; i += blockDim.x) dst[i] = src[i];
     __syncthreads();
@@ -222,7 +238,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
   // All reactions in snake order (round r gives group g the record at r*NG + g,
   // or at r*NG + NG-1-g for odd r, so that the costliest spread over the groups
   // and every group's total is close to the mean), the next record on its way
-  // to L1 during this one: body(record)
+  // to L1 during this one: body(record, its address)
   auto each_reaction = [&](auto body) {
     const RxnRec *recs = TB(rxn_by_cost);
 #pragma unroll 1
@@ -232,7 +248,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
         const int nx = (r + 1) * NG + ((r & 1) ? g : NG - 1 - g);
         if (nx < m.nrxn) asm volatile("prefetch.global.L1 [%0];" ::"l"(recs + nx));
       }
-      if (at < m.nrxn) body(load_rxn(recs + at));
+      if (at < m.nrxn) body(load_rxn(recs + at), recs + at);
     }
   };
   // the padding row of the Jacobian's records (the g/RT rows are free then)
@@ -317,12 +333,13 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
     int need = 0, npass = 1;
 #pragma unroll 1
     for (int pass = 0; pass < npass; ++pass) {
+      const bool p1 = JAC && pass == 1;
       // temperature of the rates: T' in pass 1
       double Tq[V], lq[V], iq[V];
       FORV {
         Tq[k] = Tr[k];
         lq[k] = logT[k];
-        if (pass == 1) {
+        if (p1) {
           Tq[k] = (yS[k] + yS[k] * kp.sqrt_ur) * kp.Tref;
           if (Tq[k] > 1.0e4) Tq[k] = 1.0e4;
           lq[k] = log(Tq[k]);
@@ -347,7 +364,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
             pc[k] += c[k];
             pcv[k] += ((cp - 1.0) * riw) * y[k];
           }
-          if (pass == 1) {  // the changes of g/RT
+          if (p1) {  // the changes of g/RT
             FORV {
               double cp, h, g0;
               nasa_cp_h_g(th, Tr[k], logT[k], &cp, &h, &g0);
@@ -370,7 +387,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
       }
       if (pass == 0) {
         need = __syncthreads_or(need);
-        if (jac) npass = need ? 3 : 2;
+        if (JAC && jac) npass = need ? 3 : 2;
       } else {
         __syncthreads();
       }
@@ -384,9 +401,9 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
         Csum[k] = cs;
         cv[k] = c2;
       }
-      each_reaction([&](const RxnRec &R) {
+      each_reaction([&](const RxnRec &R, const RxnRec *rec) {
         double f0[V], r0[V];
-        if (pass == 1) {
+        if (p1) {
           double dl[V], di[V];
           FORV {
             const double z = (Tq[k] - Tr[k]) / Tr[k];  // sqrt(eps), or 0 beyond the temperature clamp
@@ -397,11 +414,16 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
           ldv<V>(sROP + R.fwd * TS + q, f0);
           if (R.rev >= 0) ldv<V>(sROP + R.rev * TS + q, r0);
         }
-        double gs[V];
-        if (pass == 1 && (R.flags & kRevKeq)) gibbs_from_fits<V>(SB(thermo), R, Tq, lq, gs);
-        else gibbs_from_rows<TS, V, false>(R, q, sG, gs);
-        reaction_eval<TS, V, false>(m, R, q, sC, gs, sROP, Tq, lq, iq, Csum, kp.lim, nullptr, tab);
-        if (pass == 1) {
+        if (MAXT > 512 && p1) {
+          if constexpr (MAXT > 512)
+            eval_aside<TS>(m, rec, q, sC, sG, sROP, Tq[0], lq[0], iq[0], Csum[0], kp.lim, tab, SB(thermo));
+        } else {
+          double gs[V];
+          if (p1 && (R.flags & kRevKeq)) gibbs_from_fits<V>(SB(thermo), R, Tq, lq, gs);
+          else gibbs_from_rows<TS, V, false>(R, q, sG, gs);
+          reaction_eval<TS, V, false>(m, R, q, sC, gs, sROP, Tq, lq, iq, Csum, kp.lim, nullptr, tab);
+        }
+        if (p1) {
           double x[V];
           ldv<V>(sROP + R.fwd * TS + q, x);
           FORV x[k] -= f0[k];
@@ -446,7 +468,7 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
               }
           }
           const double mws = SB(mw)[s];
-          if (pass == 1) {
+          if (p1) {
             const double *th = SB(thermo) + 16 * s, *wd = wdot + (size_t)s * ld + st0;
             FORV {
               const double mult = 1.0 / ((yS[k] + yS[k] * kp.sqrt_ur) - yS[k]);
@@ -471,25 +493,25 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
         }
         FORV pe[k] = warp_group_sum<GS>(pe[k]);
         if (wlead) FORV PT(0, w, k) = pe[k];
-        if (pass != 1) zero_row();
+        if (!p1) zero_row();
       }
       __syncthreads();
       double tdq[V];
       FORV {
         double es = 0.0;
         for (int ww = 0; ww < NW; ++ww) es += PT(0, ww, k);
-        const double ys = pass == 1 ? yS[k] + yS[k] * kp.sqrt_ur : yS[k];
+        const double ys = p1 ? yS[k] + yS[k] * kp.sqrt_ur : yS[k];
         tdq[k] = -es * kRu * ys / cv[k] + 0.0;
         if (pass == 0) td[k] = tdq[k];
       }
       if (g == 0 && pass == 0 && ydot) put(ydot + (size_t)S * ld, tdq);
-      if (g == 0 && pass == 1) {
+      if (g == 0 && p1) {
         double d[V];
         FORV d[k] = (tdq[k] - td[k]) * (1.0 / ((yS[k] + yS[k] * kp.sqrt_ur) - yS[k]));
         put(jac + (size_t)(TB(col_ptr)[S] + S) * ld, d);
       }
       __syncthreads();  // the energy partials are read before their rows are reused
-      if (jac == nullptr || pass == 1 || (pass == 0 && need)) continue;
+      if (!JAC || jac == nullptr || p1 || (pass == 0 && need)) continue;
       // ---- analytic Jacobian: the species-column entries (the flat item list of
       // devmech.h) in equal work shares over the groups, the temperature row of
       // each column from per-(group, column) partial sums kept in the g/RT and
@@ -647,7 +669,8 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
 template <int TS, int V, bool GLOBAL, int MAXT, bool STAGE, int MINB>
 cudaError_t launch_one(const DevMech &m, const RatesJacArgs &a, const KinParams &kp,
                        const LaunchCfg &cfg, cudaStream_t stream) {
-  auto *kern = rates_jac_kernel<TS, V, GLOBAL, MAXT, STAGE, MINB>;
+  auto *kern = MAXT > 512 && !a.jac ? rates_jac_kernel<TS, V, GLOBAL, MAXT, STAGE, MINB, (MAXT <= 512)>
+                                    : rates_jac_kernel<TS, V, GLOBAL, MAXT, STAGE, MINB, true>;
   const int threads = std::min(cfg.warps * 32, MAXT);
   const int ntiles = (a.n + TS - 1) / TS;
   if (ntiles == 0) return cudaSuccess;
@@ -656,25 +679,29 @@ cudaError_t launch_one(const DevMech &m, const RatesJacArgs &a, const KinParams 
   if (smem > 227 * 1024) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  // the smallest shared-memory carve-out that holds the workspace (and the
-  // staged tables), so the rest of the SM's 256 KB stays L1
-  const int pct = (int)((100 * MINB * (smem + 1024) + 228 * 1024 - 1) / (228 * 1024));
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct < 100 ? pct : 100);
-  if (e != cudaSuccess) return e;
-  int grid = ntiles;
+  int dev = 0, sms = 148, per_sm = 1, grid = ntiles;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (GLOBAL) {
     if (cfg.grid > 0) grid = std::min(cfg.grid, ntiles);
     if ((size_t)grid * slice > a.scratch_bytes) return cudaErrorInvalidValue;
-  } else {
+  }
+  // The smallest shared-memory carve-out that holds the workspace (and the
+  // tables beside it), so the rest of the SM's 256 KB stays L1.  With more CTAs
+  // than SMs: of CTAs of fewer than 8 warps as many as make 8 (ten species,
+  // 65,536 states, 8-state tiles by 4 warps: 990 us with one CTA's share, 522
+  // with two), and of those with a global workspace, which have the species
+  // tables only, as many as registers allow.
+  int ctas = MINB;
+  if (grid > sms) ctas = std::max(ctas, (GLOBAL && !STAGE ? 16 : 8) * 32 / threads);
+  const int pct = (int)((100 * ctas * (smem + 1024) + 228 * 1024 - 1) / (228 * 1024));
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct < 100 ? pct : 100);
+  if (e != cudaSuccess) return e;
+  if (!GLOBAL && ntiles > sms) {
     // persistent CTAs: one copy of the staged tables each, and the next
     // tile's inputs are fetched ahead
-    int dev = 0, sms = 148, per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (ntiles > sms) {
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
-      grid = std::min(ntiles, sms * std::max(1, per_sm));
-    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+    grid = std::min(ntiles, sms * std::max(1, per_sm));
   }
   const auto al16 = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
   const int vec = V > 1 && a.ld % 2 == 0 && al16(a.Y) && al16(a.wdot) && al16(a.jac) && al16(a.ydot);
@@ -686,26 +713,49 @@ cudaError_t launch_one(const DevMech &m, const RatesJacArgs &a, const KinParams 
 
 }  // namespace
 
+// More CTAs than SMs in a launch with a global workspace.
+inline bool many_ctas(const RatesJacArgs &a, const LaunchCfg &cfg) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int ntiles = (a.n + cfg.ts - 1) / cfg.ts;
+  return (cfg.grid > 0 ? std::min(cfg.grid, ntiles) : ntiles) > sms;
+}
+
 // The kernels of one tile size (one translation unit each, to compile side by
-// side).  Up to 16 warps may use 128 registers a thread, 32 warps (one state
-// per thread only) 64; two resident CTAs of up to 8 warps 128.  Staged tables
-// and two resident CTAs only with tiles of at most 16 states in shared memory
+// side).  Up to 8 warps may use 255 registers a thread (128 of them, two CTAs
+// resident, on request), up to 16 warps 128, 32 warps (one state per thread
+// only) 64: the more warps hide latency, the fewer registers hold values in
+// flight.  8 warps with 128 registers instead: 32,768 53-species states, 32-state
+// tiles, two states a thread 939 -> 1,005 us, four 911 -> 1,125.  With a global
+// workspace and more CTAs than SMs, 128: several are resident then (ten species,
+// 65,536 states, 16-state tiles 779 -> 533 us; 53 species 1,152 -> 1,306).
+// Staged tables and two resident CTAs only with tiles of at most 16 states
 // (larger tiles leave no room).
+template <int TS, int V, bool GLOBAL>
+cudaError_t launch_tvg(const DevMech &m, const RatesJacArgs &a, const KinParams &kp, const LaunchCfg &cfg,
+                       cudaStream_t stream) {
+  if constexpr (TS <= 16) {
+    if (cfg.stage) {
+      if (cfg.warps <= 8) return launch_one<TS, V, GLOBAL, 256, true, 1>(m, a, kp, cfg, stream);
+      if (cfg.warps <= 16) return launch_one<TS, V, GLOBAL, 512, true, 1>(m, a, kp, cfg, stream);
+      if constexpr (V == 1) return launch_one<TS, V, GLOBAL, 1024, true, 1>(m, a, kp, cfg, stream);
+      return cudaErrorInvalidValue;
+    }
+    if (cfg.minb == 2) return launch_one<TS, V, GLOBAL, 256, false, 2>(m, a, kp, cfg, stream);
+  }
+  if (cfg.stage || cfg.minb != 1) return cudaErrorInvalidValue;
+  if (cfg.warps <= (GLOBAL && many_ctas(a, cfg) ? 0 : 8)) return launch_one<TS, V, GLOBAL, 256, false, 1>(m, a, kp, cfg, stream);
+  if (cfg.warps <= 16) return launch_one<TS, V, GLOBAL, 512, false, 1>(m, a, kp, cfg, stream);
+  if constexpr (V == 1) return launch_one<TS, V, GLOBAL, 1024, false, 1>(m, a, kp, cfg, stream);
+  return cudaErrorInvalidValue;
+}
+
 template <int TS, int V>
 cudaError_t launch_tv(const DevMech &m, const RatesJacArgs &a, const KinParams &kp, const LaunchCfg &cfg,
                       cudaStream_t stream) {
-  if (cfg.global_ws) {
-    if (cfg.warps <= 16) return launch_one<TS, V, true, 512, false, 1>(m, a, kp, cfg, stream);
-    if constexpr (V == 1) return launch_one<TS, V, true, 1024, false, 1>(m, a, kp, cfg, stream);
-    return cudaErrorInvalidValue;
-  }
-  if constexpr (TS <= 16) {
-    if (cfg.stage && cfg.warps <= 16) return launch_one<TS, V, false, 512, true, 1>(m, a, kp, cfg, stream);
-    if (cfg.minb == 2 && !cfg.stage) return launch_one<TS, V, false, 256, false, 2>(m, a, kp, cfg, stream);
-  }
-  if (cfg.warps <= 16) return launch_one<TS, V, false, 512, false, 1>(m, a, kp, cfg, stream);
-  if constexpr (V == 1) return launch_one<TS, V, false, 1024, false, 1>(m, a, kp, cfg, stream);
-  return cudaErrorInvalidValue;
+  return cfg.global_ws ? launch_tvg<TS, V, true>(m, a, kp, cfg, stream)
+                       : launch_tvg<TS, V, false>(m, a, kp, cfg, stream);
 }
 
 template <int TS>
