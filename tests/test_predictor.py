@@ -192,6 +192,28 @@ def test_gpu_weight_gradient_is_one_chain(torch):
 
 
 @pytest.mark.gpu
+def test_gpu_capture_after_an_evaluation(torch):
+    """An evaluation leaves the workspace that gradients of as many rows need,
+    so they can be captured in a CUDA graph, where nothing can be allocated."""
+    from zerork_b200.predictor import Mlp
+    rng = np.random.default_rng(8)
+    nets = [Mlp(56, 54, 64, 2, seed=3) for _ in range(2)]
+    x = torch.from_numpy(rng.standard_normal((320, 56)).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.standard_normal((320, 54)).astype(np.float32)).cuda()
+    loss = torch.zeros(2, dtype=torch.float32, device="cuda")
+    Mlp(56, 54, 64, 2, seed=3).gradients(x, t, loss[:1])  # loads the kernels
+    nets[0].forward(x)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        nets[0].gradients(x, t, loss[:1], stream=torch.cuda.current_stream().cuda_stream)
+    g.replay()
+    torch.cuda.synchronize()
+    nets[1].gradients(x, t, loss[1:])
+    assert np.array_equal(nets[0].grads()[0], nets[1].grads()[0]) and loss[0].item() == loss[1].item()
+
+
+@pytest.mark.gpu
 def test_gpu_training_reduces_loss(torch):
     from zerork_b200.predictor import train
     rng = np.random.default_rng(4)

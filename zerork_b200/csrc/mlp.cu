@@ -477,9 +477,11 @@ void Mlp::get_grads(float *w, float *b) const {
 }
 
 // Workspace for `rows` rows (a multiple of 16): the bf16 input of every layer
-// and, for a training step, the pre-activations, the loss gradients of every
-// layer, the errors and the rows' squared errors.
-cudaError_t Mlp::carve(int rows, bool train, Work &w) {
+// and a training step's pre-activations, loss gradients of every layer, errors
+// and rows' squared errors.  (All of it for an evaluation too: any call of the
+// same size then finds its workspace, also one being captured, where nothing
+// can be allocated.)
+cudaError_t Mlp::carve(int rows, Work &w) {
   const int L = (int)dims_.size() - 1;
   for (int pass = 0; pass < 2; ++pass) {  // sizes, then pointers
     size_t used = 0;
@@ -489,11 +491,9 @@ cudaError_t Mlp::carve(int rows, bool train, Work &w) {
       return q;
     };
     for (int l = 0; l < L; ++l) w.X[l] = (bf16 *)take((size_t)rows * dims_[l] * sizeof(bf16));
-    if (train) {
-      for (int l = 1; l <= L; ++l) w.Z[l] = (float *)take((size_t)rows * dims_[l] * sizeof(float));
-      for (int l = 1; l <= L; ++l) w.dZ[l] = (bf16 *)take((size_t)rows * dims_[l] * sizeof(bf16));
-      w.row_sq = (float *)take((size_t)rows * sizeof(float));
-    }
+    for (int l = 1; l <= L; ++l) w.Z[l] = (float *)take((size_t)rows * dims_[l] * sizeof(float));
+    for (int l = 1; l <= L; ++l) w.dZ[l] = (bf16 *)take((size_t)rows * dims_[l] * sizeof(bf16));
+    w.row_sq = (float *)take((size_t)rows * sizeof(float));
     if (pass == 0 && used > ws_bytes_) {
       cudaFree(ws_);
       ws_ = nullptr;
@@ -523,7 +523,7 @@ cudaError_t Mlp::hidden_layers(int n, int rows, const float *x, const Work &w, b
 cudaError_t Mlp::forward(int n, const float *x, float *y, cudaStream_t s) {
   const int rows = pad16(std::max(n, 1)), L = (int)dims_.size() - 1;
   Work w;
-  cudaError_t e = carve(rows, false, w);
+  cudaError_t e = carve(rows, w);
   if (e != cudaSuccess || (e = hidden_layers(n, rows, x, w, false, s)) != cudaSuccess) return e;
   layer_forward<1><<<dim3(tiles(dims_[L], kBN), tiles(rows, kBM)), 128, 0, s>>>(
       rows, dims_[L], dims_[L - 1], w.X[L - 1], (const bf16 *)wbf_ + woff_[L - 1], master_ + nw_ + boff_[L - 1],
@@ -538,7 +538,7 @@ cudaError_t Mlp::backward(int n, const float *x, const float *t, float *loss_dev
   if (n % 16) return cudaErrorInvalidValue;
   const int L = (int)dims_.size() - 1;
   Work w;
-  cudaError_t e = carve(n, true, w);
+  cudaError_t e = carve(n, w);
   if (e != cudaSuccess || (e = hidden_layers(n, n, x, w, true, s)) != cudaSuccess) return e;
   layer_forward<2><<<dim3(tiles(dims_[L], kBN), tiles(n, kBM)), 128, 0, s>>>(
       n, dims_[L], dims_[L - 1], w.X[L - 1], (const bf16 *)wbf_ + woff_[L - 1], master_ + nw_ + boff_[L - 1], w.Z[L],

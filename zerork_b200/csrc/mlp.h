@@ -41,7 +41,7 @@ class Mlp {
     __nv_bfloat16 *X[kMlpMaxLayers], *dZ[kMlpMaxLayers + 1];
     float *Z[kMlpMaxLayers + 1], *row_sq;  // Z of the output layer: the errors
   };
-  cudaError_t carve(int rows, bool train, Work &w);
+  cudaError_t carve(int rows, Work &w);
   cudaError_t hidden_layers(int n, int rows, const float *x, const Work &w, bool keep, cudaStream_t s);
   int n_in_, n_out_;
   std::vector<int> dims_;
