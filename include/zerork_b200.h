@@ -200,10 +200,10 @@ int zrk_plugin_num_species(struct zerork_handle_impl *h);
 int zrk_plugin_graph_stats(struct zerork_handle_impl *h, long *captures, long *launches);
 
 /* Integrator launch-mapping autotuner: times the dense path's CTA sizes
- * (128/256/512 threads) or the sparse path's warps per CTA (4/8/12) on a
- * sample of the given reactors (at most 2 per SM) over dt / 20, keeps the
- * fastest as the handle's gpu_threads / gpu_warps_per_cta option and
- * returns it with its kernel time.  The inputs are not modified.  No
+ * (automatic and 128/256/512 threads) or the sparse path's warps per CTA
+ * (4/8/12) on a sample of the given reactors (at most 8 per SM) over dt / 20,
+ * keeps the fastest as the handle's gpu_threads / gpu_warps_per_cta option
+ * (0: automatic) and returns it with its kernel time.  The inputs are not modified.  No
  * counterpart in the reference (its GPU path has fixed launch sizes). */
 int zrk_plugin_autotune(struct zerork_handle_impl *h, int n, double dt, const double *T,
                         const double *P, const double *mass_fractions, int *best, float *best_ms);

@@ -431,3 +431,40 @@ def test_integrator_autotune(gpu, mech_dir):
     assert p.get_int("gpu_threads") == best
     assert np.array_equal(T, T0) and np.array_equal(Y, Y0)
     assert p.solve(1e-3, T, P, Y) == 0
+
+
+@pytest.mark.parametrize("name,n,dt", [("c1_h2", 1000, 1e-3), ("c1_h2", 64, 1e-3), ("dme", 600, 1e-5)])
+def test_autotune_is_not_slower_than_automatic(gpu, mech_dir, name, n, dt):
+    """The tuned CTA size against the automatic one on the reactors it was tuned
+    on, over the interval it was timed over: within a tenth (timings on one GPU
+    repeat to a few percent)."""
+    import zerork_b200 as zb
+    from plugin_cases import mech_path
+    from zerork_b200 import mechgen
+    from zerork_b200.plugin import Plugin
+    if name == "dme":
+        mf, tf = mech_path("dme_24_mech.txt"), mech_path("dme_24_therm.txt")
+        pm = zb.Mechanism(mf, tf, device=False)
+        r = np.random.default_rng(4)
+        sp = [s.lower() for s in pm.species]
+        T, P = r.uniform(700.0, 1500.0, n), 101325.0 * r.uniform(1.0, 50.0, n)
+        Y = np.zeros((n, pm.nsp))
+        Y[:, sp.index("ch3och3")] = r.uniform(0.3, 2.0, n)
+        Y[:, sp.index("o2")], Y[:, sp.index("n2")] = 3.0, 3.0 * 3.76
+        Y *= pm.table("mw")
+        Y /= Y.sum(1, keepdims=True)
+    else:
+        g, (mf, tf) = synth(name, mech_dir)
+        T, P, Y = mechgen.reactor_states(g, n, "c1", seed=6)
+    tuned, plain = Plugin(mf, tf, max_steps=20000), Plugin(mf, tf, max_steps=20000)
+    best, _ = tuned.autotune(dt, T, P, Y)
+    assert tuned.get_int("gpu_threads") == best and best in (0, 128, 256, 512)
+    ms = []
+    for p in (tuned, plain):
+        t = []
+        for _ in range(3):
+            Tg, Pg, Yg = T.copy(), P.copy(), np.ascontiguousarray(Y.copy())
+            p.solve(dt / 20.0, Tg, Pg, Yg, raise_on_fail=False)
+            t.append(p.last_stats()["kernel_ms"])
+        ms.append(min(t))
+    assert ms[0] <= 1.1 * ms[1], (best, ms)

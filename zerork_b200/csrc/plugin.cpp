@@ -388,9 +388,13 @@ int zrk_plugin_graph_stats(zerork_handle h, long *captures, long *launches) {
 }
 
 // Integrator launch-mapping autotuner: the CTA size of the dense-block path
-// (128, 256, 512 threads) or the warps per CTA of the sparse path (4, 8, 12),
-// each timed on the same sample of the caller's reactors over a short
-// interval; the fastest becomes the handle's gpu_threads / gpu_warps_per_cta.
+// (automatic, 128, 256, 512 threads) or the warps per CTA of the sparse path
+// (4, 8, 12), each timed on the same sample of the caller's reactors over a
+// short interval; the fastest becomes the handle's gpu_threads /
+// gpu_warps_per_cta.  The automatic size (dense_threads in solver.cpp) depends
+// on the number of reactors and on more sizes than the fixed ones; it stays when
+// it beats them by more than the timings' noise.  Its rule turns at four
+// reactors an SM, so the sample goes beyond that.
 int zrk_plugin_autotune(zerork_handle h, int n, double dt, const double *T, const double *P,
                         const double *mf, int *best, float *best_ms) {
   if (!h) return ZRK_ERR_INVALID_HANDLE;
@@ -401,7 +405,7 @@ int zrk_plugin_autotune(zerork_handle h, int n, double dt, const double *T, cons
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int ns = h->solver->nsp();
-  const int m = std::min(n, 2 * sms);
+  const int m = std::min(n, 8 * sms);
   const double dtt = dt / 20.0;
   zrk::SolveOptions o = options_of(h);
   int method = o.method;
@@ -412,8 +416,8 @@ int zrk_plugin_autotune(zerork_handle h, int n, double dt, const double *T, cons
                        nullptr, &tot) < 0)
     return ZRK_ERR_CUDA;
   method = tot.method;
-  const std::vector<int> cand = method == 1 ? std::vector<int>{128, 256, 512} : std::vector<int>{4, 8, 12};
-  float bms = 1e30f;
+  const std::vector<int> cand = method == 1 ? std::vector<int>{0, 128, 256, 512} : std::vector<int>{4, 8, 12};
+  float bms = 1e30f, auto_ms = 1e30f;
   int bc = cand.back();
   for (int c : cand) {
     zrk::SolveOptions oc = o;
@@ -425,10 +429,16 @@ int zrk_plugin_autotune(zerork_handle h, int n, double dt, const double *T, cons
     if (h->solver->solve(oc, m, dtt, T1.data(), P1.data(), Y1.data(), ns, nullptr, nullptr, nullptr, 2.0,
                          nullptr, &tot) < 0)
       continue;
-    if (tot.kernel_ms < bms) {
+    if (c == 0) {
+      auto_ms = tot.kernel_ms;
+    } else if (tot.kernel_ms < bms) {
       bms = tot.kernel_ms;
       bc = c;
     }
+  }
+  if (auto_ms < 0.98f * bms) {
+    bms = auto_ms;
+    bc = 0;
   }
   h->iopt[method == 1 ? "gpu_threads" : "gpu_warps_per_cta"] = bc;
   if (best) *best = bc;
