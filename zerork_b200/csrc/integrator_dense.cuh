@@ -634,6 +634,9 @@ __device__ __noinline__ int invert_cta(const DevMech &m, const Smem &s, const do
   return __syncthreads_or(perm[n]);
 }
 
+// Columns of a panel for nc chunks of 32 unknowns.
+__host__ __device__ constexpr int panel_width(bool f64, int nc) { return !f64 || nc <= 4 ? 8 : nc <= 6 ? 6 : 4; }
+
 // invert_cta for the register-chunk count nc = ceil(n / 32) (1..8).
 template <class LT, bool SH>
 __device__ __forceinline__ int invert_any(int nc, const DevMech &m, const Smem &s, const double *J,
@@ -645,8 +648,8 @@ __device__ __forceinline__ int invert_any(int nc, const DevMech &m, const Smem &
     case 3: return invert_cta<LT, 3, 8, SH>(m, s, J, c, n, lda);
     case 4: return invert_cta<LT, 4, 8, SH>(m, s, J, c, n, lda);
     case 5:
-    case 6: return invert_cta<LT, 6, F64 ? 6 : 8, SH>(m, s, J, c, n, lda);
-    default: return invert_cta<LT, 8, F64 ? 4 : 8, SH>(m, s, J, c, n, lda);
+    case 6: return invert_cta<LT, 6, panel_width(F64, 6), SH>(m, s, J, c, n, lda);
+    default: return invert_cta<LT, 8, panel_width(F64, 8), SH>(m, s, J, c, n, lda);
   }
 }
 

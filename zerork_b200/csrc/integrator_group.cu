@@ -54,7 +54,7 @@ struct GroupKArgs {
   double *slots;     // one slot of slot_stride doubles per group position
   long slot_stride;
   int lda;
-  int ws_doubles;    // shared memory of the reduction slots and the rates workspace
+  int matrix_at;     // where in shared memory (doubles) a factorization keeps its matrix
   double *part;      // [n_group][kPart]
   const double *T, *P, *Y, *ysrc, *dpdt, *tdel_in;
 };
@@ -75,12 +75,12 @@ __device__ Bound bind(const GroupKArgs &k, double *smem) {
   double *p = smem;
   Smem &s = b.s;
   s.red = p; p += 128;
-  s.rows = p;  // the inversion's pivot rows over the rates workspace
+  s.rows = p;  // the inversion's pivot rows over the rates workspace (group_smem)
   s.C = p; p += S;
   s.G = p; p += S;
   s.U = p; p += S;
   s.ROP = p; p += m.nstep;
-  s.part = p; p += net_slots(S);
+  s.part = p;
   s.mlp = nullptr;
   s.Jsm = nullptr;
   s.V = nullptr;
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(512) grp_start(GroupKArgs k, double t_off, dou
   }
   __syncthreads();
   int bad = jac_cta(k.m, k.o, s, b.hdr[0], t_off, s.y, s.f0, b.J);
-  if (!bad) bad = factor_g(k, b, c, fac_smem ? smem + k.ws_doubles : nullptr);
+  if (!bad) bad = factor_g(k, b, c, fac_smem ? smem + k.matrix_at : nullptr);
   put_part(k, 4, bad ? 1.0 : 0.0);
 }
 
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(512) grp_factor(GroupKArgs k, double t_abs, do
     bad = rhs_cta(k.m, k.o, s, b.hdr[0], t_abs, s.ypred, s.f0, false, nullptr);
     if (!bad) bad = jac_cta(k.m, k.o, s, b.hdr[0], t_abs, s.ypred, s.f0, b.J);
   }
-  if (!bad) bad = factor_g(k, b, c, fac_smem ? smem + k.ws_doubles : nullptr);
+  if (!bad) bad = factor_g(k, b, c, fac_smem ? smem + k.matrix_at : nullptr);
   put_part(k, 4, bad ? 1.0 : 0.0);
 }
 
@@ -667,14 +667,14 @@ cudaError_t integrate_group(const DevMech &m, const IntegOpts &o, const IntegArg
   drv.st = stream;
   drv.part_h = part_host;
   make_consts(drv.bc);
-  // reduction slots, then the rates workspace or the inversion's pivot rows
-  const size_t ws = std::max(3 * (size_t)S + m.nstep + net_slots(S), (size_t)kPanelMax * n);
-  drv.k.ws_doubles = (int)(128 + ws);
-  drv.smem = (128 + ws) * sizeof(double);
   const size_t kSmemMax = 227 * 1024;
-  drv.smem_fac = drv.smem + (size_t)n * lda * sizeof(double);
-  drv.fac_smem = drv.smem_fac <= kSmemMax ? 1 : 0;
-  if (!drv.fac_smem) drv.smem_fac = drv.smem;
+  const GroupSmem g = group_smem(S, m.nstep, m.net_chunks > 0 ? net_slots(S) : 0,
+                                 (size_t)panel_width(true, (n + 31) / 32) * n, (size_t)n * lda, kSmemMax / sizeof(double));
+  if (!g.chunks) drv.k.m.net_chunks = 0;
+  drv.k.matrix_at = (int)g.matrix_at;
+  drv.smem = g.eval * sizeof(double);
+  drv.smem_fac = g.fac * sizeof(double);
+  drv.fac_smem = g.fac_smem ? 1 : 0;
   if (drv.smem > kSmemMax) return cudaErrorInvalidValue;
   cudaError_t e;
   // every kernel may use up to smem_fac of dynamic shared memory

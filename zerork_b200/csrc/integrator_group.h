@@ -16,6 +16,30 @@ struct GroupCounters {
   long first_fail = 0;  // status of the first group whose attempts all failed
 };
 
+// Dynamic shared memory of the group kernels, in doubles: 128 reduction slots,
+// then the rates workspace of 3 nsp + nstep doubles and the net rates' partial
+// sums (part doubles).  A factorization has its pivot rows (rows doubles) over
+// the rates and, when it fits in `limit`, the matrix of `matrix` doubles behind
+// the larger of the two, over the partial sums, which are dead by then.  A
+// mechanism whose partial sums do not fit sums its net rates without them.
+struct GroupSmem {
+  size_t matrix_at, eval, fac;  // offset of the matrix; sizes without and with it
+  bool chunks, fac_smem;        // partial sums used; matrix in shared memory
+};
+inline GroupSmem group_smem(size_t nsp, size_t nstep, size_t part, size_t rows, size_t matrix, size_t limit) {
+  const size_t ws = 3 * nsp + nstep;
+  GroupSmem g;
+  g.matrix_at = 128 + (ws > rows ? ws : rows);
+  g.chunks = part > 0 && 128 + ws + part <= limit;
+  g.eval = 128 + ws + (g.chunks ? part : 0);
+  if (g.eval < g.matrix_at) g.eval = g.matrix_at;
+  g.fac = g.matrix_at + matrix;
+  if (g.fac < g.eval) g.fac = g.eval;
+  g.fac_smem = g.fac <= limit;
+  if (!g.fac_smem) g.fac = g.eval;
+  return g;
+}
+
 // Doubles of device workspace per reactor of a group (the reactor's BDF
 // vectors, history, Jacobian and Newton-matrix inverse).
 size_t group_slot_doubles(const DevMech &m);
