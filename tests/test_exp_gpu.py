@@ -1,5 +1,6 @@
 """The kernels' interleaved exponentials, logarithms and quotients
-(zerork_b200/csrc/kinetics_dev.cuh) against extended precision.
+(zerork_b200/csrc/kinetics_dev.cuh) and the series of a rate's change with
+temperature (kinetics_kernel.cuh) against extended precision.
 
 Bounds: the exponential's polynomial is truncated at 4e-18, its argument
 reduction and the last two roundings cost at most one unit in the last place;
@@ -138,3 +139,47 @@ def test_quotient_ends(probe):
         x[:, j], y[:, j] = a, d
         with np.errstate(all="ignore"):
             assert np.allclose(probe.three(x.ravel(), y.ravel()), (x / y).ravel(), rtol=2.3e-16, atol=0.0, equal_nan=True)
+
+
+CHANGE = r"""
+#include "kinetics_kernel.cuh"
+__global__ void k(int n, const double *x, const double *w, double *out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  zrk::RxnRec R = {};
+  R.n = 1.0;  // the exponent is dlogT
+  R.rev = -1;
+  R.nr = 1;
+  const double c[1] = {1.0}, dl[1] = {x[i]}, di[1] = {0.0};
+  double rop[1] = {w[i]};  // the limited constant over a limit of 1
+  out[i] = zrk::rop_change<1, 1>(R, 0, c, c, rop, dl, di, w[i] > 0.0 ? 1.0 : 0.0) ? rop[0] : -1.0;
+}
+extern "C" int run(int n, const double *x, const double *w, double *out) {
+  k<<<(n + 255) / 256, 256>>>(n, x, w, out);
+  return (int)cudaDeviceSynchronize();
+}
+"""
+
+
+@pytest.mark.parametrize("w", [1e-9, 0.1, 0.5, 0.9, 0.999])
+def test_rate_change(tmp_path, w):
+    """e (1 - w) / (1 + w e) w, e = expm1(x), over all |x| that the series take
+    (below 1e-4; beyond, the rate is left alone).  Truncation 1e-16 and six
+    roundings."""
+    if not have_gpu():
+        pytest.skip("no CUDA device")
+    import torch
+    from zerork_b200 import build
+    src, so = str(tmp_path / "change.cu"), str(tmp_path / "change.so")
+    with open(src, "w") as f:
+        f.write(CHANGE)
+    subprocess.run([build.nvcc(), "-shared", "-o", so, src] + build._flags(src), check=True)
+    x = np.concatenate([np.linspace(-0.999e-4, 0.999e-4, 2000), 10.0 ** np.linspace(-12, -4.01, 500), [1.001e-4, -2e-4]])
+    t = [torch.from_numpy(a).cuda() for a in (x, np.full_like(x, w), np.zeros_like(x))]
+    assert C.CDLL(so).run(len(x), *[C.c_void_p(a.data_ptr()) for a in t]) == 0
+    got = t[2].cpu().numpy()
+    assert np.all(got[-2:] == -1.0)
+    X, W = x[:-2].astype(np.longdouble), np.longdouble(w)
+    e = np.expm1(X)
+    exact = e * (1 - W) / (1 + W * e) * W
+    assert np.max(np.abs(got[:-2] / exact - 1)) <= 1e-16 + 6 * 2.0 ** -53

@@ -88,10 +88,11 @@ static __device__ __noinline__ double over_each(double r, const double *y, int s
 // by the factor 1 + e, e = expm1(n dlogT - Ta dinvT), an equilibrium constant
 // by that of its g/RT changes (dG rows); the step limiter's k L / (k + L)
 // makes it e (1 - w) / (1 + w e) with w = k / (k + L), the limited constant
-// over L.  |e| is a few 1e-6 (the step is sqrt(eps) T), so three terms of each
-// series are exact to rounding.  Falloff and PLOG rates, and exponents beyond
-// that (|e| > 1e-4), are evaluated at T' and the old rates subtracted.
-// Returns false, with the rates as they were, for those.
+// over L.  |e| is a few 1e-6 (the step is sqrt(eps) T); below 1e-4 what the four
+// terms of the exponential's series leave out is e^4 / 120 < 1e-18 relative, and
+// of the limiter's (w e)^4 = 1e-16.  Falloff and PLOG rates, and exponents beyond
+// 1e-4, are evaluated at T' and the old rates subtracted.  Returns false, with
+// the rates as they were, for those.
 template <int TS, int V>
 __device__ __forceinline__ bool rop_change(const RxnRec &R, int q, const double *__restrict__ sC,
                                            const double *__restrict__ sdG, double *sROP, const double (&dlogT)[V],
@@ -120,7 +121,7 @@ __device__ __forceinline__ bool rop_change(const RxnRec &R, int q, const double 
     ldv<V>(sROP + step * TS + q, r);
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      e[k] = x[k] * (1.0 + x[k] * (0.5 + x[k] * (1.0 / 6.0)));
+      e[k] = x[k] * (1.0 + x[k] * (0.5 + x[k] * (1.0 / 6.0 + x[k] * (1.0 / 24.0))));
       c[k] = 1.0;
     }
     if (limited) {
@@ -136,7 +137,7 @@ __device__ __forceinline__ bool rop_change(const RxnRec &R, int q, const double 
             x = over_each(r[k], sC + q + k, TS, count, spc[0] | spc[1] << 16, spc[2] | spc[3] << 16,
                           spc[4] | spc[5] << 16);
           const double w = x / lim, we = w * e[k];
-          e[k] = e[k] * (1.0 - w) * (1.0 - we * (1.0 - we));
+          e[k] = e[k] * (1.0 - w) * (1.0 - we * (1.0 - we * (1.0 - we)));
         }
     }
 #pragma unroll
