@@ -189,8 +189,9 @@ __device__ __noinline__ void eval_aside(const DevMech &m, const RxnRec *rec, int
 }
 
 // JAC: with the Jacobian when jac is given; without, never (a kernel of its own
-// for more than 16 warps: 65,536 53-species rates 338 us with 64 registers for
-// both, 268 so).
+// where the Jacobian's code costs rates alone: more than 16 warps, whose 64
+// registers spilled, 32,768 53-species rates 438 -> 268 us, and two resident
+// CTAs, the mapping of large calls for rates, 100,003 states 766 -> 603).
 template <int TS, int V, bool GLOBAL, int MAXT, bool STAGE, int MINB, bool JAC>
 __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
     const __grid_constant__ DevMech m, int n, int ld, const double *__restrict__ Tin, const double *__restrict__ Pin,
@@ -670,8 +671,9 @@ __global__ void __launch_bounds__(MAXT, MINB) rates_jac_kernel(
 template <int TS, int V, bool GLOBAL, int MAXT, bool STAGE, int MINB>
 cudaError_t launch_one(const DevMech &m, const RatesJacArgs &a, const KinParams &kp,
                        const LaunchCfg &cfg, cudaStream_t stream) {
-  auto *kern = MAXT > 512 && !a.jac ? rates_jac_kernel<TS, V, GLOBAL, MAXT, STAGE, MINB, (MAXT <= 512)>
-                                    : rates_jac_kernel<TS, V, GLOBAL, MAXT, STAGE, MINB, true>;
+  constexpr bool kOwn = MAXT > 512 || (MINB == 2 && !GLOBAL);  // rates alone have a kernel of their own
+  auto *kern = kOwn && !a.jac ? rates_jac_kernel<TS, V, GLOBAL, MAXT, STAGE, MINB, !kOwn>
+                              : rates_jac_kernel<TS, V, GLOBAL, MAXT, STAGE, MINB, true>;
   const int threads = std::min(cfg.warps * 32, MAXT);
   const int ntiles = (a.n + TS - 1) / TS;
   if (ntiles == 0) return cudaSuccess;
