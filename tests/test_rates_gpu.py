@@ -292,6 +292,29 @@ def test_sri_parameter_count_variants(torch):
     _check(pm, ot, T, P, Y, w, j)
 
 
+@pytest.mark.parametrize("star", ["1e400", "1e308", "1e30", "1e15", "1e-30"])
+def test_troe_filler_temperatures(torch, star, tmp_path):
+    """Troe temperatures that mechanism files use to switch a term on or off for
+    good, the infinite one (a number beyond the range) among them: each term is
+    the constant 1 or absent, as in the oracle."""
+    import re
+
+    import zerork_b200 as zb
+    from plugin_cases import mech_path
+    with open(mech_path("troe_test.mech")) as f:
+        text = f.read()
+    for i in (1, 2):  # T***, T*
+        def put(k):
+            w = k.group(1).split()
+            return "troe / " + " ".join(w[:i] + [star] + w[i + 1:]) + " /"
+        (tmp_path / "m.mech").write_text(re.sub(r"(?i)troe\s*/([^/]*)/", put, text))
+        pm = zb.Mechanism(str(tmp_path / "m.mech"), mech_path("const_specific_heat.therm"))
+        assert np.all(pm.table("fo_par").reshape(-1, 8)[:, 3 + i] == float(star))
+        T, P, Y = _shipped_states(pm.nsp, 40, seed=5)
+        w, j, _ = _run(torch, pm, T, P, Y)
+        _check(pm, oracle_tables(pm), T, P, Y, w, j)
+
+
 def _conc(pm, T, P, Y):
     mw = pm.table("mw")
     rho = P / (8.314462618e3 * T * np.sum(Y / mw, axis=1))

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cstring>
 #include <stdexcept>
 #include <string>
@@ -297,12 +298,16 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     }
   }
   sq_step.push_back(make_int2(0, 0));  // the record fetched past the end
-  // Troe's -1 / T*** and -1 / T* in their places (0 where the term is absent)
+  // Troe's -1 / T*** and -1 / T* in their places (0 where the term is absent; an
+  // infinite temperature's term is there, and constant)
   std::vector<double> fo_par(t.fo_par);
   for (size_t k = 0; k < t.fo_type.size(); ++k)
     if (t.fo_type[k] == kTroe3 || t.fo_type[k] == kTroe4)
       for (int i : {4, 5})
-        if (fo_par[8 * k + i] != 0.0) fo_par[8 * k + i] = -1.0 / fo_par[8 * k + i];
+        if (double &x = fo_par[8 * k + i]; x != 0.0) {
+          x = -1.0 / x;
+          if (x == 0.0) x = -DBL_MIN;
+        }
   Blob b;
   const size_t h = 16;
   size_t o_rbc = b.add(rec_by_cost, h);
