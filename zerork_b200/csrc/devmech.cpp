@@ -225,7 +225,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     return idx;
   };
-  std::vector<double> rc(t.nrxn), sc2(ns), cc(ns);
+  std::vector<double> rc(t.nrxn), sc2(ns);
   for (int j = 0; j < t.nrxn; ++j) {
     const RxnRec &R = rec[j];
     double c = 1.0 + 0.1 * (R.nr + R.np);
@@ -238,13 +238,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
     }
     rc[j] = c;
   }
-  for (int k = 0; k < ns; ++k) {
-    sc2[k] = (sd_ptr[k + 1] - sd_ptr[k]) + (sc_ptr[k + 1] - sc_ptr[k]);
-    double w = 0.0;
-    for (int kk = p.col_ptr[k]; kk < p.col_ptr[k + 1]; ++kk)
-      w += 1.0 + (nzd_ptr[kk + 1] - nzd_ptr[kk]) + (nzc_ptr[kk + 1] - nzc_ptr[kk]);
-    cc[k] = w;
-  }
+  for (int k = 0; k < ns; ++k) sc2[k] = (sd_ptr[k + 1] - sd_ptr[k]) + (sc_ptr[k + 1] - sc_ptr[k]);
   // reactions of one kind together (a warp's groups then run one kind's code),
   // costliest kind first, by cost within
   auto kind_of = [&](int j) {
@@ -253,7 +247,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   };
   std::vector<int> rxn_order = sorted_by(rc);
   std::stable_sort(rxn_order.begin(), rxn_order.end(), [&](int a, int b) { return kind_of(a) < kind_of(b); });
-  const std::vector<int> spc_order = sorted_by(sc2), col_order = sorted_by(cc);
+  const std::vector<int> spc_order = sorted_by(sc2);
 
   // The tables of the rates kernel first, 16-byte aligned and contiguous:
   // the kernel may stage [blob, blob + hot_bytes) in shared memory.
@@ -329,11 +323,9 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   size_t o_jw = b.add(jw), o_jt = b.add(jt), o_jtp = b.add(jt_ptr);
   size_t o_jfc = b.add(jf_col);
   size_t o_snr = b.add(sn_rec), o_sns = b.add(sn_step), o_ne = b.add(net_ent), o_ns = b.add(net_slot), o_np = b.add(net_ptr);
-  size_t o_lr = b.add(p.last_row);
   size_t o_ndp = b.add(nzd_ptr), o_nds = b.add(nzd_step), o_ncp = b.add(nzc_ptr), o_ncs = b.add(nzc_step);
   size_t o_jrp = b.add(jr_ptr), o_jrk = b.add(jr_kk), o_jrc = b.add(jr_col);
   size_t o_rc = b.add(nz_rc);
-  size_t o_ro = b.add(rxn_order), o_co = b.add(col_order);
   bytes_ = b.bytes.size();
   check(cudaMalloc(&blob_, bytes_), "cudaMalloc(mechanism tables)");
   check(cudaMemcpy(blob_, b.bytes.data(), bytes_, cudaMemcpyHostToDevice), "cudaMemcpy(mechanism tables)");
@@ -377,7 +369,6 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.net_ptr = (const int *)P(o_np);
   view_.col_ptr = (const int *)P(o_cp);
   view_.row_idx = (const int *)P(o_ri);
-  view_.last_row = (const int *)P(o_lr);
   view_.nzd_ptr = (const int *)P(o_ndp);
   view_.nzd_step = (const int *)P(o_nds);
   view_.nzc_ptr = (const int *)P(o_ncp);
@@ -395,9 +386,7 @@ DeviceMechanism::DeviceMechanism(const MechTables &t, const JacPattern &p) {
   view_.jr_kk = (const int *)P(o_jrk);
   view_.jr_col = (const int *)P(o_jrc);
   view_.nz_rc = (const int *)P(o_rc);
-  view_.rxn_order = (const int *)P(o_ro);
   view_.spc_order = (const int *)P(o_so);
-  view_.col_order = (const int *)P(o_co);
   view_.rxn_by_cost = (const RxnRec *)P(o_rbc);
   view_.rxn_slots = (const int4 *)P(o_slot);
   view_.thermo_t = (const double *)P(o_tht);

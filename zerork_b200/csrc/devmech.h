@@ -48,7 +48,6 @@ struct alignas(16) Eff {
 // Plain-pointer view of the device tables (all device addresses).
 struct DevMech {
   int nsp, nrxn, nstep, nnz;
-  int max_list;  // unused by kernels, kept for diagnostics
   const double *mw, *inv_mw, *ru_inv_mw, *thermo;  // thermo: [nsp*16]
   const double *thermo_t;  // the same, coefficient by coefficient: [16][nsp]
   const RxnRec *rxn;
@@ -82,7 +81,7 @@ struct DevMech {
   const int4 *sq_rec;
   const int2 *sq_step;
   // Jacobian pattern and per-nonzero gather lists
-  const int *col_ptr, *row_idx, *last_row;
+  const int *col_ptr, *row_idx;
   const int *nzd_ptr, *nzd_step, *nzc_ptr, *nzc_step;
   // Species-column Jacobian entries as one flat list in column-major order
   // without each column's temperature row (nj items; column j holds items
@@ -106,12 +105,10 @@ struct DevMech {
   // [jr_ptr[i], jr_ptr[i+1])
   const int *jr_ptr, *jr_kk, *jr_col;
   const int *nz_rc;  // per Jacobian nonzero: row | column << 16
-  // work lists sorted by decreasing estimated cost, for snake-order
-  // assignment to thread groups: reactions, species (production gathers),
-  // species Jacobian columns
-  const int *rxn_order, *spc_order, *col_order;
-  // the reaction records in rxn_order order (position p holds reaction
-  // rxn_order[p]): one load instead of two dependent ones per work item
+  // work lists for snake-order assignment to thread groups: species by
+  // decreasing length of their lists (production gathers), and the reaction
+  // records by kind and decreasing estimated cost
+  const int *spc_order;
   const RxnRec *rxn_by_cost;
   // The same records for one reactor per CTA, a reaction a lane: grouped by
   // kind (PLOG, falloff, third body, the rest) in blocks of 32 of one kind,

@@ -77,7 +77,7 @@ __device__ __forceinline__ int rhs_warp(const DevMech &m, const IntegOpts &o, co
   if (o.cp || w.src.dpdt != 0.0 || w.src.esrc != 0.0)
     source_T_v(m, o.cp != 0, w.src, t, y, clamp, o.mmf, v0, T_force, lane, 32,
                [](double x) { return wsum(x); }, T, v);
-  const double logT = log(T), invT = 1.0 / T, lprt = log(kPatmD / (kRuD * T));
+  const double logT = log(T), invT = 1.0 / T;
   const double dens = 1.0 / v;
   const double ush = o.cp ? 0.0 : 1.0;  // h/RT - 1 = u/RT; c_p/R - 1 = c_v/R
   double pc = 0.0, pcv = 0.0;
