@@ -108,6 +108,28 @@ def test_group_sources_constant_pressure_ignition(gpu, mech_dir):
         assert np.all(np.abs(ign[hit] - so["t_ign"][hit]) <= 2e-2 * so["t_ign"][hit])
 
 
+@pytest.mark.parametrize("species,reactions", [(160, 900), (200, 600)])
+def test_group_of_many_species(gpu, species, reactions, tmp_path):
+    """Where the net rates' partial sums lie under the Newton matrix (160
+    species) and where the factorization is in global memory with panels of four
+    columns (200): end states against the warp-per-reactor integrator's at the
+    same tolerances (1e-8 relative a step, some hundred steps)."""
+    from zerork_b200 import mechgen
+    from zerork_b200.plugin import Plugin
+    spec = mechgen.SynthSpec(name="g", n_species=species, n_reactions=reactions, elements=("C", "H", "O", "N", "AR"),
+                             n_third_body=60, n_falloff=40, n_irreversible=80, n_troe=None, seed=77)
+    g = mechgen.generate(spec)
+    mf, tf = g.write(str(tmp_path))
+    T, P, Y = mechgen.reactor_states(g, 3, "c3", seed=2)
+    out = []
+    for o in (dict(gpu_method=3, n_reactors_max=3), dict(gpu_method=2)):
+        Tg, Pg, Yg = T.copy(), P.copy(), np.ascontiguousarray(Y.copy())
+        assert Plugin(mf, tf, max_steps=20000, **o).solve(1e-9, Tg, Pg, Yg) == 0
+        out.append((Tg, Yg))
+    assert np.all(np.abs(out[0][0] - out[1][0]) <= 1e-5 * out[1][0])
+    assert np.max(np.abs(out[0][1] - out[1][1])) <= 1e-6
+
+
 def test_group_failure_fails_the_group(gpu, mech_dir):
     """A group whose every attempt fails reports FAILED_SOLVE for each of its
     reactors and leaves their states unchanged."""

@@ -380,35 +380,51 @@ def test_rates_tc_per_step_limiter(torch, mech, therm):
 
 
 @pytest.mark.parametrize("jac", [True, False])
-def test_default_mapping_edges(torch, jac, mech_dir):
-    """The mapping that a call takes from its size gives the results of a fixed
-    one at the edges of every rule (tile remainders, waves of 148 tiles, two
-    CTAs per SM), with odd and even leading dimensions (16-byte accesses or
-    not) and with clamped states (zero mass fractions) among the others.
-    Bound: both are within TOL of the oracle's rounding scale elsewhere; here
-    net rates against the largest rate of the state, entries against the
-    largest of their column."""
+@pytest.mark.parametrize("name,shapes", [
+    ("c1_h2", ((1, 1), (31, 33), (4737, 4740))),
+    ("c2_53", ((1, 1), (7, 9), (9, 10), (1184, 1184), (1185, 1187), (2369, 2370), (4735, 4735), (4736, 4738))),
+    ("c3_160", ((3, 3), (1185, 1186))),
+    ("c4_650", ((1, 1), (9, 9), (500, 502)))])  # workspace in global memory
+def test_default_mapping_edges(torch, name, shapes, jac, mech_dir):
+    """The mapping that a call takes from its size at the edges of every rule
+    (tile remainders, waves of 148 tiles, two CTAs per SM), with odd and even
+    leading dimensions (16-byte accesses or not) and with clamped states (zero
+    mass fractions) among the others: states at the ends, at tile edges and
+    clamped ones against the oracle at TOL of its rounding scale, and all of
+    them, loosely, against a fixed mapping (1e-9 of the state's largest entry:
+    misplaced results, not rounding)."""
     import zerork_b200 as zb
     from zerork_b200 import mechgen
-    g, (m, t) = synth("c2_53", mech_dir)
+    g, (m, t) = synth(name, mech_dir)
     auto, fixed = zb.Mechanism(m, t), zb.Mechanism(m, t)
-    fixed.set_launch(8, 1, 8)
-    T, P, Y = mechgen.rate_states(g, 4740, seed=17)
-    Y[5::7, 3:20] = 0.0
-    for n, ld in ((1, 1), (7, 9), (9, 10), (1184, 1184), (1185, 1187), (2369, 2370), (4735, 4735), (4736, 4738)):
+    fixed.set_launch(8, 1, 8, name == "c4_650", grid=40 if name == "c4_650" else 0)
+    ot = oracle_tables(auto)
+    T, P, Y = mechgen.rate_states(g, max(n for n, _ in shapes), seed=17)
+    Y[5::7, 3:8 if name == "c1_h2" else 20] = 0.0
+    mw = auto.table("mw")
+    for n, ld in shapes:
         dev = [torch.from_numpy(a[:n].copy()).cuda() for a in (T, P)]
         Yd = torch.zeros((auto.nsp, ld), dtype=torch.float64, device="cuda")
-        Yd[:, :n] = torch.from_numpy(np.ascontiguousarray(Y[:n].T)).cuda()
+        Yd[:, :n] = torch.from_numpy(np.ascontiguousarray(Y[:n].T))
         out = []
         for pm in (auto, fixed):
             W = torch.zeros((pm.nsp, ld), dtype=torch.float64, device="cuda")
             J = torch.zeros((pm.nnz, ld), dtype=torch.float64, device="cuda") if jac else None
             D = torch.zeros((pm.nsp + 1, ld), dtype=torch.float64, device="cuda")
             pm.rates_jac(dev[0], dev[1], Yd, W, J, D, n=n)
-            out.append([x.cpu().numpy() for x in (W, J, D) if x is not None])
+            out.append([x.cpu().numpy() for x in (W, D, J) if x is not None])
         for a, b in zip(*out):
             assert np.all(a[:, n:] == 0.0)
             assert np.all(np.abs(a - b) <= 1e-9 * np.abs(b).max(axis=0, keepdims=True)), n
+        idx = sorted({i for i in (0, 5, 7, 8, 12, 15, 16, 31, 32, n // 2, n - 2, n - 1) if 0 <= i < n})
+        if name == "c4_650":
+            idx = idx[:3] + idx[-2:]
+        wo, jo, ws, js = ot.batch_rates_jac_scaled(T[idx], P[idx], Y[idx])
+        assert scaled_err(out[0][0][:, idx].T, wo, ws) < TOL, n
+        v = 8314.462618 * T[idx] * (Y[idx] / mw).sum(1) / P[idx]
+        assert scaled_err(out[0][1][:-1, idx].T, wo * mw * v[:, None], ws * mw * v[:, None]) < TOL, n
+        if jac:
+            assert scaled_err(out[0][2][:, idx].T, jo, js) < TOL, n
 
 
 def test_small_rate_calls(torch, mech_dir):
