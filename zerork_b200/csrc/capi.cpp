@@ -50,19 +50,20 @@ LaunchCfg default_launch(const DevMech &m) {
 }
 
 // The mapping of a call of n states on a handle whose mapping was not set.
-// 16 warps, one CTA per SM; what remains is the tile size.  A wave of 148
-// tiles costs, relative to 8-state tiles, 1.5 with 16 states and 2.25 with 32
-// (53 species: 50, 76 and 114 us a wave; in global workspace, 650 species: 1,
-// 1.56 and 2.7), so the fewest weighted waves win: 8-state tiles up to some
-// 1,200 states, 32-state tiles for large batches (131,072 states, when the rule
-// was made: 3.19 ms, against 4.23 with 16 and 4.7 with 8; 2.85 now).  A thread
-// takes two states where there are reactions enough for the groups (8-state
-// tiles: 325 reactions 56 us a wave with one state, 69 with two; 900 reactions
-// 128 and 113).  A mechanism of a few dozen reactions costs the same per tile
-// at any size (27 reactions: 28-30 us), so it takes the largest, one state a
-// thread (262,144 states 1.38 ms, 2.12 with two).  Without the Jacobian two
-// 8-warp CTAs of 16-state tiles hide more latency (131,072 states 1.12 ms
-// against 1.19).
+// 16 warps, one CTA per SM; what remains is the tile size.  The fewest waves of
+// 148 tiles win, weighted 1, 1.5 and 2.25 for tiles of 8, 16 and 32 states (in
+// global workspace 1, 1.56 and 2.7): 8-state tiles up to some 1,200 states,
+// 32-state tiles for large batches.  The weights are those of the kernel when
+// the rule was made; a wave of 53 species takes 54, 72 and 105 us now (1, 1.3,
+// 2.0) and one of 650 species 458, 907 and 1,645 (1, 2.0, 3.6).  131,072
+// 53-species states: 2.88 ms with 32, 3.73 with 16, 5.16 with 8.  A thread takes
+// two states where there are reactions enough for the groups (8-state tiles, 325
+// reactions 54 us a wave with one state, 64 with two; 900 reactions 120 and 105;
+// nothing between was measured).  A mechanism of a few dozen reactions costs the
+// same per tile at any size (27 reactions: 27-29 us), so it takes the largest,
+// one state a thread (262,144 states 1.22 ms, 1.93 with two); the line at 128
+// reactions is a guess between 27 and 325.  Without the Jacobian two 8-warp CTAs
+// of 16-state tiles hide more latency (131,072 states 0.79 ms against 1.09).
 static LaunchCfg pick_launch(const DevMech &m, int n, bool jac) {
   const size_t kMaxSmem = 227 * 1024;
   int dev = 0, sms = 148;

@@ -340,7 +340,10 @@ __device__ __forceinline__ void third_body(const Eff *__restrict__ eff, int ne, 
 // reduced pressure comes from the difference of the two limits' exponents,
 // Pr = exp(a_low - a_high) [M], which needs no division; a falloff reaction's
 // five or six exponentials, its two logarithms and its quotients then form one
-// chain of a few interleaved groups.
+// chain of a few interleaved groups.  (Troe temperatures such as 1e-30 or 1e15,
+// with which files switch a term off or on, put an exponent beyond the fast
+// range, and that group's exponentials go the library's way one by one: 7 of the
+// dimethyl ether mechanism's 14 Troe reactions.)
 template <int TS, int V, bool PAIR = true>
 __device__ __forceinline__ void reaction_eval(const DevMech &m, const RxnRec &R, int q,
                                               const double *__restrict__ sC,

@@ -282,15 +282,18 @@ cudaError_t ReactorSolver::solve_with_callback(int method, const IntegOpts &io, 
   return cudaSuccess;
 }
 
-// Threads of the dense integrator.  A call lasts as long as its slowest
-// reactor, so a reactor gets a warp for each of its blocks of 32 reactions
-// (devmech.h rxn_slots), 12 when that would be 13 to 16 (barriers then cost what
-// the warps give: 13 blocks, 1000 cells: 72.9 ms with 384 threads, 75.1 with
-// 416, 94.9 with 256) and 16 beyond (900 reactions: 399 ms with 512, 447 with
-// 384).  27 reactions, 64 reactors: 41.1 ms with 96 threads, 45.2 with 64, 52.5
-// with 32; with more small reactors than the SMs hold side by side their
-// number counts instead (1000 reactors: 127 ms with 96, 101 with 32), and the
-// unknowns decide.
+// Threads of the dense integrator.  A call over a long interval lasts as long as
+// its slowest reactor, so a reactor gets a warp for each of its blocks of 32
+// reactions (devmech.h rxn_slots), 12 when that would be 13 to 16 (barriers then
+// cost what the warps give: 13 blocks, 1000 cells over 10 us: 75.9 ms with 384
+// threads, 78.5 with 416, 99.1 with 256) and 16 beyond (900 reactions, 148
+// reactors: 206 ms with 512, 231 with 384).  27 reactions, 64 reactors: 39.5 ms
+// with 96 threads, 42.1 with 64, 57.6 with 32; with more small reactors than the
+// SMs hold side by side their number counts instead (1000 reactors: 119 ms with
+// 96, 104 with 32), and the unknowns decide.  The rule rests on these
+// mechanisms, and on slowest reactors that last: the same 1000 cells over 2 us
+// take 42.5 ms with 384 threads and 31.8 with 256, two reactors an SM, which
+// zrk_plugin_autotune finds.
 static int dense_threads(const DevMech &m, int n, int sms) {
   const int work = std::max(m.nsp + 1, m.nrxn / 2);
   int threads = 32;
