@@ -354,6 +354,25 @@ def test_rates_tc_vs_reference_golden(torch, name, mech_dir):
     assert scaled_err(rop, gd["rop"], np.abs(gd["rop"])) < TOL
 
 
+def test_rates_tc_of_a_large_mechanism(torch, mech_dir):
+    """650 species, too many for tiles of 8 states: calls run a state per CTA
+    whatever their size (up to one state per SM, and beyond)."""
+    import zerork_b200 as zb
+    from zerork_b200 import mechgen
+    g, (m, t) = synth("c4_650", mech_dir)
+    pm = zb.Mechanism(m, t)
+    ot = oracle_tables(pm)
+    T, P, Y = mechgen.rate_states(g, 1500, seed=23)
+    Cc = _conc(pm, T, P, Y)
+    lim = np.full(pm.nstep, 1e22)
+    for n in (148, 149, 1500):
+        net, cre, des, rop = _tc_run(torch, pm, T[:n], Cc[:n], lim)
+        for i in (0, n // 2, n - 1):
+            on, oc, od, orop = ot.rates(T[i], Cc[i], lim)
+            assert scaled_err(net[i], on, np.abs(oc) + np.abs(od)) < TOL
+            assert scaled_err(rop[i], orop, np.abs(orop)) < TOL
+
+
 @pytest.mark.parametrize("mech,therm", SHIPPED)
 def test_rates_tc_per_step_limiter(torch, mech, therm):
     """Per-step limits (some steps unlimited, L = 0) and no limiter at all,

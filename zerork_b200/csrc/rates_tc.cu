@@ -171,6 +171,9 @@ cudaError_t launch_rates_tc(const DevMech &m, const RatesTCArgs &a, cudaStream_t
   if (rates_tc_smem_bytes(m, 32, 256) <= kMax) return launch_tv<32, 2, 1>(m, a, 256, stream);
   if (rates_tc_smem_bytes(m, 16, 256) <= kMax) return launch_tv<16, 1, 1>(m, a, 256, stream);
   if (rates_tc_smem_bytes(m, 8, 256) <= kMax) return launch_tv<8, 1, 1>(m, a, 256, stream);
+  // a mechanism too large for tiles of 8 runs a state at a time at any size, not
+  // only up to one per SM
+  if (rates_tc_smem_bytes(m, 1, 256) <= kMax) return launch_tv<1, 1, 2>(m, a, 256, stream);
   return cudaErrorInvalidValue;
 }
 
